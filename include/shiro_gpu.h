@@ -68,7 +68,7 @@ extern "C" {
  * (shiro_gpu_render_batch; the flag of the call's first request decides):
  * when all the call's paths fit one pool (ShiroWavefrontConfig.
  * paths_in_flight), the forward stages also log every bounce's hits and
- * light-sample visibility (21 bytes per path and bounce of device memory),
+ * light-sample visibility (17 bytes per path and bounce of device memory),
  * and the paths' radiance records and logs stay on the device.  A
  * shiro_gpu_adjoint of one of the call's requests (this flag aside) that
  * follows it, with no wavefront render, adjoint, autotuning, upload,
@@ -362,9 +362,9 @@ int shiro_gpu_render_batch(ShiroGpuContext* ctx, const ShiroRenderDesc* requests
 
 /* Wavefront tuning (tile of paths in flight per wave, waves in flight, block
  * sizes, register cap, lane refill).  Zero fields leave the current value
- * (use_graph is always taken).  Defaults: 8 388 608 paths per wave, two waves
- * in flight, blocks of 128, graphs on, 128 registers, refill every 4 nodes
- * once 8 lanes are idle.  The autotuner sets these itself when
+ * (use_graph is always taken).  Defaults: 33 554 432 paths per wave, two waves
+ * in flight, blocks of 256 (closest hits) and 128, graphs on, 96 registers in
+ * the shade stage, refill every 3 nodes once 8 lanes are idle.  The autotuner sets these itself when
  * shiro_gpu_autotune is called. */
 typedef struct ShiroWavefrontConfig {
     uint32_t paths_in_flight;
@@ -446,7 +446,7 @@ int shiro_gpu_adjoint(ShiroGpuContext* ctx, const ShiroRenderDesc* request, cons
  * light is known); 0 one thread per path (the whole replay, tracing
  * included, in one kernel, after a wavefront pass for the paths' radiance).
  * Both accumulate the same gradients (up to the order of their float
- * atomics).  The wavefront form holds 21 bytes per path slot and bounce of
+ * atomics).  The wavefront form holds 17 bytes per path slot and bounce of
  * device memory for its logs. */
 int shiro_gpu_set_adjoint_form(ShiroGpuContext* ctx, uint32_t wavefront);
 

@@ -1130,10 +1130,14 @@ int build_bvh(const BvhInput& in, cudaStream_t stream, BvhOutput* out, std::stri
         largeHi.z = std::max(largeHi.z, lt.hi[2]);
     }
 
-    // Node array: [top root if needed] + emitted Morton nodes -------------
+    // Node array: [top nodes if needed] + emitted Morton nodes ------------
+    // The top: one root with the Morton tree and one leaf of the large
+    // triangles; or, when a leaf holds one triangle (the tree the wide BVH is
+    // collapsed from), a chain of roots with a large triangle each.
     const bool mortonTree = m >= 2 && mortonRootIsNode;
+    const bool chain = in.maxLeaf == 1 && L > 1;
     const bool needTop = !mortonTree || L > 0;
-    const uint32_t offset = needTop ? 1u : 0u;
+    const uint32_t offset = chain ? L : (needTop ? 1u : 0u);
     const uint32_t nodeCountOut = offset + (mortonTree ? emittedMorton : 0u);
     float4* nodes = nullptr;
     BVH_CHECK(cudaMalloc(&nodes, 4 * sizeof(float4) * static_cast<size_t>(nodeCountOut)));
@@ -1146,7 +1150,26 @@ int build_bvh(const BvhInput& in, cudaStream_t stream, BvhOutput* out, std::stri
     }
     const float4 emptyLo = make_float4(FLT_MAX, FLT_MAX, FLT_MAX, 0), emptyHi = make_float4(-FLT_MAX, -FLT_MAX, -FLT_MAX, 0);
     const int emptyLink = leaf_link_host(0, 1);
-    if (needTop) {
+    if (chain) {
+        // node k: large triangle k beside node k + 1 (the last: beside the Morton tree)
+        float4 restLo = emptyLo, restHi = emptyHi;
+        int rest = emptyLink;
+        if (m > 0) {
+            restLo = mortonLo;
+            restHi = mortonHi;
+            rest = mortonTree ? static_cast<int>(offset) : leaf_link_host(0, static_cast<int>(m));
+        }
+        for (uint32_t k = L; k-- > 0;) {
+            const LargeTri& lt = in.largeSlots[k];
+            const float4 lo = make_float4(lt.lo[0], lt.lo[1], lt.lo[2], 0), hi = make_float4(lt.hi[0], lt.hi[1], lt.hi[2], 0);
+            k_write_root<<<1, 1, 0, stream>>>(nodes + 4 * static_cast<size_t>(k), restLo, restHi, rest, lo, hi,
+                                              leaf_link_host(static_cast<int>(m + k), 1));
+            BVH_CHECK(cudaGetLastError());
+            restLo = make_float4(std::min(restLo.x, lo.x), std::min(restLo.y, lo.y), std::min(restLo.z, lo.z), 0);
+            restHi = make_float4(std::max(restHi.x, hi.x), std::max(restHi.y, hi.y), std::max(restHi.z, hi.z), 0);
+            rest = static_cast<int>(k);
+        }
+    } else if (needTop) {
         int l0 = emptyLink, l1 = emptyLink;
         float4 b0lo = emptyLo, b0hi = emptyHi, b1lo = emptyLo, b1hi = emptyHi;
         if (m > 0) {
@@ -1316,7 +1339,7 @@ __global__ void k_collapse_wide(const float4* __restrict__ nodes2, const float4*
     // the slots of this wide node: replay the cost table's decisions from
     // binary node task.x with 8 slots
     Entry e[8];
-    int n = 0, tris = 0;
+    int n = 0;
     {
         struct Pending {
             Entry e;
@@ -1349,8 +1372,6 @@ __global__ void k_collapse_wide(const float4* __restrict__ nodes2, const float4*
             st[sp++] = {ca, j};
             st[sp++] = {cb, k - j};
         }
-        for (int i = 0; i < n; ++i)
-            if (e[i].link < 0) tris += leaf_count(e[i].link);
     }
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     for (int i = 0; i < n; ++i)
@@ -1413,16 +1434,15 @@ __global__ void k_collapse_wide(const float4* __restrict__ nodes2, const float4*
     }
     int inner = 0;
     for (int i = 0; i < n; ++i) inner += e[i].link >= 0 ? 1 : 0;
+    const int tris = n - inner;  // one per leaf
     const uint32_t childBase = inner ? atomicAdd(nodeCounter, static_cast<unsigned int>(inner)) : 0u;
     const uint32_t triBase = tris ? atomicAdd(triCounter, static_cast<unsigned int>(tris)) : 0u;
     uint8_t q[6][8];
-    uint8_t meta[8];
-    uint32_t imask = 0;
+    uint32_t imask = 0, leaf = 0;
     int rank = 0, off = 0;
     for (int s = 0; s < 8; ++s) {
         const int i = childIn[s];
         if (i < 0) {
-            meta[s] = static_cast<uint8_t>(kWideEmptyMeta);
             for (int k = 0; k < 3; ++k) {
                 q[k][s] = 255;
                 q[3 + k][s] = 0;
@@ -1437,28 +1457,21 @@ __global__ void k_collapse_wide(const float4* __restrict__ nodes2, const float4*
         }
         if (e[i].link >= 0) {
             imask |= 1u << s;
-            meta[s] = 0;
             const unsigned int slot = atomicAdd(nextCount, 1u);
             nextTasks[slot] = make_int2(e[i].link, static_cast<int>(childBase) + rank);
             ++rank;
         } else {
-            const uint32_t enc = ~static_cast<uint32_t>(e[i].link);
-            const uint32_t first = enc >> 3, cnt = (enc & 7u) + 1u;
-            meta[s] = static_cast<uint8_t>(((cnt - 1u) << 5) | static_cast<uint32_t>(off));
-            for (uint32_t k = 0; k < cnt; ++k) {
-                const size_t src = 3 * static_cast<size_t>(first + k), dst = 3 * (static_cast<size_t>(triBase) + off + k);
-                trisOut[dst] = tris2[src];
-                trisOut[dst + 1] = tris2[src + 1];
-                trisOut[dst + 2] = tris2[src + 2];
-            }
-            off += static_cast<int>(cnt);
+            leaf |= 1u << s;
+            const size_t src = 3 * static_cast<size_t>(~static_cast<uint32_t>(e[i].link) >> 3);
+            const size_t dst = 3 * (static_cast<size_t>(triBase) + off);
+            for (int k = 0; k < 3; ++k) trisOut[dst + k] = tris2[src + k];
+            ++off;
         }
     }
     float4* o = out + 5 * static_cast<size_t>(task.y);
-    o[0] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(ex[0] | (ex[1] << 8) | (ex[2] << 16) | (imask << 24)));
-    const uint32_t m0 = meta[0] | (meta[1] << 8) | (meta[2] << 16) | (static_cast<uint32_t>(meta[3]) << 24);
-    const uint32_t m1 = meta[4] | (meta[5] << 8) | (meta[6] << 16) | (static_cast<uint32_t>(meta[7]) << 24);
-    o[1] = make_float4(__uint_as_float(childBase), __uint_as_float(triBase), __uint_as_float(m0), __uint_as_float(m1));
+    o[0] = make_float4(lo[0], lo[1], lo[2], __uint_as_float((ex[2] << 23) | imask));
+    o[1] = make_float4(__uint_as_float(childBase), __uint_as_float(triBase), __uint_as_float(leaf | (leaf << 8)),
+                       __uint_as_float((ex[0] << 23) | (ex[1] << 7)));
     uint32_t w[12];
     for (int r = 0; r < 6; ++r) {
         w[2 * r] = q[r][0] | (q[r][1] << 8) | (q[r][2] << 16) | (static_cast<uint32_t>(q[r][3]) << 24);

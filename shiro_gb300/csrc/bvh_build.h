@@ -43,14 +43,15 @@ inline int leaf_link_host(int first, int count) { return ~((first << 3) | (count
 // Compressed 8-wide BVH (after Ylitie, Karras and Laine, "Efficient
 // incoherent ray traversal on GPUs through compressed wide BVHs", HPG 2017),
 // collapsed from a binary BVH.  Node layout (80 B = 5 x float4):
-//   [0] origin.xyz, bits: ex | ey << 8 | ez << 16 | imask << 24; ex..ez are
-//       biased float exponents of the per-axis power-of-two scales, imask
-//       bit i marks child slot i as an internal node
-//   [1] childBase, triBase, meta[0..3], meta[4..7]: internal children are
-//       wide nodes childBase + (number of internal children in lower slots);
-//       a leaf child's meta byte is (count - 1) << 5 | offset, its triangles
-//       are triBase + offset .. + count - 1 of the wide BVH's own triangle
-//       array (offset + count <= 32); an empty slot has meta 0xff
+//   [0] origin.xyz, bits: ez << 23 | imask; ex, ey, ez are the biased float
+//       exponents of the per-axis power-of-two scales, imask bit i marks child
+//       slot i as an internal node
+//   [1] childBase, triBase, leaf mask | leaf mask << 8, ex << 23 | ey << 7
+//       (each scale is one mask or shift away from its float): internal children are wide nodes
+//       childBase + (number of internal children in lower slots); bit i of
+//       the leaf mask marks child slot i as a leaf of one triangle, entry
+//       triBase + (number of leaf children in lower slots) of the wide BVH's
+//       own triangle array; an empty slot is in neither mask
 //   [2..4] qlo.x[8] qlo.y[8] qlo.z[8] qhi.x[8] qhi.y[8] qhi.z[8] bytes; a
 //       child box is origin + q * scale, rounded outward and widened by one
 //       step per side at build time (origin = node box minus one step)
@@ -58,9 +59,7 @@ inline int leaf_link_host(int first, int count) { return ~((first << 3) | (count
 // ((s & 1) ? -x : +x, (s & 2) ? -y : +y, (s & 4) ? -z : +z) from the node
 // centre, so a ray visits slots in the order of s ^ (7 ^ octant) to go
 // roughly front to back without sorting.
-constexpr uint32_t kWideEmptyMeta = 0xffu;
-constexpr uint32_t kWideMaxTris = 32;  // triangle bits of one node
-constexpr uint32_t kWideLeaf = 1;      // leaf size of the binary tree the wide BVH is collapsed from
+constexpr uint32_t kWideLeaf = 1;  // leaf size of the binary tree the wide BVH is collapsed from
 
 struct WideOutput {
     float4* nodes = nullptr;  // cudaMalloc'ed, 5 float4 per node
@@ -70,8 +69,8 @@ struct WideOutput {
     uint32_t depth = 0;
 };
 
-// Collapses a binary BVH (scene.cuh layout, root = node 0, leaves of at most
-// 8 triangles in `tris2`) into compressed wide nodes; which binary nodes
+// Collapses a binary BVH (scene.cuh layout, root = node 0, leaves of one
+// triangle in `tris2`) into compressed wide nodes; which binary nodes
 // become wide nodes minimises a surface-area cost (optimal collapse over
 // at most 8 slots per node, evaluated bottom-up on the device).
 int collapse_wide(const float4* nodes2, uint32_t nodeCount2, const float4* tris2, uint32_t triCount2, cudaStream_t stream,

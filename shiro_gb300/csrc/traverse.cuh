@@ -57,8 +57,7 @@ struct LocalCounter {
 
 struct HitRec {
     float t, u, v;
-    uint32_t slot;  // leaf-order triangle index, 0xffffffff on a miss
-    uint32_t gid;   // global triangle index (meshes in order)
+    uint32_t gid;  // global triangle index (meshes in order), 0xffffffff on a miss
 };
 
 struct RayInv {
@@ -86,6 +85,19 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float r;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
+}
+
+// Two fused multiply-adds with one instruction (fma.rn.f32x2, sm_100 and
+// later): (x, y) * a + b on register pairs, each half rounded as __fmaf_rn.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint32_t x, uint32_t y, uint64_t a, uint64_t b, float* r0, float* r1) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack2(__uint_as_float(x), __uint_as_float(y))), "l"(a), "l"(b));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(*r0), "=f"(*r1) : "l"(r));
 }
 
 // Entry / exit of both child boxes of a node (slab test, fused form).
@@ -133,8 +145,9 @@ __device__ __forceinline__ bool tri_test(const V3& o, const V3& d, float tMin, f
 
 
 // Children of wide node `node` hit within [0, tmax]: internal ones as bits
-// (slot ^ octInv) of *inner (nearest first = lowest bit), leaf triangles as
-// bits of *tris relative to *triBase.
+// (slot ^ octInv) of *inner (nearest first = lowest bit), leaf slots (one
+// triangle each) as bits 0-7 of *tris with the node's leaf mask in bits 8-15
+// (wide_tri takes the triangles off it).
 //
 // A quantised plane q of an axis lies at t = (origin + q * scale - o) * inv
 // = (2^23 + q) * A + (B - 2^23 * A) with A = scale * inv (exact: scale is a
@@ -142,22 +155,28 @@ __device__ __forceinline__ bool tri_test(const V3& o, const V3& d, float tMin, f
 // the float 2^23 + q, and the bias B - 2^23 * A is formed once per node, so a
 // plane costs one permute and one FMA; the bias rounds to within half a
 // quantisation step, which the builder covers by widening every child box by
-// one step.  Empty slots hold an inverted box (q_lo = 255, q_hi = 0) and the
-// meta byte 0xff.
+// one step.  The near and far plane of an axis share A and B and go through
+// one packed FMA; the children's outcomes are gathered as sign bits.  The test
+// is bound by instruction issue and the integer / min-max pipe (ncu: 68 % of
+// issue slots, 57 % of that pipe): packed FMAs, sign gathering and the
+// one-operation scale and mask words took the 1080p field frame from 111.6 to
+// 107.9 ms.  Empty slots hold an inverted box (q_lo = 255, q_hi = 0), which
+// can only pass when rounding collapses all its planes to one distance; they
+// are in neither mask.
 __device__ __forceinline__ void wide_node(const DevScene& s, uint32_t node, const RayInv& r, float tmax, uint32_t octInv,
                                           uint32_t* childBase, uint32_t* imask, uint32_t* inner, uint32_t* triBase,
                                           uint32_t* tris) {
     const float4* np = s.nodes8 + 5 * static_cast<size_t>(node);
     const float4 a = __ldg(np), b = __ldg(np + 1);
     const float4 q0 = __ldg(np + 2), q1 = __ldg(np + 3), q2 = __ldg(np + 4);
-    const uint32_t eb = __float_as_uint(a.w);
-    const float sx = __uint_as_float((eb & 0xffu) << 23), sy = __uint_as_float(((eb >> 8) & 0xffu) << 23),
-                sz = __uint_as_float(((eb >> 16) & 0xffu) << 23);
+    const uint32_t eb = __float_as_uint(a.w), exy = __float_as_uint(b.w);
+    const float sx = __uint_as_float(exy & 0xffff0000u), sy = __uint_as_float(exy << 16),
+                sz = __uint_as_float(eb & 0xffff0000u);
     const float ax = sx * r.inv.x, ay = sy * r.inv.y, az = sz * r.inv.z;
     const float bx = __fmaf_rn(-8388608.0f, ax, __fmaf_rn(a.x, r.inv.x, -r.ood.x));
     const float by = __fmaf_rn(-8388608.0f, ay, __fmaf_rn(a.y, r.inv.y, -r.ood.y));
     const float bz = __fmaf_rn(-8388608.0f, az, __fmaf_rn(a.z, r.inv.z, -r.ood.z));
-    const uint32_t im = eb >> 24;
+    const uint32_t im = eb & 0xffu;
     // near / far plane words per axis: a negative direction enters through
     // the upper planes (inv < 0 makes their distances the smaller ones)
     const bool nx = r.inv.x < 0.0f, ny = r.inv.y < 0.0f, nz = r.inv.z < 0.0f;
@@ -167,61 +186,66 @@ __device__ __forceinline__ void wide_node(const DevScene& s, uint32_t node, cons
                    hy1 = __float_as_uint(q2.y), hz0 = __float_as_uint(q2.z), hz1 = __float_as_uint(q2.w);
     const uint32_t nw[6] = {nx ? hx0 : lx0, nx ? hx1 : lx1, ny ? hy0 : ly0, ny ? hy1 : ly1, nz ? hz0 : lz0, nz ? hz1 : lz1};
     const uint32_t fw[6] = {nx ? lx0 : hx0, nx ? lx1 : hx1, ny ? ly0 : hy0, ny ? ly1 : hy1, nz ? lz0 : hz0, nz ? lz1 : hz1};
-    uint32_t hit = 0;
+    const uint64_t axx = pack2(ax, ax), ayy = pack2(ay, ay), azz = pack2(az, az);
+    const uint64_t bxx = pack2(bx, bx), byy = pack2(by, by), bzz = pack2(bz, bz);
+    uint32_t miss = 0;  // bit i: child i is missed
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 7; i >= 0; --i) {
         const int h = i >> 2;
         const uint32_t sel = static_cast<uint32_t>(i & 3) | 0x7540u;  // byte i -> float 2^23 + q
-        const float x0 = __fmaf_rn(__uint_as_float(__byte_perm(nw[0 + h], 0x4b000000u, sel)), ax, bx);
-        const float y0 = __fmaf_rn(__uint_as_float(__byte_perm(nw[2 + h], 0x4b000000u, sel)), ay, by);
-        const float z0 = __fmaf_rn(__uint_as_float(__byte_perm(nw[4 + h], 0x4b000000u, sel)), az, bz);
-        const float x1 = __fmaf_rn(__uint_as_float(__byte_perm(fw[0 + h], 0x4b000000u, sel)), ax, bx);
-        const float y1 = __fmaf_rn(__uint_as_float(__byte_perm(fw[2 + h], 0x4b000000u, sel)), ay, by);
-        const float z1 = __fmaf_rn(__uint_as_float(__byte_perm(fw[4 + h], 0x4b000000u, sel)), az, bz);
+        float x0, x1, y0, y1, z0, z1;
+        fma2(__byte_perm(nw[0 + h], 0x4b000000u, sel), __byte_perm(fw[0 + h], 0x4b000000u, sel), axx, bxx, &x0, &x1);
+        fma2(__byte_perm(nw[2 + h], 0x4b000000u, sel), __byte_perm(fw[2 + h], 0x4b000000u, sel), ayy, byy, &y0, &y1);
+        fma2(__byte_perm(nw[4 + h], 0x4b000000u, sel), __byte_perm(fw[4 + h], 0x4b000000u, sel), azz, bzz, &z0, &z1);
         const float lo = fmax3(x0, y0, fmaxf(z0, 0.0f));
         const float hi = fmin3(x1, y1, fminf(z1, tmax));
-        hit |= (lo <= hi ? 1u : 0u) << i;
+        // the sign of hi - lo (never rounded to the other sign) shifts in
+        miss = __funnelshift_l(__float_as_uint(hi - lo), miss, 1);
     }
     // internal children: bit i moves to bit i ^ octInv
-    uint32_t in = hit & im;
+    uint32_t in = im & ~miss;
     if (octInv & 1u) in = ((in & 0x55u) << 1) | ((in >> 1) & 0x55u);
     if (octInv & 2u) in = ((in & 0x33u) << 2) | ((in >> 2) & 0x33u);
     if (octInv & 4u) in = ((in & 0x0fu) << 4) | ((in >> 4) & 0x0fu);
-    // leaf children: their triangles' bits from the meta bytes
-    const uint64_t meta = (static_cast<uint64_t>(__float_as_uint(b.w)) << 32) | __float_as_uint(b.z);
-    uint32_t lf = hit & ~im, tb = 0;
-    while (lf) {
-        const uint32_t i = static_cast<uint32_t>(__ffs(lf) - 1);
-        lf &= lf - 1u;
-        const uint32_t mt = static_cast<uint32_t>(meta >> (8u * i)) & 0xffu;
-        // an empty slot's inverted box can only pass when rounding collapses
-        // all its planes to one distance; it never contributes triangles
-        if (mt != 0xffu) tb |= ((2u << (mt >> 5)) - 1u) << (mt & 31u);
-    }
     *childBase = __float_as_uint(b.x);
     *triBase = __float_as_uint(b.y);
     *imask = im;
     *inner = in;
-    *tris = tb;
+    *tris = __float_as_uint(b.z) & ~miss;
+}
+
+// Whether a node's triangle word (wide_node) still holds triangles to test.
+__device__ __forceinline__ bool wide_has_tri(uint32_t bits) { return (bits & 0xffu) != 0u; }
+
+// Takes the next triangle off a node's triangle word: its index in the wide
+// order (the leaf slots' triangles lie one after another from triBase on).
+__device__ __forceinline__ uint32_t wide_tri(uint32_t triBase, uint32_t& bits) {
+    const uint32_t low = bits & (0u - bits);  // the lowest slot left (bits 0-7 are not all clear)
+    bits ^= low;
+    return triBase + static_cast<uint32_t>(__popc((bits >> 8) & (low - 1u)));
 }
 
 __device__ __forceinline__ uint32_t ray_oct_inv(const V3& d) {
     return 7u ^ ((d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u));
 }
 
-// Wide-BVH traversal as resumable state (one node and its triangles per
-// step), so a caller may interleave rays: the wavefront stages refill a lane
-// with a new ray as soon as its ray finishes.  Stack entries are groups of
-// sibling wide nodes still to visit: (childBase, remaining inner bits << 8 |
-// imask); the caller owns the stack array.
+constexpr uint32_t kNoNode = 0xffffffffu;
+
+// Wide-BVH traversal as resumable state, so that a caller may interleave rays
+// (the wavefront stages refill a lane with a new ray as soon as its ray
+// finishes) and choose when a node's triangles are tested.  Stack entries are
+// groups of sibling wide nodes still to visit: (childBase, remaining inner
+// bits << 8 | imask); the caller owns the stack array.  A ray is finished when
+// neither a node nor a triangle is left.
 struct WideTrav {
     V3 o, d;
     RayInv r;
     uint32_t octInv;
     float tmax;                 // closest: the best distance so far; occlusion: maxDist
     float bu, bv;
-    uint32_t bestGid, bestSlot;
-    uint32_t node;              // next node to visit
+    uint32_t bestGid;           // closest: 0xffffffff while nothing is hit
+    uint32_t node;              // next node to visit, kNoNode when none is left
+    uint32_t tBase, tBits;      // triangles of the visited node not tested yet
     int sp;
     uint32_t visits;
 };
@@ -235,18 +259,30 @@ __device__ __forceinline__ void wide_init(WideTrav& t, const V3& o, const V3& d,
     t.bu = 0.0f;
     t.bv = 0.0f;
     t.bestGid = 0xffffffffu;
-    t.bestSlot = 0xffffffffu;
     t.node = 0;
+    t.tBase = 0;
+    t.tBits = 0;
     t.sp = 0;
     t.visits = 0;
 }
 
-// Moves to the next node of the traversal; false when none is left (or on a
-// violated bound, which also sets the error word and clears the hit).
-__device__ __forceinline__ bool wide_next(const DevScene& s, WideTrav& t, uint2* stack, uint32_t gBase, uint32_t gImask,
+// Ends a ray whose bounds check failed: the error word is set, the ray hits
+// nothing.
+__device__ __forceinline__ void wide_abort(const DevScene& s, WideTrav& t, uint32_t err) {
+    atomicOr(s.error, err);
+    t.bestGid = 0xffffffffu;
+    t.node = kNoNode;
+    t.tBits = 0;
+}
+
+// Moves to the next node of the traversal (kNoNode when none is left).
+__device__ __forceinline__ void wide_next(const DevScene& s, WideTrav& t, uint2* stack, uint32_t gBase, uint32_t gImask,
                                           uint32_t gInner) {
     if (gInner == 0u) {
-        if (t.sp == 0) return false;
+        if (t.sp == 0) {
+            t.node = kNoNode;
+            return;
+        }
         --t.sp;
         gBase = stack[t.sp].x;
         gInner = stack[t.sp].y >> 8;
@@ -257,74 +293,46 @@ __device__ __forceinline__ bool wide_next(const DevScene& s, WideTrav& t, uint2*
     t.node = gBase + __popc(gImask & ((1u << slot) - 1u));
     if (gInner) {
         if (t.sp >= kStackWide) {
-            atomicOr(s.error, kErrStackOverflow);
-            t.bestSlot = 0xffffffffu;
-            return false;
+            wide_abort(s, t, kErrStackOverflow);
+            return;
         }
         stack[t.sp++] = make_uint2(gBase, (gInner << 8) | gImask);
     }
-    return true;
 }
 
-// Closest hit: up to `steps` nodes; true when finished (result in t.tmax,
-// t.bu, t.bv, t.bestSlot, t.bestGid).
-template <typename Ctr>
-__device__ __forceinline__ bool wide_closest_advance(const DevScene& s, WideTrav& t, uint2* stack, int steps, Ctr& ctr) {
-    for (int k = 0; k < steps; ++k) {
-        if (++t.visits > kMaxVisits) {
-            atomicOr(s.error, kErrTraversalLimit);
-            t.bestSlot = 0xffffffffu;
-            return true;
-        }
-        ctr.node();
-        uint32_t gBase, gImask, gInner, tBase, tBits;
-        wide_node(s, t.node, t.r, t.tmax, t.octInv, &gBase, &gImask, &gInner, &tBase, &tBits);
-        while (tBits) {
-            const uint32_t kk = tBase + static_cast<uint32_t>(__ffs(tBits) - 1);
-            tBits &= tBits - 1u;
-            ctr.tri();
-            const float4* tp = s.tris + 3 * static_cast<size_t>(kk);
-            const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
-            float tt, u, v;
-            if (!tri_test(t.o, t.d, kRayEpsilon, FLT_MAX, ta, tb, tc, &tt, &u, &v)) continue;
-            const uint32_t gid = __float_as_uint(ta.w);
-            if (tt < t.tmax || (tt == t.tmax && gid < t.bestGid)) {
-                t.tmax = tt;
-                t.bestGid = gid;
-                t.bestSlot = kk;
-                t.bu = u;
-                t.bv = v;
-            }
-        }
-        if (!wide_next(s, t, stack, gBase, gImask, gInner)) return true;
+// Visits t.node (its triangles go to tBase / tBits) and moves to the next.
+__device__ __forceinline__ void wide_visit(const DevScene& s, WideTrav& t, uint2* stack) {
+    if (++t.visits > kMaxVisits) {
+        wide_abort(s, t, kErrTraversalLimit);
+        return;
     }
-    return false;
+    uint32_t gBase, gImask, gInner;
+    wide_node(s, t.node, t.r, t.tmax, t.octInv, &gBase, &gImask, &gInner, &t.tBase, &t.tBits);
+    wide_next(s, t, stack, gBase, gImask, gInner);
 }
 
-// Any hit in [1e-4, t.tmax]: up to `steps` nodes; -1 while running, else
-// 1 occluded / 0 clear.
-template <typename Ctr>
-__device__ __forceinline__ int wide_occluded_advance(const DevScene& s, WideTrav& t, uint2* stack, int steps, Ctr& ctr) {
-    for (int k = 0; k < steps; ++k) {
-        if (++t.visits > kMaxVisits) {
-            atomicOr(s.error, kErrTraversalLimit);
-            return 0;
-        }
-        ctr.onode();
-        uint32_t gBase, gImask, gInner, tBase, tBits;
-        wide_node(s, t.node, t.r, t.tmax, t.octInv, &gBase, &gImask, &gInner, &tBase, &tBits);
-        while (tBits) {
-            const uint32_t kk = tBase + static_cast<uint32_t>(__ffs(tBits) - 1);
-            tBits &= tBits - 1u;
-            ctr.otri();
-            const float4* tp = s.tris + 3 * static_cast<size_t>(kk);
-            const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
-            float tt, u, v;
-            if (tri_test(t.o, t.d, kRayEpsilon, t.tmax, ta, tb, tc, &tt, &u, &v)) return 1;
-        }
-        if (!wide_next(s, t, stack, gBase, gImask, gInner)) return 0;
+// Tests one pending triangle; keeps the closest hit (ties: the lower global
+// index).
+__device__ __forceinline__ void wide_test_closest(const DevScene& s, WideTrav& t) {
+    const float4* tp = s.tris + 3 * static_cast<size_t>(wide_tri(t.tBase, t.tBits));
+    const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+    float tt, u, v;
+    if (!tri_test(t.o, t.d, kRayEpsilon, FLT_MAX, ta, tb, tc, &tt, &u, &v)) return;
+    const uint32_t gid = __float_as_uint(ta.w);
+    if (tt < t.tmax || (tt == t.tmax && gid < t.bestGid)) {
+        t.tmax = tt;
+        t.bestGid = gid;
+        t.bu = u;
+        t.bv = v;
     }
-    return -1;
+}
+
+// Tests one pending triangle for any hit in [1e-4, t.tmax].
+__device__ __forceinline__ bool wide_test_any(const DevScene& s, WideTrav& t) {
+    const float4* tp = s.tris + 3 * static_cast<size_t>(wide_tri(t.tBase, t.tBits));
+    const float4 ta = __ldg(tp), tb = __ldg(tp + 1), tc = __ldg(tp + 2);
+    float tt, u, v;
+    return tri_test(t.o, t.d, kRayEpsilon, t.tmax, ta, tb, tc, &tt, &u, &v);
 }
 
 template <typename Ctr>
@@ -332,13 +340,19 @@ __device__ bool trace_closest_wide(const DevScene& s, const V3& o, const V3& d, 
     WideTrav t;
     uint2 stack[kStackWide];
     wide_init(t, o, d, FLT_MAX);
-    wide_closest_advance(s, t, stack, 0x7fffffff, ctr);
+    do {
+        ctr.node();
+        wide_visit(s, t, stack);
+        while (wide_has_tri(t.tBits)) {
+            ctr.tri();
+            wide_test_closest(s, t);
+        }
+    } while (t.node != kNoNode);
     out->t = t.tmax;
     out->u = t.bu;
     out->v = t.bv;
-    out->slot = t.bestSlot;
     out->gid = t.bestGid;
-    return t.bestSlot != 0xffffffffu;
+    return t.bestGid != 0xffffffffu;
 }
 
 template <typename Ctr>
@@ -346,7 +360,15 @@ __device__ bool trace_occluded_wide(const DevScene& s, const V3& o, const V3& d,
     WideTrav t;
     uint2 stack[kStackWide];
     wide_init(t, o, d, maxDist);
-    return wide_occluded_advance(s, t, stack, 0x7fffffff, ctr) == 1;
+    do {
+        ctr.onode();
+        wide_visit(s, t, stack);
+        while (wide_has_tri(t.tBits)) {
+            ctr.otri();
+            if (wide_test_any(s, t)) return true;
+        }
+    } while (t.node != kNoNode);
+    return false;
 }
 
 template <typename Ctr>
@@ -355,7 +377,7 @@ __device__ __noinline__ bool trace_closest(const DevScene& s, const V3 o, const 
     if (s.nodes8) return trace_closest_wide(s, o, d, out, ctr);
     const RayInv r = ray_inv(o, d);
     float bestT = FLT_MAX;
-    uint32_t bestGid = 0xffffffffu, bestSlot = 0xffffffffu;
+    uint32_t bestGid = 0xffffffffu;
     float bu = 0.0f, bv = 0.0f;
     int stackNode[kStack];
     float stackT[kStack];
@@ -365,7 +387,7 @@ __device__ __noinline__ bool trace_closest(const DevScene& s, const V3 o, const 
     for (;;) {
         if (++visits > kMaxVisits) {
             atomicOr(s.error, kErrTraversalLimit);
-            bestSlot = 0xffffffffu;
+            bestGid = 0xffffffffu;
             break;
         }
         if (node >= 0) {
@@ -380,7 +402,7 @@ __device__ __noinline__ bool trace_closest(const DevScene& s, const V3 o, const 
                 const bool swap = t1 < t0;
                 if (sp >= kStack) {
                     atomicOr(s.error, kErrStackOverflow);
-                    bestSlot = 0xffffffffu;
+                    bestGid = 0xffffffffu;
                     break;
                 }
                 stackNode[sp] = swap ? c0 : c1;
@@ -410,7 +432,6 @@ __device__ __noinline__ bool trace_closest(const DevScene& s, const V3 o, const 
                 if (t < bestT || (t == bestT && gid < bestGid)) {
                     bestT = t;
                     bestGid = gid;
-                    bestSlot = k;
                     bu = u;
                     bv = v;
                 }
@@ -431,9 +452,8 @@ __device__ __noinline__ bool trace_closest(const DevScene& s, const V3 o, const 
     out->t = bestT;
     out->u = bu;
     out->v = bv;
-    out->slot = bestSlot;
     out->gid = bestGid;
-    return bestSlot != 0xffffffffu;
+    return bestGid != 0xffffffffu;
 }
 
 // Any hit with t in [1e-4, maxDist] (Occluded, CpuPathTracer.cpp:468-475).
