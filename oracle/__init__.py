@@ -31,7 +31,7 @@ def build_port() -> str:
 
 
 def build_ref() -> str | None:
-    if not os.path.isdir(REF_TREE):
+    if not os.path.exists(os.path.join(REF_TREE, "src", "render", "EnvironmentMap.cpp")):  # no reference sources here
         return None
     subprocess.run(["make", "-s", "-C", HERE, "ref", f"REF={REF_TREE}"], check=True)
     return REF_LIB
