@@ -335,19 +335,29 @@ __device__ __forceinline__ bool wide_test_any(const DevScene& s, WideTrav& t) {
     return tri_test(t.o, t.d, kRayEpsilon, t.tmax, ta, tb, tc, &tt, &u, &v);
 }
 
+// The one-thread forms test a node's triangles before they move on: with the
+// move first, lanes without triangles ran ahead of the others and the warp
+// fell apart (90 instead of 31 ms for the 961x541 15-spp field frame).
 template <typename Ctr>
 __device__ bool trace_closest_wide(const DevScene& s, const V3& o, const V3& d, HitRec* out, Ctr& ctr) {
     WideTrav t;
     uint2 stack[kStackWide];
     wide_init(t, o, d, FLT_MAX);
-    do {
+    for (;;) {
+        if (++t.visits > kMaxVisits) {
+            wide_abort(s, t, kErrTraversalLimit);
+            break;
+        }
         ctr.node();
-        wide_visit(s, t, stack);
+        uint32_t gBase, gImask, gInner;
+        wide_node(s, t.node, t.r, t.tmax, t.octInv, &gBase, &gImask, &gInner, &t.tBase, &t.tBits);
         while (wide_has_tri(t.tBits)) {
             ctr.tri();
             wide_test_closest(s, t);
         }
-    } while (t.node != kNoNode);
+        wide_next(s, t, stack, gBase, gImask, gInner);
+        if (t.node == kNoNode) break;
+    }
     out->t = t.tmax;
     out->u = t.bu;
     out->v = t.bv;
@@ -360,15 +370,21 @@ __device__ bool trace_occluded_wide(const DevScene& s, const V3& o, const V3& d,
     WideTrav t;
     uint2 stack[kStackWide];
     wide_init(t, o, d, maxDist);
-    do {
+    for (;;) {
+        if (++t.visits > kMaxVisits) {
+            wide_abort(s, t, kErrTraversalLimit);
+            return false;
+        }
         ctr.onode();
-        wide_visit(s, t, stack);
+        uint32_t gBase, gImask, gInner;
+        wide_node(s, t.node, t.r, t.tmax, t.octInv, &gBase, &gImask, &gInner, &t.tBase, &t.tBits);
         while (wide_has_tri(t.tBits)) {
             ctr.otri();
             if (wide_test_any(s, t)) return true;
         }
-    } while (t.node != kNoNode);
-    return false;
+        wide_next(s, t, stack, gBase, gImask, gInner);
+        if (t.node == kNoNode) return false;
+    }
 }
 
 template <typename Ctr>
