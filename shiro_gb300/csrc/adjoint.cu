@@ -46,7 +46,7 @@ __device__ __noinline__ V3 adj_path(const DevScene& s, const DevRequest& q, cons
                                     uint32_t sampleIndex, const V3 delta, const V3 Ltot, float* depthOut,
                                     const bool kGrad) {
     NullCounter ctr;
-    const Sampler smp{x, y, sampleIndex};
+    const Sampler smp{x, y, sampleIndex, s.radical};
     PathState ps;
     init_path(q, smp, ps);
     // throughput under the sampling parameters: Russian roulette decides on it
@@ -118,11 +118,11 @@ __device__ __noinline__ V3 adj_path(const DevScene& s, const DevRequest& q, cons
                 float lp, nl;
                 if (!emissive_geometry(s, v, smp, depth, &ld, &L, &lp, &nl, &reach)) return false;
                 Ls = L;
-                const float bp = bsdf_pdf_rec(rec, ms, v.w, v.n, v.cn, v.view, ld);
+                const float bp = bsdf_pdf_rec(rec, ms, v.n, v.cn, v.view, ld);
                 w = nl * power_heuristic(lp, bp) / lp;
             } else if (k < s.distantCount) {
                 const DevDistant l = s.distant[k];
-                ld = normalize(l.direction * -1.0f);
+                ld = l.toLight;
                 const float nl = sclamp(dot(v.n, ld), 0.0f, 1.0f);
                 if (nl <= 0.0f) return false;
                 L = l.radiance;
@@ -154,7 +154,7 @@ __device__ __noinline__ V3 adj_path(const DevScene& s, const DevRequest& q, cons
                 ld = light_to_world(d, local);
                 const float nl = sclamp(dot(v.n, ld), 0.0f, 1.0f);
                 if (nl <= 0.0f) return false;
-                const float bp = bsdf_pdf_rec(rec, ms, v.w, v.n, v.cn, v.view, ld);
+                const float bp = bsdf_pdf_rec(rec, ms, v.n, v.cn, v.view, ld);
                 const float mis = power_heuristic(lp, bp);
                 w = nl * mis / lp;
             }
@@ -202,13 +202,13 @@ __device__ __noinline__ V3 adj_path(const DevScene& s, const DevRequest& q, cons
             if (ps.specDepth >= q.specularDepth) break;
             ++ps.specDepth;
             const V3 sn = coat ? v.cn : v.n;
-            const float sr = coat ? roughness_for(ms.coat_roughness, ms.coat_anisotropy, ms.coat_rotation)
-                                  : roughness_for(base_roughness(ms), ms.specular_anisotropy, ms.specular_rotation);
+            const float4 r7 = rec[7];
+            const float sr = coat ? r7.y : r7.x;
             const V3 hv = ggx_half(sn, ds, sr);
             next = normalize(reflect(ps.rd, hv));
             const float rc = sclamp(dot(sn, next), 0.0f, 1.0f);
             if (rc <= 0.0f) break;
-            pdf = smax((rw / tw) * bsdf_pdf_rec(rec, ms, v.w, v.n, v.cn, v.view, next), 1.0e-6f);
+            pdf = smax((rw / tw) * bsdf_pdf_rec(rec, ms, v.n, v.cn, v.view, next), 1.0e-6f);
             f = evalE(next);
             delta2 = sr <= kDeltaRoughness;
         }

@@ -81,6 +81,7 @@ struct ContextImpl {
     DeviceBlock aovScratch;
     DeviceBlock probeScratch;
     uint32_t* errorWord = nullptr;
+    float* radicalTable = nullptr;  // DevScene::radical, built when the context is created
     // device address of the static path-record array of shiro_gpu_render_static
     // (render_static.cu), looked up when the context is created; staticError
     // says why it is NULL

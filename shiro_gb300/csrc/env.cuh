@@ -145,18 +145,30 @@ __device__ __forceinline__ uint32_t env_cdf_search(const float* cdf, uint32_t be
     return lo - 1u;
 }
 
+static __device__ __noinline__ size_t env_pick_cdf(const DevEnv& e, const V2 u) {
+    const uint32_t r = env_cdf_search(e.rowCdf, 0u, e.h, u.y);
+    const uint32_t off = r * (e.w + 1u);
+    const uint32_t c = env_cdf_search(e.condCdf, off, off + e.w, u.x);
+    return static_cast<size_t>(r) * e.w + (c - off);
+}
+
+// A direction drawn uniformly over the sphere (maps without an importance
+// table and constant domes).
+static __device__ __noinline__ V3 sphere_direction(const V2 u) {
+    const float y = 1.0f - 2.0f * u.y;
+    const float r = sqrtf(smax(0.0f, 1.0f - y * y));
+    const float phi = kTwoPi * u.x;
+    return V3{sinf(phi) * r, y, cosf(phi) * r};
+}
+static __device__ __noinline__ V3 env_evaluate_out(const DevEnv& e, const V3 local) { return env_evaluate(e, local); }
+
 // The texel a 2-D sample picks in a lat-long map with an importance table:
 // the CDF search of SampleCdf (row on u.y, column on u.x), or the alias
 // lookup (bucket floor(u.y * n) - exact for a power-of-two n, as u.y * n then
 // only shifts the exponent - accepted when u.x is below its threshold, else
 // its alias).
 __device__ __forceinline__ size_t env_pick(const DevEnv& e, const V2& u, bool useCdf) {
-    if (useCdf) {
-        const uint32_t r = env_cdf_search(e.rowCdf, 0u, e.h, u.y);
-        const uint32_t off = r * (e.w + 1u);
-        const uint32_t c = env_cdf_search(e.condCdf, off, off + e.w, u.x);
-        return static_cast<size_t>(r) * e.w + (c - off);
-    }
+    if (useCdf) return env_pick_cdf(e, u);
     const uint32_t n = e.w * e.h;
     uint32_t i = static_cast<uint32_t>(u.y * static_cast<float>(n));
     i = i >= n ? n - 1u : i;
@@ -181,13 +193,10 @@ __device__ __forceinline__ V3 env_sample(const DevEnv& e, const V2& u, bool useC
         *pdf = a.w;
         return {b.x, b.y, b.z};
     }
-    const float y = 1.0f - 2.0f * u.y;
-    const float r = sqrtf(smax(0.0f, 1.0f - y * y));
-    const float phi = kTwoPi * u.x;
-    const V3 d{sinf(phi) * r, y, cosf(phi) * r};
+    const V3 d = sphere_direction(u);
     *dir = d;
     *pdf = kInvFourPi;
-    return env_evaluate(e, d);
+    return env_evaluate_out(e, d);
 }
 
 // ---- dome light helpers (CpuPathTracer.cpp:315-384) -----------------------
@@ -228,10 +237,7 @@ __device__ __forceinline__ bool sample_dome(const DevScene& s, const DevDome& d,
     if (d.env >= 0) {
         lr = env_sample(s.envs[d.env], u, useCdf, &ld, &lp);
     } else {
-        const float y = 1.0f - 2.0f * u.y;
-        const float r = sqrtf(smax(0.0f, 1.0f - y * y));
-        const float phi = 2.0f * kPi * u.x;
-        ld = V3{sinf(phi) * r, y, cosf(phi) * r};
+        ld = sphere_direction(u);  // (2 kPi = kTwoPi: a power of two times kPi)
         lp = kInvFourPi;
         lr = V3{1.0f, 1.0f, 1.0f};
     }

@@ -172,48 +172,6 @@ __device__ __forceinline__ float emitter_pdf(const DevScene& s, uint32_t gid, co
 // Origin of the shadow rays of a vertex (:1527).
 __device__ __forceinline__ V3 shadow_origin(const Vertex& v) { return v.hit.position + v.n * kRayEpsilon; }
 
-// Distant light i (:1529-1540): false when the light is below the horizon;
-// otherwise the direction and the clamped contribution if unoccluded.
-template <typename Ctr>
-__device__ __forceinline__ bool light_distant(const DevScene& s, const DevRequest& q, const Vertex& v, uint32_t i, V3* dir,
-                                              V3* c, Ctr& ctr) {
-    const DevDistant l = s.distant[i];
-    const V3 ld = normalize(l.direction * -1.0f);
-    const float nl = sclamp(dot(v.n, ld), 0.0f, 1.0f);
-    if (nl <= 0.0f) return false;
-    const Mat& m = s.materials[v.hit.material];
-    ctr.bsdf_eval();
-    *dir = ld;
-    *c = clamp24(q, bsdf_eval_rec(bsdf_rec(s, v.hit.material), m, v.n, v.cn, v.view, ld) * l.radiance * nl);
-    return true;
-}
-
-// Sample k of dome light li (:1542-1573).
-template <typename Ctr>
-__device__ __forceinline__ bool light_dome(const DevScene& s, const DevRequest& q, const Vertex& v, const Sampler& smp,
-                                           uint32_t depth, uint32_t li, uint32_t k, V3* dir, V3* c, Ctr& ctr) {
-    const uint32_t dim = kDirectDimBase + depth * kDirectDepthStride + li * kDirectLightStride + k * kDirectSampleStride;
-    V3 ld, lr;
-    float lp = 0.0f;
-    if (s.domes[li].env >= 0) {
-        ctr.env_sample();
-        ctr.env_eval();
-    }
-    const bool useCdf = (q.flags & SHIRO_RENDER_ENV_CDF) != 0u;
-    if (!sample_dome(s, s.domes[li], smp.next2d(dim), useCdf, &ld, &lr, &lp) || lp <= 0.0f) return false;
-    const float nl = sclamp(dot(v.n, ld), 0.0f, 1.0f);
-    if (nl <= 0.0f) return false;
-    const Mat& m = s.materials[v.hit.material];
-    ctr.bsdf_pdf();
-    ctr.bsdf_eval();
-    const float4* rec = bsdf_rec(s, v.hit.material);
-    const float bp = bsdf_pdf_rec(rec, m, v.w, v.n, v.cn, v.view, ld);
-    const float mis = power_heuristic(lp, bp);
-    *dir = ld;
-    *c = clamp24(q, bsdf_eval_rec(rec, m, v.n, v.cn, v.view, ld) * lr * (nl * mis / lp));
-    return true;
-}
-
 // Adds the unoccluded contributions in the reference's order: distant lights,
 // then per dome the average of its samples.  `visible(k, dir, c)` returns
 // whether light sample k (in that order) is present and unoccluded.
@@ -246,14 +204,20 @@ __device__ __forceinline__ V3 sum_direct(const DevScene& s, const DevRequest& q,
 // an emitter, its direction *ld from the vertex, the emitted radiance *le,
 // the sample's solid-angle pdf *lp, the cosine *nl at the vertex and the
 // reach of its shadow ray, which stops short of the light.
-__device__ __forceinline__ bool emissive_geometry(const DevScene& s, const Vertex& v, const Sampler& smp, uint32_t depth,
-                                                  V3* ld, V3* le, float* lp, float* nl, float* maxDist) {
-    if (!has_emitters(s)) return false;
+struct EmissiveSample {
+    V3 ld, le;
+    float lp, nl, maxDist;  // maxDist < 0: no sample
+};
+static __device__ __noinline__ EmissiveSample emissive_sample(const DevScene& s, const V3 position, const V3 n,
+                                                              uint32_t hitGid, const Sampler smp, uint32_t depth) {
+    EmissiveSample o;
+    o.maxDist = -1.0f;
+    if (!has_emitters(s)) return o;
     const uint32_t db = kEmissiveDimBase + depth * kEmissiveDepthStride;
     const uint32_t k = sample_emitter(s, smp.next1d(db + 0u));
     const float4 e0 = __ldg(&s.emissive[3 * k]), e1 = __ldg(&s.emissive[3 * k + 1]), e2 = __ldg(&s.emissive[3 * k + 2]);
     const uint32_t gid = __float_as_uint(e0.w);
-    if (gid == v.hit.gid) return false;
+    if (gid == hitGid) return o;
     const V2 u = smp.next2d(db + 1u);
     const float su = sqrtf(sclamp(u.x, 0.0f, 1.0f));  // UniformTriangleBarycentrics, :240-253
     const float b0 = 1.0f - su;
@@ -262,55 +226,74 @@ __device__ __forceinline__ bool emissive_geometry(const DevScene& s, const Verte
     const uint4 tv = __ldg(&s.triVerts[gid]);
     const V3 p = f4xyz(__ldg(&s.positions[tv.x])) * b0 + f4xyz(__ldg(&s.positions[tv.y])) * b1 +
                  f4xyz(__ldg(&s.positions[tv.z])) * b2;  // TrianglePoint, :224-238
-    const V3 to = p - v.hit.position;
+    const V3 to = p - position;
     const float d2 = dot(to, to);
-    if (d2 <= 1.0e-10f) return false;
+    if (d2 <= 1.0e-10f) return o;
     const float dist = sqrtf(d2);
-    *ld = to / dist;
-    *nl = sclamp(dot(v.n, *ld), 0.0f, 1.0f);
-    const float cosL = fabsf(dot(f4xyz(e2), *ld * -1.0f));
-    if (*nl <= 0.0f || cosL <= 0.0f) return false;
+    o.ld = to / dist;
+    o.nl = sclamp(dot(n, o.ld), 0.0f, 1.0f);
+    const float cosL = fabsf(dot(f4xyz(e2), o.ld * -1.0f));
+    if (o.nl <= 0.0f || cosL <= 0.0f) return o;
     const float sel = e0.y / s.emissiveSum;
     const float areaPdf = sel / smax(e0.x, 1.0e-6f);
-    *lp = areaPdf * d2 / smax(cosL, 1.0e-6f);
-    if (*lp <= 0.0f) return false;
-    *le = f4xyz(e1);
-    *maxDist = smax(dist - 2.0f * kRayEpsilon, kRayEpsilon);
-    return true;
+    o.lp = areaPdf * d2 / smax(cosL, 1.0e-6f);
+    if (o.lp <= 0.0f) return o;
+    o.le = f4xyz(e1);
+    o.maxDist = smax(dist - 2.0f * kRayEpsilon, kRayEpsilon);
+    return o;
+}
+__device__ __forceinline__ bool emissive_geometry(const DevScene& s, const Vertex& v, const Sampler& smp, uint32_t depth,
+                                                  V3* ld, V3* le, float* lp, float* nl, float* maxDist) {
+    const EmissiveSample e = emissive_sample(s, v.hit.position, v.n, v.hit.gid, smp, depth);
+    *ld = e.ld;
+    *le = e.le;
+    *lp = e.lp;
+    *nl = e.nl;
+    *maxDist = e.maxDist;
+    return !(e.maxDist < 0.0f);
 }
 
-// The emissive-triangle sample (:1578-1628); its shadow ray stops short of
-// the light (*maxDist).
-template <typename Ctr>
-__device__ __forceinline__ bool light_emissive(const DevScene& s, const DevRequest& q, const Vertex& v, const Sampler& smp,
-                                               uint32_t depth, V3* dir, V3* c, float* maxDist, Ctr& ctr) {
-    V3 ld, le;
-    float lp, nl;
-    if (!emissive_geometry(s, v, smp, depth, &ld, &le, &lp, &nl, maxDist)) return false;
-    const Mat& m = s.materials[v.hit.material];
-    ctr.bsdf_pdf();
-    ctr.bsdf_eval();
-    const float4* rec = bsdf_rec(s, v.hit.material);
-    const float bp = bsdf_pdf_rec(rec, m, v.w, v.n, v.cn, v.view, ld);
-    const float mis = power_heuristic(lp, bp);
-    *dir = ld;
-    *c = clamp24(q, bsdf_eval_rec(rec, m, v.n, v.cn, v.view, ld) * le * (nl * mis / lp));
-    return true;
-}
-
-// Light sample k of a vertex, in sum_direct's order; *maxDist is the reach
-// of its shadow ray.
+// Light sample k of a vertex, in sum_direct's order: a distant light
+// (:1529-1540), a dome sample (:1542-1573) or the emissive triangle
+// (:1578-1628).  False when the light is below the horizon or the sample
+// fails; otherwise the direction, the clamped contribution if unoccluded and
+// the reach of the shadow ray (*maxDist).  The kinds share one evaluation of
+// the BSDF (and, but for distant lights, its pdf for the MIS weight).
 template <bool kExt, typename Ctr>
 __device__ __forceinline__ bool light_sample(const DevScene& s, const DevRequest& q, const Vertex& v, const Sampler& smp,
                                              uint32_t depth, uint32_t k, V3* dir, V3* c, float* maxDist, Ctr& ctr) {
     *maxDist = FLT_MAX;
-    if (k < s.distantCount) return light_distant(s, q, v, k, dir, c, ctr);
+    V3 ld, lr;
+    float lp = 0.0f, nl;
+    const bool mis = k >= s.distantCount;
     const uint32_t r = k - s.distantCount;
-    if constexpr (kExt) {
-        if (r >= s.domeCount * q.domeSamples) return light_emissive(s, q, v, smp, depth, dir, c, maxDist, ctr);
+    if (!mis) {
+        const DevDistant l = s.distant[k];
+        ld = l.toLight;
+        lr = l.radiance;
+        nl = sclamp(dot(v.n, ld), 0.0f, 1.0f);
+        if (nl <= 0.0f) return false;
+    } else if (kExt && r >= s.domeCount * q.domeSamples) {
+        if (!emissive_geometry(s, v, smp, depth, &ld, &lr, &lp, &nl, maxDist)) return false;
+    } else {
+        const uint32_t li = r / q.domeSamples, j = r - li * q.domeSamples;
+        const uint32_t dim = kDirectDimBase + depth * kDirectDepthStride + li * kDirectLightStride + j * kDirectSampleStride;
+        if (s.domes[li].env >= 0) {
+            ctr.env_sample();
+            ctr.env_eval();
+        }
+        const bool useCdf = (q.flags & SHIRO_RENDER_ENV_CDF) != 0u;
+        if (!sample_dome(s, s.domes[li], smp.next2d(dim), useCdf, &ld, &lr, &lp) || lp <= 0.0f) return false;
+        nl = sclamp(dot(v.n, ld), 0.0f, 1.0f);
+        if (nl <= 0.0f) return false;
     }
-    const uint32_t li = r / q.domeSamples, j = r - li * q.domeSamples;
-    return light_dome(s, q, v, smp, depth, li, j, dir, c, ctr);
+    ctr.bsdf_eval();
+    if (mis) ctr.bsdf_pdf();
+    const float4 e = bsdf_eval_pdf_rec(bsdf_rec(s, v.hit.material), s.materials[v.hit.material], v.n, v.cn, v.view, ld, mis);
+    const float w = mis ? nl * power_heuristic(lp, e.w) / lp : nl;
+    *dir = ld;
+    *c = clamp24(q, f4xyz(e) * lr * w);
+    return true;
 }
 
 // MIS weight of an environment hit after a non-delta bounce (:1679-1688).
@@ -401,6 +384,60 @@ __device__ __forceinline__ void toggle_medium(const Mat& m, PathState& ps) {
     }
 }
 
+// The transmission lobe (:1811-1925): a thin-walled pane, a smooth or a rough
+// dielectric.  tr: the roughness it is sampled with, tp its selection
+// probability.  Out of line and by value: few hits take it, and inlined it
+// pushed the other lobes out of the instruction cache.
+constexpr uint32_t kTransmitDelta = 1u, kTransmitTir = 2u, kTransmitMedium = 4u;
+struct TransmitSample {
+    V3 next, f;
+    float pdf;
+    uint32_t bits;  // kTransmit*
+};
+static __device__ __noinline__ TransmitSample transmit(const Mat& m, const V3 ngf, const V3 cn, const V3 view, const V3 rd,
+                                                       const V2 ds, float tr, bool inside, float tp) {
+    TransmitSample o;
+    o.f = V3{0.0f, 0.0f, 0.0f};
+    o.pdf = 1.0f;
+    const float mt = sclamp(m.transmission, 0.0f, 1.0f) * (1.0f - sclamp(m.metallic, 0.0f, 1.0f));
+    if (m.thin_walled) {
+        o.next = rd;
+        const float refl = fresnel_dielectric(fabsf(dot(ngf, view)), 1.0f, smax(m.ior, 1.0f));
+        const float pane = thin_pane_transmittance(refl);
+        const V3 scale = transmission_surface_tint(m) * coat_transmission_scale(m, cn, view, o.next) * mt;
+        const float ac = smax(fabsf(dot(ngf, o.next)), 1.0e-4f);
+        o.f = scale * pane / ac;
+        o.pdf = tp;
+        o.bits = kTransmitDelta;
+        return o;
+    }
+    const float etaI = inside ? smax(m.ior, 1.0f) : 1.0f;
+    const float etaT = inside ? 1.0f : smax(m.ior, 1.0f);
+    const float ratio = etaI / etaT;
+    const float rel = etaT / smax(etaI, 1.0f);
+    const V3 mn0 = tr <= kDeltaRoughness ? ngf : ggx_half(ngf, ds, tr);
+    const V3 mn = dot(mn0, view) < 0.0f && tr > kDeltaRoughness ? mn0 * -1.0f : mn0;
+    o.bits = tr <= kDeltaRoughness ? kTransmitDelta : 0u;
+    if (!refract_dir(rd, mn, ratio, &o.next)) {
+        o.next = normalize(reflect(rd, mn));
+        o.bits |= kTransmitTir;
+        return o;
+    }
+    o.bits |= kTransmitMedium;
+    if (tr <= kDeltaRoughness) {
+        const float refl = fresnel_dielectric(fabsf(dot(ngf, view)), etaI, etaT);
+        const V3 scale = transmission_surface_tint(m) * coat_transmission_scale(m, cn, view, o.next) * mt;
+        const float ac = smax(fabsf(dot(ngf, o.next)), 1.0e-4f);
+        const float transport = 1.0f / smax(rel * rel, 1.0e-6f);
+        o.f = scale * (1.0f - refl) * transport / ac;
+        o.pdf = tp;
+    } else {
+        o.f = transmission_lobe(m, ngf, cn, view, o.next, etaI, etaT, tr);
+        o.pdf = smax(tp * transmission_pdf(ngf, view, o.next, etaT / etaI, tr), 1.0e-6f);
+    }
+    return o;
+}
+
 // Lobe choice (transmission first, then diffuse / base specular / coat),
 // direction sampling, throughput update and Russian roulette (:1746-2013).
 // Returns false when the path ends at this vertex.
@@ -412,7 +449,8 @@ __device__ __forceinline__ bool continue_path(const DevScene& s, const DevReques
     const float4* rec = bsdf_rec(s, v.hit.material);
     const float dw = v.w.diffuse, cw = v.w.coat;
     float bw = v.w.spec;
-    const float rawTw = kExt ? transmission_weight(m) : 0.0f;
+    const float4 r7 = rec[7];
+    const float rawTw = kExt ? r7.w : 0.0f;
     float tw = rawTw;
     if (kExt && rawTw > 0.0f) {
         const float etaI = ps.inside ? smax(m.ior, 1.0f) : 1.0f;
@@ -432,7 +470,8 @@ __device__ __forceinline__ bool continue_path(const DevScene& s, const DevReques
     uint32_t type = kBounceDiffuse;
     bool delta = false;
     bool chooseT = false, chooseC = false;
-    bool reflEval = true;  // f is the reflection BSDF at `next`
+    bool reflEval = true;   // f is the reflection BSDF at `next`
+    bool reflPdf = false;   // and pdf its sampling pdf there
     if (kExt && sel < tw) {
         chooseT = true;
     } else {
@@ -443,67 +482,32 @@ __device__ __forceinline__ bool continue_path(const DevScene& s, const DevReques
     if (kExt && chooseT) {  // :1811-1925
         if (ps.specDepth >= q.specularDepth) return false;
         ++ps.specDepth;
-        type = kBounceTransmission;
-        const float tp = smax(tw / total, 1.0e-6f);
-        const float tr =
-            m.thin_walled ? 0.0f : roughness_for(transmission_roughness(m), m.specular_anisotropy, m.specular_rotation);
-        const float mt = sclamp(m.transmission, 0.0f, 1.0f) * (1.0f - sclamp(m.metallic, 0.0f, 1.0f));
-        if (m.thin_walled) {
-            next = ps.rd;
-            const float refl = fresnel_dielectric(fabsf(dot(v.ngf, v.view)), 1.0f, smax(m.ior, 1.0f));
-            const float pane = thin_pane_transmittance(refl);
-            const V3 scale = transmission_surface_tint(m) * coat_transmission_scale(m, v.cn, v.view, next) * mt;
-            const float ac = smax(fabsf(dot(v.ngf, next)), 1.0e-4f);
-            f = scale * pane / ac;
-            pdf = tp;
-            delta = true;
-            reflEval = false;
+        const TransmitSample t = transmit(m, v.ngf, v.cn, v.view, ps.rd, ds, m.thin_walled ? 0.0f : r7.z, ps.inside,
+                                          smax(tw / total, 1.0e-6f));
+        next = t.next;
+        delta = (t.bits & kTransmitDelta) != 0u;
+        if (t.bits & kTransmitTir) {  // total internal reflection: the reflection lobes take the path
+            if (rw <= 0.0f) return false;
+            reflPdf = true;
+            type = kBounceReflective;
+            chooseT = false;
         } else {
-            const float etaI = ps.inside ? smax(m.ior, 1.0f) : 1.0f;
-            const float etaT = ps.inside ? 1.0f : smax(m.ior, 1.0f);
-            const float ratio = etaI / etaT;
-            const float rel = etaT / smax(etaI, 1.0f);
-            const float refl = fresnel_dielectric(fabsf(dot(v.ngf, v.view)), etaI, etaT);
-            const V3 mn0 = tr <= kDeltaRoughness ? v.ngf : ggx_half(v.ngf, ds, tr);
-            const V3 mn = dot(mn0, v.view) < 0.0f && tr > kDeltaRoughness ? mn0 * -1.0f : mn0;
-            if (!refract_dir(ps.rd, mn, ratio, &next)) {
-                // total internal reflection: the reflection lobes take the path
-                next = normalize(reflect(ps.rd, mn));
-                if (rw <= 0.0f) return false;
-                ctr.bsdf_pdf();
-                pdf = smax((rw / total) * bsdf_pdf_rec(rec, m, v.w, v.n, v.cn, v.view, next), 1.0e-6f);
-                type = kBounceReflective;
-                delta = tr <= kDeltaRoughness;
-                chooseT = false;
-            } else if (tr <= kDeltaRoughness) {
-                const V3 scale = transmission_surface_tint(m) * coat_transmission_scale(m, v.cn, v.view, next) * mt;
-                const float ac = smax(fabsf(dot(v.ngf, next)), 1.0e-4f);
-                const float transport = 1.0f / smax(rel * rel, 1.0e-6f);
-                f = scale * (1.0f - refl) * transport / ac;
-                pdf = tp;
-                toggle_medium(m, ps);
-                delta = true;
-                reflEval = false;
-            } else {
-                f = transmission_lobe(m, v.ngf, v.cn, v.view, next, etaI, etaT, tr);
-                pdf = smax(tp * transmission_pdf(v.ngf, v.view, next, etaT / etaI, tr), 1.0e-6f);
-                toggle_medium(m, ps);
-                delta = tr <= kDeltaRoughness;
-                reflEval = false;
-            }
+            type = kBounceTransmission;
+            f = t.f;
+            pdf = t.pdf;
+            if (t.bits & kTransmitMedium) toggle_medium(m, ps);
+            reflEval = false;
         }
     } else if (type == kBounceReflective) {  // base specular or coat
         if (ps.specDepth >= q.specularDepth) return false;
         ++ps.specDepth;
         const V3 sn = chooseC ? v.cn : v.n;
-        const float sr = chooseC ? roughness_for(m.coat_roughness, m.coat_anisotropy, m.coat_rotation)
-                                 : roughness_for(base_roughness(m), m.specular_anisotropy, m.specular_rotation);
+        const float sr = chooseC ? r7.y : r7.x;
         const V3 hv = ggx_half(sn, ds, sr);
         next = normalize(reflect(ps.rd, hv));
         const float rc = sclamp(dot(sn, next), 0.0f, 1.0f);
         if (rc <= 0.0f) return false;
-        ctr.bsdf_pdf();
-        pdf = smax((rw / total) * bsdf_pdf_rec(rec, m, v.w, v.n, v.cn, v.view, next), 1.0e-6f);
+        reflPdf = true;
         delta = sr <= kDeltaRoughness;
     } else {  // diffuse
         if (ps.diffDepth >= q.diffuseDepth) return false;
@@ -516,7 +520,10 @@ __device__ __forceinline__ bool continue_path(const DevScene& s, const DevReques
     // chose different lobes runs the BSDF once
     if (reflEval) {
         ctr.bsdf_eval();
-        f = bsdf_eval_rec(rec, m, v.n, v.cn, v.view, next);
+        if (reflPdf) ctr.bsdf_pdf();
+        const float4 e = bsdf_eval_pdf_rec(rec, m, v.n, v.cn, v.view, next, reflPdf);
+        f = f4xyz(e);
+        if (reflPdf) pdf = smax((rw / total) * e.w, 1.0e-6f);
     }
     const float cosT = chooseT ? smax(fabsf(dot(v.ngf, next)), 1.0e-4f) : sclamp(dot(v.n, next), 0.0f, 1.0f);
     if (cosT <= 0.0f) return false;
@@ -558,7 +565,7 @@ __device__ __forceinline__ PathResult trace_path(const DevScene& s, const DevReq
     res.albedo = V3{0.0f, 0.0f, 0.0f};
     res.normal = V3{0.0f, 0.0f, 0.0f};
     res.depth = __int_as_float(0x7f800000);  // +inf
-    const Sampler smp{x, y, sampleIndex};
+    const Sampler smp{x, y, sampleIndex, s.radical};
     PathState ps;
     init_path(q, smp, ps);
     for (uint32_t depth = 0; depth < q.maxDepth; ++depth) {

@@ -40,7 +40,9 @@ void launch_env_pick(const DevEnv& e, const float2* u, uint32_t n, bool useCdf, 
 cudaError_t preload_plain_kernels();
 // out[2k], out[2k+1] = Sampler{px, py, index}.next2d(branch) of tuple k
 // (tuples packed as uint4 px, py, index, branch).
-void launch_sample_probe(const uint4* tuples, uint32_t n, float* out, cudaStream_t stream);
+void launch_sample_probe(const uint4* tuples, uint32_t n, const float* table, float* out, cudaStream_t stream);
+// Fills a table of 24 x kQmcTable radical inverses (sampler.cuh).
+void launch_qmc_table(float* table, cudaStream_t stream);
 void launch_primary_hits(const DevScene& s, const DevRequest& q, uint32_t* prim, float* t, cudaStream_t stream);
 // Work counts of every stride-th path (12 totals, see ShiroWorkCounts).
 void launch_count_paths(const DevScene& s, const DevRequest& q, uint32_t stride, unsigned long long* totals,

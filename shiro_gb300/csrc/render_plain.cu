@@ -74,7 +74,7 @@ __global__ void k_primary_hits(const DevScene s, const DevRequest q, uint32_t* _
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= q.width * q.height) return;
     const uint32_t y = i / q.width, x = i - y * q.width;
-    const Sampler smp{x, y, q.sampleStart};
+    const Sampler smp{x, y, q.sampleStart, s.radical};
     V3 o, d;
     camera_ray(q, x, y, smp.next2d(0u), &o, &d);
     HitRec h;
@@ -125,12 +125,18 @@ __global__ void __launch_bounds__(128) k_count_paths(const DevScene s, const Dev
     }
 }
 
+__global__ void k_qmc_table(float* __restrict__ table) {
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < 24u * kQmcTable) table[e] = qmc_radical_dim(e / kQmcTable, e % kQmcTable);
+}
+
 // The sampler of the kernels on explicit tuples (diagnostic).
-__global__ void k_sample_probe(const uint4* __restrict__ tuples, uint32_t n, float* __restrict__ out) {
+__global__ void k_sample_probe(const uint4* __restrict__ tuples, uint32_t n, const float* __restrict__ table,
+                               float* __restrict__ out) {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint4 t = tuples[k];
-    const V2 v = Sampler{t.x, t.y, t.z}.next2d(t.w);
+    const V2 v = Sampler{t.x, t.y, t.z, table}.next2d(t.w);
     out[2 * static_cast<size_t>(k)] = v.x;
     out[2 * static_cast<size_t>(k) + 1] = v.y;
 }
@@ -174,9 +180,13 @@ inline unsigned grid(uint64_t n, unsigned b) { return static_cast<unsigned>((n +
 
 }  // namespace
 
-void launch_sample_probe(const uint4* tuples, uint32_t n, float* out, cudaStream_t stream) {
+void launch_sample_probe(const uint4* tuples, uint32_t n, const float* table, float* out, cudaStream_t stream) {
     if (n == 0) return;
-    k_sample_probe<<<grid(n, 256), 256, 0, stream>>>(tuples, n, out);
+    k_sample_probe<<<grid(n, 256), 256, 0, stream>>>(tuples, n, table, out);
+}
+
+void launch_qmc_table(float* table, cudaStream_t stream) {
+    k_qmc_table<<<grid(24u * kQmcTable, 256), 256, 0, stream>>>(table);
 }
 
 void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBase, uint32_t count, float4* records,

@@ -70,13 +70,26 @@ static __device__ __noinline__ float qmc_radical_dim(uint32_t dim, uint32_t i) {
     return acc;
 }
 
-__device__ __forceinline__ float qmc_dim(uint32_t px, uint32_t py, uint32_t index, uint32_t dim) {  // :56-71
+// The radical inverses of the first kQmcTable indices in every base, built
+// once per context (k_qmc_table): table[k * kQmcTable + i] =
+// qmc_radical_dim(k, i).  A path draws about six dimensions per hit, and the
+// digit loop was a tenth of the hit shading's instructions; the lanes of a
+// warp shade neighbouring samples, so they read neighbouring entries.
+constexpr uint32_t kQmcTable = 4096u;
+
+__device__ __forceinline__ float qmc_radical(const float* table, uint32_t dim, uint32_t i) {
+    if (i < kQmcTable && table) return __ldg(&table[(dim % 24u) * kQmcTable + i]);
+    return qmc_radical_dim(dim, i);
+}
+
+static __device__ __noinline__ float qmc_dim(const float* table, uint32_t px, uint32_t py, uint32_t index,
+                                         uint32_t dim) {  // :56-71
     if (dim < 2u) {
         const float step = dim == 0u ? 0.7548776662466927f : 0.5698402909980532f;
         const float v = 0.5f + step * static_cast<float>(index);
         return v - floorf(v);
     }
-    const float seq = qmc_radical_dim(dim, index + 1u);
+    const float seq = qmc_radical(table, dim, index + 1u);
     const uint32_t key = px * 0x8da6b343u ^ py * 0xd8163841u ^ dim * 0xcb1ab31fu ^ 0x9e3779b9u;
     const float rot = static_cast<float>(qmc_scramble(key) & 0x00ffffffu) / 16777216.0f;
     const float v = seq + rot;
@@ -85,11 +98,12 @@ __device__ __forceinline__ float qmc_dim(uint32_t px, uint32_t py, uint32_t inde
 
 struct Sampler {
     uint32_t px, py, index;
+    const float* table;  // DevScene::radical (NULL: every inverse is computed)
     // OpenQmcSampler::Next2D / Next1D (OpenQmcSampler.cpp:110-135)
     __device__ __forceinline__ V2 next2d(uint32_t branch) const {
-        return {qmc_dim(px, py, index, branch * 2u), qmc_dim(px, py, index, branch * 2u + 1u)};
+        return {qmc_dim(table, px, py, index, branch * 2u), qmc_dim(table, px, py, index, branch * 2u + 1u)};
     }
-    __device__ __forceinline__ float next1d(uint32_t branch) const { return qmc_dim(px, py, index, branch * 2u); }
+    __device__ __forceinline__ float next1d(uint32_t branch) const { return qmc_dim(table, px, py, index, branch * 2u); }
 };
 
 }  // namespace shiro_gpu

@@ -42,7 +42,8 @@ struct DevDome {
 };
 
 struct DevDistant {
-    V3 direction, radiance;
+    V3 toLight;  // normalize(direction * -1), formed at upload
+    V3 radiance;
 };
 
 // Shading record of a triangle (make_surface): everything a hit needs past
@@ -68,6 +69,7 @@ struct DevScene {
     const DevDome* domes;
     const DevEnv* envs;
     uint32_t* error;                // device error word (kErr* bits)
+    const float* radical;           // radical inverses of small indices (sampler.cuh)
     uint32_t nodeCount;
     uint32_t triCount;
     uint32_t distantCount;

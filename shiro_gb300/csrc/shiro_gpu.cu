@@ -24,6 +24,7 @@
 #include "bsdf.cuh"
 #include "env.cuh"
 #include "kernels.h"
+#include "sampler.cuh"
 
 using namespace shiro_gpu;
 
@@ -92,6 +93,7 @@ ContextImpl::~ContextImpl() {
     free_block(&aovScratch);
     free_block(&probeScratch);
     if (errorWord) cudaFree(errorWord);
+    if (radicalTable) cudaFree(radicalTable);
     if (ownStream) cudaStreamDestroy(ownStream);
 }
 
@@ -721,6 +723,14 @@ uint64_t hash_spans(std::vector<HashSpan> spans) {
     return h;
 }
 
+// normalize(direction * -1) with the device's float operations, each rounded
+// as there.
+V3 to_light(const V3& direction) {
+    const V3 d = direction * -1.0f;
+    const float l = std::sqrt(dot(d, d));
+    return l > 0.0f ? d / l : V3{0.0f, 0.0f, 0.0f};
+}
+
 // What an upload derives from the materials, lights and environments
 // (everything but the geometry): emissive-triangle tables, materials and
 // their BSDF records, distant lights, domes with their importance tables.
@@ -803,7 +813,7 @@ int upload_shading(ContextImpl* ctx, const ShiroSceneDesc* sd) {
     if ((rc = build_bsdf_recs(ctx)) != SHIRO_OK) return rc;
     std::vector<DevDistant> distant(sd->distant_light_count);
     for (uint32_t i = 0; i < sd->distant_light_count; ++i)
-        distant[i] = DevDistant{ld3(sd->distant_lights[i].direction), ld3(sd->distant_lights[i].radiance)};
+        distant[i] = DevDistant{to_light(ld3(sd->distant_lights[i].direction)), ld3(sd->distant_lights[i].radiance)};
     if ((rc = upload(ctx, distant, &s.distant, "distant lights")) != SHIRO_OK) return rc;
     s.distantCount = sd->distant_light_count;
 
@@ -839,6 +849,7 @@ int upload_shading(ContextImpl* ctx, const ShiroSceneDesc* sd) {
 int finish_upload(ContextImpl* ctx) {
     DevScene& s = ctx->scene;
     s.error = ctx->errorWord;
+    s.radical = ctx->radicalTable;
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "scene upload");
     ctx->hasScene = true;
@@ -926,6 +937,12 @@ int shiro_gpu_create(int device, ShiroGpuContext** out) {
     e = cudaStreamCreateWithFlags(&c.ownStream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&c.errorWord, 16);
     if (e == cudaSuccess) e = cudaMemset(c.errorWord, 0, 16);
+    if (e == cudaSuccess) e = cudaMalloc(&c.radicalTable, 24u * kQmcTable * sizeof(float));
+    if (e == cudaSuccess) {
+        launch_qmc_table(c.radicalTable, c.ownStream);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c.ownStream);
     if (e != cudaSuccess) {
         gCreateError = std::string("context setup: ") + cudaGetErrorString(e);
         delete ctx;
@@ -1460,7 +1477,7 @@ int shiro_gpu_sample(ShiroGpuContext* handle, const uint32_t* px, const uint32_t
     float* dout = reinterpret_cast<float*>(dt + n);
     cudaError_t e = cudaMemcpyAsync(dt, tuples.data(), n * sizeof(uint4), cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sample probe upload");
-    launch_sample_probe(dt, n, dout, ctx->stream);
+    launch_sample_probe(dt, n, ctx->radicalTable, dout, ctx->stream);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out2, dout, n * 2 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);

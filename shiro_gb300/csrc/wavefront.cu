@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(128) wf_generate(WfView v) {
         const uint32_t pix = sg.pixelStart + local / q.sampleCount;
         const uint32_t smpIdx = q.sampleStart + (local - (local / q.sampleCount) * q.sampleCount);
         const uint32_t y = pix / q.width, x = pix - y * q.width;
-        const Sampler smp{x, y, smpIdx};
+        const Sampler smp{x, y, smpIdx, nullptr};
         PathState ps;
         init_path(q, smp, ps);
         v.ro[j] = make_float4(ps.ro.x, ps.ro.y, ps.ro.z, 0.0f);
@@ -699,7 +699,7 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
             h.gid = __float_as_uint(h4.w);
             {
                 const Vertex vx = make_vertex(s, ps.ro, ps.rd, h);
-                const Sampler smp{id.x, id.y, id.z};
+                const Sampler smp{id.x, id.y, id.z, s.radical};
                 bool anyLight = false, cont;
                 if (kExt && !enter_hit(s, smp, depth, vx, h.t, ps)) {
                     cont = depth + 1u < q.maxDepth;  // passes through an opacity cut-out
@@ -983,7 +983,7 @@ __global__ void __launch_bounds__(128) wa_generate(WfView v, AdjWave aw) {
             const uint32_t pix = sg.pixelStart + local / q.sampleCount;
             const uint32_t smpIdx = q.sampleStart + (local - (local / q.sampleCount) * q.sampleCount);
             const uint32_t y = pix / q.width, x = pix - y * q.width;
-            const Sampler smp{x, y, smpIdx};
+            const Sampler smp{x, y, smpIdx, nullptr};
             PathState ps;
             init_path(q, smp, ps);
             v.ro[j] = make_float4(ps.ro.x, ps.ro.y, ps.ro.z, 0.0f);
@@ -1058,22 +1058,24 @@ template <bool kExt>
 __device__ __forceinline__ bool wa_light(const DevScene& s, const DevRequest& q, const AdjView& a, const Vertex& vx,
                                          const Sampler& smp, uint32_t depth, uint32_t k, const float4* rec, const Mat& ms,
                                          V3* ld, V3* c, V3* gL, V3* gE, V3* local, bool* envMark) {
-    V3 L, domeRad{0.0f, 0.0f, 0.0f};
+    V3 L, f, domeRad{0.0f, 0.0f, 0.0f};
     float w;
     int32_t envIdx = -1;
     *local = V3{0.0f, 0.0f, 0.0f};
     if (kExt && k >= s.distantCount + s.domeCount * q.domeSamples) {  // the emissive-triangle sample
         float lp, nl, reach;
         if (!emissive_geometry(s, vx, smp, depth, ld, &L, &lp, &nl, &reach)) return false;
-        const float bp = bsdf_pdf_rec(rec, ms, vx.w, vx.n, vx.cn, vx.view, *ld);
-        w = nl * power_heuristic(lp, bp) / lp;
+        const float4 e = bsdf_eval_pdf_rec(rec, ms, vx.n, vx.cn, vx.view, *ld, true);
+        f = f4xyz(e);
+        w = nl * power_heuristic(lp, e.w) / lp;
     } else if (k < s.distantCount) {
         const DevDistant l = s.distant[k];
-        *ld = normalize(l.direction * -1.0f);
+        *ld = l.toLight;
         const float nl = sclamp(dot(vx.n, *ld), 0.0f, 1.0f);
         if (nl <= 0.0f) return false;
         L = l.radiance;
         w = nl;
+        f = bsdf_eval_rec(rec, ms, vx.n, vx.cn, vx.view, *ld);
     } else {
         const uint32_t r = k - s.distantCount;
         const uint32_t li = r / q.domeSamples, jj = r - li * q.domeSamples;
@@ -1098,11 +1100,11 @@ __device__ __forceinline__ bool wa_light(const DevScene& s, const DevRequest& q,
         *ld = light_to_world(d, *local);
         const float nl = sclamp(dot(vx.n, *ld), 0.0f, 1.0f);
         if (nl <= 0.0f) return false;
-        const float bp = bsdf_pdf_rec(rec, ms, vx.w, vx.n, vx.cn, vx.view, *ld);
-        const float mis = power_heuristic(lp, bp);
+        const float4 e = bsdf_eval_pdf_rec(rec, ms, vx.n, vx.cn, vx.view, *ld, true);
+        f = f4xyz(e);
+        const float mis = power_heuristic(lp, e.w);
         w = nl * mis / lp;
     }
-    const V3 f = bsdf_eval_rec(rec, ms, vx.n, vx.cn, vx.view, *ld);
     const V3 raw = f * L * w;
     *c = clamp24(q, raw);
     const float sc = clamp_scale(q, raw, kDirectSampleClamp);
@@ -1153,7 +1155,7 @@ __global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw
             aw.vtx[3 * static_cast<size_t>(j)] = make_float4(vx.n.x, vx.n.y, vx.n.z, __uint_as_float(mat));
             aw.vtx[3 * static_cast<size_t>(j) + 1] = make_float4(vx.cn.x, vx.cn.y, vx.cn.z, 0.0f);
             aw.vtx[3 * static_cast<size_t>(j) + 2] = make_float4(vx.view.x, vx.view.y, vx.view.z, 0.0f);
-            const Sampler smp{id.x, id.y, id.z};
+            const Sampler smp{id.x, id.y, id.z, s.radical};
             // an opacity cut-out the path passes through (the forward's decision;
             // no media, transmission being refused): the hit is not shaded
             const bool shaded = !kExt || enter_hit(s, smp, depth, vx, h.t, ps);
@@ -1199,8 +1201,8 @@ __global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw
                 if (tw <= 0.0f) break;
                 const float sel = smp.next1d(base + 1u) * tw;
                 const V2 ds = smp.next2d(base + 2u);
-                float pdf;
-                bool delta2 = false;
+                float pdf = 0.0f;
+                bool delta2 = false, wantPdf = false;
                 const float rs = sel - 0.0f;
                 uint32_t type = kBounceDiffuse;
                 if (rs < vx.w.diffuse) {
@@ -1215,16 +1217,18 @@ __global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw
                     if (ps.specDepth >= q.specularDepth) break;
                     ++ps.specDepth;
                     const V3 sn = coat ? vx.cn : vx.n;
-                    const float sr = coat ? roughness_for(ms.coat_roughness, ms.coat_anisotropy, ms.coat_rotation)
-                                          : roughness_for(base_roughness(ms), ms.specular_anisotropy, ms.specular_rotation);
+                    const float4 r7 = rec[7];
+                    const float sr = coat ? r7.y : r7.x;
                     const V3 hv = ggx_half(sn, ds, sr);
                     next = normalize(reflect(ps.rd, hv));
                     const float rc = sclamp(dot(sn, next), 0.0f, 1.0f);
                     if (rc <= 0.0f) break;
-                    pdf = smax((rw / tw) * bsdf_pdf_rec(rec, ms, vx.w, vx.n, vx.cn, vx.view, next), 1.0e-6f);
+                    wantPdf = true;
                     delta2 = sr <= kDeltaRoughness;
                 }
-                f = bsdf_eval_rec(rec, ms, vx.n, vx.cn, vx.view, next);
+                const float4 ev = bsdf_eval_pdf_rec(rec, ms, vx.n, vx.cn, vx.view, next, wantPdf);
+                f = f4xyz(ev);
+                if (wantPdf) pdf = smax((rw / tw) * ev.w, 1.0e-6f);
                 const float cosT = sclamp(dot(vx.n, next), 0.0f, 1.0f);
                 if (cosT <= 0.0f) break;
                 ps.T = clamp12(q, ps.T * f * (cosT / pdf));
