@@ -652,58 +652,85 @@ __device__ __forceinline__ void write_record(const WfView& v, uint32_t j, const 
 
 // Shade stage, compiled with several register caps (the autotuner picks) and
 // with / without the extended lobes (kExt, chosen by the scene).
+//
+// The lean stage (kExt = false) is bound by the latency of its path-state and
+// record loads at 20 warps per SM; its warps run independently.  With the
+// extended lobes the code a warp runs through outgrows the instruction cache:
+// with independent warps 32 of 38 stall cycles per instruction were spent on
+// fetching it.  There one block fills the SM (ext_shade_block) and its warps go
+// through the stage's phases together - vertex, each light sample,
+// continuation - so that one fetch serves them all: shading of the 640x480
+// 32-spp studio frame (glass, emitters, cut-outs, layered materials) 13.0 ->
+// 6.0 ms, the frame 19.1 -> 12.5 ms (with blocks of 128: 16.2, of 256: 14.3).
+// The lean stage gains nothing from it (field frame 96.0 against 96.7 ms).
 template <int kRegs, bool kExt>
 __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, uint32_t depth) {
     const uint32_t count = v.counters[kHitCount];
     uint32_t* qout = cur ? v.rayQ0 : v.rayQ1;
     uint32_t* cout = &v.counters[cur ^ 1u];
     NullCounter ctr;
+    __shared__ uint32_t blockBase;
+    const auto phase = [] {
+        if constexpr (kExt) __syncthreads();
+    };
+    // entries a block takes at a time: its threads', or fewer when the queue is too short to fill every block
+    const uint32_t share = min(blockDim.x, max(32u, ((count + gridDim.x - 1u) / gridDim.x + 31u) & ~31u));
     // whole warps fetch work together, so the warp-aggregated pushes below
     // always see the whole warp; entries [0, hits) of the shade queue
     for (;;) {
-        const uint32_t wbase = warp_fetch(&v.counters[kFetchShade]);
-        if (wbase >= count) break;
-        const uint32_t i = wbase + lane_id();
+        uint32_t i;
+        if constexpr (kExt) {
+            __syncthreads();
+            if (threadIdx.x == 0) blockBase = atomicAdd(&v.counters[kFetchShade], share);
+            __syncthreads();
+            if (blockBase >= count) break;
+            i = threadIdx.x < share ? blockBase + threadIdx.x : count;
+        } else {
+            const uint32_t wbase = warp_fetch(&v.counters[kFetchShade]);
+            if (wbase >= count) break;
+            i = wbase + lane_id();
+        }
         const bool valid = i < count;
-        bool pushRay = false, pushShadow = false;
+        bool pushRay = false;
         uint32_t lightMask = 0;
         uint32_t j = 0;
-        if (valid) {
-            j = v.shadeQ[i];
-            const uint4 id = v.ident[j];
+        if (kExt || valid) {  // (kExt: every thread passes the phases)
+            if (valid) j = v.shadeQ[i];
+            const uint4 id = valid ? v.ident[j] : make_uint4(0u, 0u, 0u, 0u);
             const DevRequest& q = v.reqs[id.w].q;
-            const float4 o = v.ro[j], d = v.rd[j], t4 = v.T[j], r4 = v.rad[j], h4 = v.hit[j];
-            const uint32_t bits = __float_as_uint(t4.w);
+            const Sampler smp{id.x, id.y, id.z, s.radical};
             PathState ps;
-            ps.ro = V3{o.x, o.y, o.z};
-            ps.rd = V3{d.x, d.y, d.z};
-            ps.prevPdf = d.w;
-            ps.T = V3{t4.x, t4.y, t4.z};
-            ps.radiance = V3{r4.x, r4.y, r4.z};
-            ps.diffDepth = bits & 0xffu;
-            ps.specDepth = (bits >> 8) & 0xffu;
-            ps.prevDelta = (bits & kFlagPrevDelta) != 0u;
-            ps.prevType = (bits >> kTypeShift) & 3u;
-            ps.inside = (bits & kFlagInside) != 0u;
-            ps.mediumActive = (bits & kFlagMedium) != 0u;
-            ps.extinction = V3{0.0f, 0.0f, 0.0f};
-            if (kExt && ps.mediumActive) {
-                const float4 m4 = v.medium[j];
-                ps.extinction = V3{m4.x, m4.y, m4.z};
-            }
-            float depth0 = r4.w;
-            HitRec h;
-            h.t = h4.x;
-            h.u = h4.y;
-            h.v = h4.z;
-            h.gid = __float_as_uint(h4.w);
-            {
-                const Vertex vx = make_vertex(s, ps.ro, ps.rd, h);
-                const Sampler smp{id.x, id.y, id.z, s.radical};
-                bool anyLight = false, cont;
-                if (kExt && !enter_hit(s, smp, depth, vx, h.t, ps)) {
-                    cont = depth + 1u < q.maxDepth;  // passes through an opacity cut-out
-                } else {
+            Vertex vx;
+            float depth0 = 0.0f;
+            bool shaded = false;  // false: an opacity cut-out the path passes through
+            if (valid) {
+                const float4 o = v.ro[j], d = v.rd[j], t4 = v.T[j], r4 = v.rad[j], h4 = v.hit[j];
+                const uint32_t bits = __float_as_uint(t4.w);
+                ps.ro = V3{o.x, o.y, o.z};
+                ps.rd = V3{d.x, d.y, d.z};
+                ps.prevPdf = d.w;
+                ps.T = V3{t4.x, t4.y, t4.z};
+                ps.radiance = V3{r4.x, r4.y, r4.z};
+                ps.diffDepth = bits & 0xffu;
+                ps.specDepth = (bits >> 8) & 0xffu;
+                ps.prevDelta = (bits & kFlagPrevDelta) != 0u;
+                ps.prevType = (bits >> kTypeShift) & 3u;
+                ps.inside = (bits & kFlagInside) != 0u;
+                ps.mediumActive = (bits & kFlagMedium) != 0u;
+                ps.extinction = V3{0.0f, 0.0f, 0.0f};
+                if (kExt && ps.mediumActive) {
+                    const float4 m4 = v.medium[j];
+                    ps.extinction = V3{m4.x, m4.y, m4.z};
+                }
+                depth0 = r4.w;
+                HitRec h;
+                h.t = h4.x;
+                h.u = h4.y;
+                h.v = h4.z;
+                h.gid = __float_as_uint(h4.w);
+                vx = make_vertex(s, ps.ro, ps.rd, h);
+                shaded = !kExt || enter_hit(s, smp, depth, vx, h.t, ps);
+                if (shaded) {
                     if (depth == 0) {
                         const float4 dc = __ldg(bsdf_rec(s, vx.hit.material) + 3);  // DiffuseColor
                         const V3 alb{dc.x, dc.y, dc.z};
@@ -713,26 +740,32 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
                         depth0 = h.t;
                     }
                     if constexpr (kExt) add_emission(s, vx, depth, ps);
-                    // this request's light samples (requests of a batch may differ in dome samples)
-                    const uint32_t nls = light_sample_count<kExt>(s, q);
-                    for (uint32_t k = 0; k < nls; ++k) {
-                        V3 dir{0.0f, 0.0f, 0.0f}, c{0.0f, 0.0f, 0.0f};
-                        float reach = 0.0f;
-                        const bool ok = light_sample<kExt>(s, q, vx, smp, depth, k, &dir, &c, &reach, ctr);
-                        anyLight |= ok;
-                        lightMask |= ok ? (1u << k) : 0u;
-                        const size_t e = static_cast<size_t>(k) * v.P + j;
-                        v.shDir[e] = make_float4(dir.x, dir.y, dir.z, ok ? reach : 0.0f);
-                        v.shC[e] = make_float4(c.x, c.y, c.z, 0.0f);
-                    }
-                    if (anyLight) {
-                        const V3 org = shadow_origin(vx);
-                        v.shOrigin[j] = make_float4(org.x, org.y, org.z, 0.0f);
-                        v.shT[j] = make_float4(ps.T.x, ps.T.y, ps.T.z, 0.0f);
-                        pushShadow = true;
-                    }
-                    cont = continue_path<kExt>(s, q, vx, smp, depth, ps, ctr) && depth + 1u < q.maxDepth;
                 }
+            }
+            phase();
+            // this request's light samples (requests of a batch may differ in dome samples)
+            const uint32_t nls = shaded ? light_sample_count<kExt>(s, q) : 0u;
+            for (uint32_t k = 0; k < (kExt ? v.lightSamples : nls); ++k) {
+                if (!kExt || k < nls) {
+                    V3 dir{0.0f, 0.0f, 0.0f}, c{0.0f, 0.0f, 0.0f};
+                    float reach = 0.0f;
+                    const bool ok = light_sample<kExt>(s, q, vx, smp, depth, k, &dir, &c, &reach, ctr);
+                    lightMask |= ok ? (1u << k) : 0u;
+                    const size_t e = static_cast<size_t>(k) * v.P + j;
+                    v.shDir[e] = make_float4(dir.x, dir.y, dir.z, ok ? reach : 0.0f);
+                    v.shC[e] = make_float4(c.x, c.y, c.z, 0.0f);
+                }
+                phase();
+            }
+            if (valid) {
+                const bool anyLight = lightMask != 0u;
+                if (anyLight) {
+                    const V3 org = shadow_origin(vx);
+                    v.shOrigin[j] = make_float4(org.x, org.y, org.z, 0.0f);
+                    v.shT[j] = make_float4(ps.T.x, ps.T.y, ps.T.z, 0.0f);
+                }
+                const bool cont =
+                    (!shaded || continue_path<kExt>(s, q, vx, smp, depth, ps, ctr)) && depth + 1u < q.maxDepth;
                 if (v.visLog && !anyLight) v.visLog[static_cast<size_t>(depth) * v.P + j] = 0u;
                 uint32_t nb = pack_state(ps);
                 if (!cont && anyLight) {
@@ -752,10 +785,14 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
             }
         }
         warp_push(cout, qout, pushRay, j);
-        warp_push(&v.counters[2], v.shadowQ, pushShadow, j);
+        warp_push(&v.counters[2], v.shadowQ, lightMask != 0u, j);
         warp_push_samples(&v.counters[4], v.shadowRayQ, lightMask, v.lightSamples, j);
     }
 }
+
+// Threads of the extended shade stage's blocks: as many as the register cap
+// lets one SM hold in a block (one block per SM).
+constexpr int ext_shade_block(uint32_t regs) { return regs == 80 ? 768 : regs == 96 ? 640 : 512; }
 
 // Miss shading (the environment and its MIS weight), one queued miss per
 // thread: entries [P - misses, P) of the shade queue.  A kernel of its own so
@@ -1835,6 +1872,7 @@ int run_waves(ContextImpl* ctx, WavefrontState* wf, const ShiroWavefrontConfig& 
                                 [&](auto kern) { return grid_for(kern, L.bExt, wf->smCount); });
     L.shadeRegs = cfg.shade_regs;
     L.ext = ctx->extendedMaterials;
+    if (L.ext) L.bShade = ext_shade_block(L.shadeRegs);
     L.gShade = with_shade_kernel(L.shadeRegs, L.ext, [&](auto kern) { return grid_for(kern, L.bShade, wf->smCount); });
     L.v.travSteps = static_cast<int>(cfg.extend_steps ? cfg.extend_steps : 4);
     L.v.refillIdle = static_cast<int>(cfg.refill_idle ? cfg.refill_idle : 8);
