@@ -17,7 +17,7 @@
 //   * a continuation BSDF value f_k scales every later contribution, which
 //     is the radiance not yet accounted for, L_rem: delta * L_rem * df_k / f_k;
 //   * a miss adds delta * T * mis * dL_env.
-// BSDF derivatives come from bsdf_eval_d (forward-mode dual numbers).
+// BSDF derivatives come from bsdf_grad (bsdf_diff.cuh).
 //
 // shiro_gpu_render_frozen evaluates the same estimator with the sampling
 // taken from the scene's parameters and the BSDF / environment values from a
@@ -171,8 +171,7 @@ __device__ __noinline__ V3 adj_path(const DevScene& s, const DevRequest& q, cons
             }
             if (kGrad) {
                 const float sc = clamp_scale(q, raw, kDirectSampleClamp);
-                const DV3 fd = bsdf_eval_d(me, v.n, v.cn, v.view, ld);
-                add_mat_grad(a, v.hit.material, fd, dT * L * (w * sc));
+                add_mat_grad(a, v.hit.material, bsdf_grad(me, v.n, v.cn, v.view, ld, dT * L * (w * sc)));
                 if (envIdx >= 0 && envIdx == a.env0) add_env_grad(a, a.evalEnv, local, dT * f * domeRad * (w * sc));
             }
             return true;
@@ -243,10 +242,9 @@ __device__ __noinline__ V3 adj_path(const DevScene& s, const DevRequest& q, cons
         }
         if (kGrad && alive && depth + 1u < q.maxDepth) {
             // every later contribution scales with f (per channel)
-            const DV3 fd = bsdf_eval_d(me, v.n, v.cn, v.view, next);
             const V3 coef{f.x > 0.0f ? delta.x * Lrem.x / f.x : 0.0f, f.y > 0.0f ? delta.y * Lrem.y / f.y : 0.0f,
                           f.z > 0.0f ? delta.z * Lrem.z / f.z : 0.0f};
-            add_mat_grad(a, v.hit.material, fd, coef);
+            add_mat_grad(a, v.hit.material, bsdf_grad(me, v.n, v.cn, v.view, next, coef));
         }
         (void)prevDir;
         if (!alive) break;

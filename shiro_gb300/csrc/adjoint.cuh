@@ -117,20 +117,35 @@ __device__ __forceinline__ void add_env_grad(const AdjView& a, const DevEnv& e, 
     }
 }
 
-// dL/dparams of material `mat` += sum_c coef_c * df_c (df from the duals).
-// The lanes on one material sum first and add once.
-__device__ __forceinline__ void add_mat_grad(const AdjView& a, uint32_t mat, const DV3& f, const V3& coef) {
-    float g[kDualN];
-#pragma unroll
-    for (int p = 0; p < kDualN; ++p) g[p] = coef.x * f.x.d[p] + coef.y * f.y.d[p] + coef.z * f.z.d[p];
+// The same for a sample of a texture with an importance table: samples of one
+// texel share its direction, so the lanes that drew it sum their coefficients
+// and only the group's first lane forms the footprint.
+__device__ __forceinline__ void add_env_grad_texel(const AdjView& a, const DevEnv& e, const V3& local, uint32_t texel,
+                                                   const V3& coef) {
+    if (!a.dEnv4) return;
+    float g[3] = {coef.x, coef.y, coef.z};
+    const bool any = coef.x != 0.0f || coef.y != 0.0f || coef.z != 0.0f;
+    const uint32_t key = any ? texel : 0xffffffffu;
+    if (!group_sum(__activemask(), key, g) || key == 0xffffffffu) return;
+    uint32_t idx[4];
+    float w[4];
+    const int n = env_footprint(e, local, idx, w);
+    for (int k = 0; k < n; ++k)
+        if (w[k] != 0.0f) atomicAdd(&a.dEnv4[idx[k]], make_float4(g[0] * w[k], g[1] * w[k], g[2] * w[k], 0.0f));
+}
+
+// dL/dparams of material `mat` += grad.  The lanes on one material sum first
+// and add once.
+__device__ __forceinline__ void add_mat_grad(const AdjView& a, uint32_t mat, const MatGrad& grad) {
+    float g[5] = {grad.base[0], grad.base[1], grad.base[2], grad.rough, grad.metal};
     const uint32_t key = mat < a.materialCount ? mat : 0xffffffffu;
     if (!group_sum(__activemask(), key, g) || key == 0xffffffffu) return;
     if (a.dBase) {
         for (int c = 0; c < 3; ++c)
             if (g[c] != 0.0f) atomicAdd(&a.dBase[3 * mat + c], g[c]);
     }
-    if (a.dRough && g[kDRough] != 0.0f) atomicAdd(&a.dRough[mat], g[kDRough]);
-    if (a.dMetal && g[kDMetal] != 0.0f) atomicAdd(&a.dMetal[mat], g[kDMetal]);
+    if (a.dRough && g[3] != 0.0f) atomicAdd(&a.dRough[mat], g[3]);
+    if (a.dMetal && g[4] != 0.0f) atomicAdd(&a.dMetal[mat], g[4]);
 }
 
 __device__ __forceinline__ float clamp_scale(const DevRequest& q, const V3& v, float mx) {

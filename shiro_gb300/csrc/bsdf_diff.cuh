@@ -1,298 +1,146 @@
-// bsdf_diff.cuh - EvaluateBsdf with forward-mode derivatives.
+// bsdf_diff.cuh - material gradients of EvaluateBsdf.
 //
-// bsdf_eval_d restates EvaluateBsdf (src/backend/cpu/CpuPathTracer.cpp:
-// 1275-1354) on dual numbers carrying the derivatives with respect to the
-// differentiable material parameters: base colour (r, g, b), specular
-// roughness and metalness.  The value part performs the same float
-// operations in the same order as bsdf_eval (bsdf.cuh), so value(f) equals
-// the forward BSDF bit for bit; clamps and max/min propagate the derivative
-// of the branch they select (zero when a bound is selected).
+// bsdf_grad differentiates EvaluateBsdf (src/backend/cpu/CpuPathTracer.cpp:
+// 1275-1354) with respect to the differentiable material parameters - base
+// colour (r, g, b), specular roughness and metalness - and contracts the
+// derivative with the caller's coefficient per colour channel.  Clamps and
+// max / min propagate the derivative of the branch they select (zero when a
+// bound is selected); the coat lobe, the tints and the cosines depend on none
+// of the parameters.
+//
+// A channel of the BSDF depends on its own channel of the base colour only,
+// the GGX terms on the roughness only, Fresnel terms and diffuse colour on
+// base colour and metalness only, so three derivatives per quantity at most
+// are carried (dual numbers with all five spent most of their operations on
+// zeros).
 #pragma once
 
 #include "bsdf.cuh"
 
 namespace shiro_gpu {
 
-constexpr int kDualN = 5;  // d/d base_r, base_g, base_b, roughness, metallic
-constexpr int kDRough = 3, kDMetal = 4;
-
-struct Dual {
-    float v;
-    float d[kDualN];
+// d(coef . f) / d parameters.
+struct MatGrad {
+    float base[3], rough, metal;
 };
 
-__device__ __forceinline__ Dual dconst(float v) {
-    Dual r;
-    r.v = v;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = 0.0f;
-    return r;
-}
-__device__ __forceinline__ Dual dvar(float v, int i) {
-    Dual r = dconst(v);
-    r.d[i] = 1.0f;
-    return r;
-}
-__device__ __forceinline__ Dual operator+(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v + b.v;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = a.d[i] + b.d[i];
-    return r;
-}
-__device__ __forceinline__ Dual operator+(const Dual& a, float b) {
-    Dual r = a;
-    r.v = a.v + b;
-    return r;
-}
-__device__ __forceinline__ Dual operator+(float a, const Dual& b) {
-    Dual r = b;
-    r.v = a + b.v;
-    return r;
-}
-__device__ __forceinline__ Dual operator-(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v - b.v;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = a.d[i] - b.d[i];
-    return r;
-}
-__device__ __forceinline__ Dual operator-(float a, const Dual& b) {
-    Dual r;
-    r.v = a - b.v;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = -b.d[i];
-    return r;
-}
-__device__ __forceinline__ Dual operator-(const Dual& a, float b) {
-    Dual r = a;
-    r.v = a.v - b;
-    return r;
-}
-__device__ __forceinline__ Dual operator*(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v * b.v;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = a.d[i] * b.v + a.v * b.d[i];
-    return r;
-}
-__device__ __forceinline__ Dual operator*(const Dual& a, float b) {
-    Dual r;
-    r.v = a.v * b;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = a.d[i] * b;
-    return r;
-}
-__device__ __forceinline__ Dual operator*(float a, const Dual& b) {
-    Dual r;
-    r.v = a * b.v;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = a * b.d[i];
-    return r;
-}
-__device__ __forceinline__ Dual operator/(const Dual& a, const Dual& b) {
-    Dual r;
-    r.v = a.v / b.v;
-    const float inv2 = 1.0f / (b.v * b.v);
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = (a.d[i] * b.v - a.v * b.d[i]) * inv2;
-    return r;
-}
-__device__ __forceinline__ Dual operator/(const Dual& a, float b) {
-    Dual r;
-    r.v = a.v / b;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = a.d[i] / b;
-    return r;
-}
-__device__ __forceinline__ Dual operator/(float a, const Dual& b) {
-    Dual r;
-    r.v = a / b.v;
-    const float k = -a / (b.v * b.v);
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = k * b.d[i];
-    return r;
-}
-__device__ __forceinline__ Dual dsqrt(const Dual& a) {
-    Dual r;
-    r.v = sqrtf(a.v);
-    const float k = r.v > 0.0f ? 0.5f / r.v : 0.0f;
-#pragma unroll
-    for (int i = 0; i < kDualN; ++i) r.d[i] = k * a.d[i];
-    return r;
-}
-// std::max / std::min / std::clamp: the derivative follows the selected value.
-__device__ __forceinline__ Dual dmax(float a, const Dual& b) { return a < b.v ? b : dconst(a); }
-__device__ __forceinline__ Dual dclamp(const Dual& x, float lo, float hi) {
-    if (x.v < lo) return dconst(lo);
-    if (hi < x.v) return dconst(hi);
-    return x;
-}
-
-struct DV3 {
-    Dual x, y, z;
+// A quantity of one channel: value and derivatives by base colour channel
+// and metalness.
+struct DualBM {
+    float v, b, m;
 };
-__device__ __forceinline__ DV3 dv3(const V3& v) { return {dconst(v.x), dconst(v.y), dconst(v.z)}; }
-__device__ __forceinline__ DV3 operator+(const DV3& a, const DV3& b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ DV3 operator*(const DV3& a, const DV3& b) { return {a.x * b.x, a.y * b.y, a.z * b.z}; }
-__device__ __forceinline__ DV3 operator*(const DV3& a, const V3& b) { return {a.x * b.x, a.y * b.y, a.z * b.z}; }
-__device__ __forceinline__ DV3 operator*(const V3& a, const DV3& b) { return {a.x * b.x, a.y * b.y, a.z * b.z}; }
-__device__ __forceinline__ DV3 operator*(const DV3& a, const Dual& s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ DV3 operator*(const DV3& a, float s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ DV3 operator*(const V3& a, const Dual& s) { return {a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ V3 dval(const DV3& a) { return {a.x.v, a.y.v, a.z.v}; }
-
-// lerp(a, b, t) = a * (1 - t) + b * t with dual b and t (spec_f0's metal lerp).
-__device__ __forceinline__ DV3 dlerp(const V3& a, const DV3& b, const Dual& t) {
-    const Dual omt = 1.0f - t;
-    return {a.x * omt + b.x * t, a.y * omt + b.y * t, a.z * omt + b.z * t};
-}
-__device__ __forceinline__ DV3 dlerp(const DV3& a, const V3& b, float t) {
-    return {a.x * (1.0f - t) + b.x * t, a.y * (1.0f - t) + b.y * t, a.z * (1.0f - t) + b.z * t};
-}
-__device__ __forceinline__ DV3 dlerp(const DV3& a, const DV3& b, float t) {
-    return {a.x * (1.0f - t) + b.x * t, a.y * (1.0f - t) + b.y * t, a.z * (1.0f - t) + b.z * t};
-}
-
-// Differentiable material parameters of one material.
-struct MatParams {
-    DV3 base;
-    Dual rough;  // m.roughness
-    Dual metal;  // sclamp(m.metallic, 0, 1)
+// A quantity of the roughness alone.
+struct DualR {
+    float v, r;
 };
 
-__device__ __forceinline__ MatParams mat_params(const Mat& m) {
-    MatParams p;
-    p.base = DV3{dvar(m.base_color[0], 0), dvar(m.base_color[1], 1), dvar(m.base_color[2], 2)};
-    p.rough = dvar(m.roughness, kDRough);
-    p.metal = dclamp(dvar(m.metallic, kDMetal), 0.0f, 1.0f);
-    return p;
+__device__ __forceinline__ DualBM operator+(const DualBM& a, const DualBM& b) { return {a.v + b.v, a.b + b.b, a.m + b.m}; }
+__device__ __forceinline__ DualBM operator*(const DualBM& a, float s) { return {a.v * s, a.b * s, a.m * s}; }
+__device__ __forceinline__ DualBM operator*(const DualBM& a, const DualBM& b) {
+    return {a.v * b.v, a.b * b.v + a.v * b.b, a.m * b.v + a.v * b.m};
 }
 
-__device__ __forceinline__ DV3 diffuse_color_d(const Mat& m, const MatParams& p) {
-    const float trans = sclamp(m.transmission, 0.0f, 1.0f);
-    const float sss = sclamp(m.subsurface, 0.0f, 1.0f);
-    const float blend = sclamp(maxc(ld3(m.subsurface_radius)) / 3.0f, 0.0f, 1.0f);
-    const DV3 tint = dlerp(p.base, ld3(m.subsurface_color), blend);
-    const DV3 base = dlerp(p.base, tint, sss);
-    return base * (sclamp(m.base_weight, 0.0f, 1.0f) * (1.0f - p.metal) * (1.0f - trans));
+__device__ __forceinline__ float schlick_weight(float x) {  // (1 - x)^5 of a clamped cosine
+    const float c = sclamp(1.0f - x, 0.0f, 1.0f);
+    return c * c * c * c * c;
 }
-__device__ __forceinline__ DV3 spec_f0_d(const Mat& m, const MatParams& p) {
-    const V3 d = ld3(m.specular_color) * (sclamp(m.specular_weight, 0.0f, 1.0f) * f0_dielectric(m.ior));
-    return dlerp(d, p.base, p.metal);
+// f0 + (1 - f0) f
+__device__ __forceinline__ DualBM schlick_d(const DualBM& f0, float f) {
+    return {f0.v + (1.0f - f0.v) * f, f0.b - f0.b * f, f0.m - f0.m * f};
 }
-__device__ __forceinline__ Dual one_minus_clamped1(const Dual& v) { return dclamp(1.0f - v, 0.0f, 1.0f); }
-__device__ __forceinline__ DV3 schlick_d(const DV3& f0, float vDotH) {
-    const float c = sclamp(1.0f - vDotH, 0.0f, 1.0f);
-    const float f = c * c * c * c * c;
-    return {f0.x + (1.0f - f0.x) * f, f0.y + (1.0f - f0.y) * f, f0.z + (1.0f - f0.z) * f};
-}
-__device__ __forceinline__ DV3 layer_transmittance_d(const DV3& f0, float nDotV, float nDotL) {
-    const DV3 fv = schlick_d(f0, sclamp(nDotV, 0.0f, 1.0f));
-    const DV3 fl = schlick_d(f0, sclamp(nDotL, 0.0f, 1.0f));
-    const DV3 s = (fv + fl) * 0.5f;
-    return {one_minus_clamped1(s.x), one_minus_clamped1(s.y), one_minus_clamped1(s.z)};
-}
-__device__ __forceinline__ Dual ggx_d_d(float nDotH, const Dual& r) {
-    const Dual a = dmax(0.02f, r * r);
-    const Dual a2 = a * a;
-    const Dual t = nDotH * nDotH * (a2 - 1.0f) + 1.0f;
-    const Dual den = dmax(1.0e-6f, t * t);
-    return a2 / (kPi * den);
-}
-__device__ __forceinline__ Dual ggx_lambda_d(float x, const Dual& a2) {
+__device__ __forceinline__ DualR ggx_lambda_d(float x, const DualR& a2) {
     const float c = smax(x, 1.0e-6f);
-    return (-1.0f + dsqrt(1.0f + a2 * (1.0f - c * c) / (c * c))) * 0.5f;
+    const float cc = c * c;
+    const float root = sqrtf(1.0f + a2.v * (1.0f - cc) / cc);
+    const float k = root > 0.0f ? 0.5f / root : 0.0f;
+    return {(-1.0f + root) * 0.5f, k * (a2.r * (1.0f - cc) / cc) * 0.5f};
 }
-__device__ __forceinline__ Dual ggx_vis_d(float nDotV, float nDotL, const Dual& r) {
-    const Dual a = dmax(0.02f, r * r);
-    const Dual a2 = a * a;
-    return 1.0f / (1.0f + ggx_lambda_d(nDotV, a2) + ggx_lambda_d(nDotL, a2));
+// Distribution x visibility / (4 nv nl) and its roughness derivative.
+__device__ __forceinline__ DualR ggx_scale_d(float nh, float nv, float nl, const DualR& r) {
+    const float rr = r.v * r.v;
+    const DualR a{smax(0.02f, rr), 0.02f < rr ? r.r * r.v + r.v * r.r : 0.0f};
+    const DualR a2{a.v * a.v, a.r * a.v + a.v * a.r};
+    const DualR t{nh * nh * (a2.v - 1.0f) + 1.0f, nh * nh * a2.r};
+    const float tt = t.v * t.v;
+    const DualR x{kPi * smax(1.0e-6f, tt), 1.0e-6f < tt ? kPi * (t.r * t.v + t.v * t.r) : 0.0f};
+    const DualR d{a2.v / x.v, (a2.r * x.v - a2.v * x.r) * (1.0f / (x.v * x.v))};
+    const DualR lv = ggx_lambda_d(nv, a2), ll = ggx_lambda_d(nl, a2);
+    const float den = 1.0f + lv.v + ll.v;
+    const DualR g{1.0f / den, -1.0f / (den * den) * (lv.r + ll.r)};
+    const float norm = smax(4.0f * nv * nl, 1.0e-6f);
+    return {d.v * g.v / norm, (d.r * g.v + d.v * g.r) / norm};
 }
-__device__ __forceinline__ DV3 spec_lobe_d(const V3& n, const V3& v, const V3& l, const DV3& f0, const Dual& r) {
+
+// Gradient of coef . EvaluateBsdf(n, cn, v, l).
+static __device__ __noinline__ MatGrad bsdf_grad(const Mat& m, const V3 n, const V3 cn, const V3 v, const V3 l,
+                                                 const V3 coef) {
+    MatGrad out{{0.0f, 0.0f, 0.0f}, 0.0f, 0.0f};
     const float nv = sclamp(dot(n, v), 0.0f, 1.0f);
     const float nl = sclamp(dot(n, l), 0.0f, 1.0f);
-    if (nv <= 0.0f || nl <= 0.0f) return dv3(V3{0.0f, 0.0f, 0.0f});
+    if (nv <= 0.0f || nl <= 0.0f) return out;
+    const float metal = sclamp(m.metallic, 0.0f, 1.0f);
+    const float dMetal = (m.metallic < 0.0f || 1.0f < m.metallic) ? 0.0f : 1.0f;
+    const V3 underCoat = coat_tint(m) * layer_transmittance(coat_f0(m), dot(cn, v), dot(cn, l));
+    // diffuse lobe: Oren-Nayar term and the colour's scale (base weight, metalness, transmission)
+    const float sigma = sclamp(m.diffuse_roughness, 0.0f, 1.0f);
+    const float radius = sclamp(maxc(ld3(m.subsurface_radius)) / 3.0f, 0.0f, 1.0f);
+    const float wrap = sclamp(m.subsurface * m.subsurface_scale *
+                                  (0.35f + 0.15f * sclamp(m.subsurface_anisotropy, -1.0f, 1.0f) + 0.1f * radius),
+                              0.0f, 0.9f);
+    const float wrapped = sclamp((nl + wrap) / (1.0f + wrap), 0.0f, 1.0f);
+    float term = wrapped / smax(nl, 1.0e-6f);
+    if (sigma != 0.0f) term = oren_nayar(sigma, n, v, l, nv, nl) * term;
+    const float trans = sclamp(m.transmission, 0.0f, 1.0f);
+    const float sss = sclamp(m.subsurface, 0.0f, 1.0f);
+    const float weight = sclamp(m.base_weight, 0.0f, 1.0f);
+    const float colorScale = weight * (1.0f - metal) * (1.0f - trans);
+    const float dColorScale = weight * -dMetal * (1.0f - trans);
+    // base specular lobe
     const V3 h = safe_normalized(v + l, n);
     const float nh = sclamp(dot(n, h), 0.0f, 1.0f);
     const float vh = sclamp(dot(v, h), 0.0f, 1.0f);
-    const Dual d = ggx_d_d(nh, r);
-    const Dual g = ggx_vis_d(nv, nl, r);
-    return schlick_d(f0, vh) * (d * g / smax(4.0f * nv * nl, 1.0e-6f));
-}
-// AdjustedRoughness on a dual base roughness (the phase factor is geometry).
-__device__ __forceinline__ Dual roughness_for_d(const Dual& r, float aniso, float rot, const Mat& m, const V3& n,
-                                                const V3& v, const V3& l) {
-    const float ca = sclamp(aniso, -0.95f, 0.95f);
-    float phase = 0.0f;
-    if (ca != 0.0f) {
-        const V3 tangent = proj_tangent(m, n);
-        const V3 td = safe_normalized(tangent - n * dot(tangent, n), ortho_x(n));
-        const V3 bt = normalize(cross(n, td));
-        const V3 h = safe_normalized(v + l, n);
-        const V3 hp = h - n * dot(n, h);
-        if (length(hp) <= 1.0e-6f) {
-            phase = cosf(rot * 2.0f * kPi);
-        } else {
-            const V3 hd = normalize(hp);
-            phase = cosf(atan2f(dot(hd, bt), dot(hd, td)) - rot * 2.0f * kPi);
-        }
+    const float rough = m.roughness + m.coat_affect_roughness * m.coat_weight * m.coat_roughness;
+    DualR r{sclamp(rough, 0.0f, 1.0f), (rough < 0.0f || 1.0f < rough) ? 0.0f : 1.0f};
+    {
+        const float ca = sclamp(m.specular_anisotropy, -0.95f, 0.95f);
+        const float k = 1.0f - 0.35f * ca * (ca != 0.0f ? aniso_phase(m.specular_rotation, m, n, v, l) : 0.0f);
+        const float x = r.v * k;
+        r = DualR{sclamp(x, 0.02f, 1.0f), (x < 0.02f || 1.0f < x) ? 0.0f : r.r * k};
     }
-    return dclamp(r * (1.0f - 0.35f * ca * phase), 0.02f, 1.0f);
-}
-
-// EvaluateBsdf with derivatives (value identical to bsdf_eval).
-static __device__ __noinline__ DV3 bsdf_eval_d(const Mat& m, const V3& n, const V3& cn, const V3& v, const V3& l) {
-    const float nv = sclamp(dot(n, v), 0.0f, 1.0f);
-    const float nl = sclamp(dot(n, l), 0.0f, 1.0f);
-    if (nv <= 0.0f || nl <= 0.0f) return dv3(V3{0.0f, 0.0f, 0.0f});
-    const MatParams p = mat_params(m);
-    const DV3 baseF0 = spec_f0_d(m, p);
-    const V3 cF0 = coat_f0(m);
-    const V3 underCoat = coat_tint(m) * layer_transmittance(cF0, dot(cn, v), dot(cn, l));
-    const DV3 underBase = layer_transmittance_d(baseF0, nv, nl);
-    const float sigma = sclamp(m.diffuse_roughness, 0.0f, 1.0f);
-    const float wrap = sclamp(m.subsurface * m.subsurface_scale *
-                                  (0.35f + 0.15f * sclamp(m.subsurface_anisotropy, -1.0f, 1.0f) +
-                                   0.1f * sclamp(maxc(ld3(m.subsurface_radius)) / 3.0f, 0.0f, 1.0f)),
-                              0.0f, 0.9f);
-    const float wrapped = sclamp((nl + wrap) / (1.0f + wrap), 0.0f, 1.0f);
-    float term;
-    if (sigma == 0.0f) {
-        term = 1.0f * (wrapped / smax(nl, 1.0e-6f));
-    } else {
-        const V3 vp = normalize(v - n * nv);
-        const V3 lp = normalize(l - n * nl);
-        const float cosPhi = length(vp) > 0.0f && length(lp) > 0.0f ? sclamp(dot(vp, lp), -1.0f, 1.0f) : 0.0f;
-        const float s2 = sigma * sigma;
-        const float orenA = 1.0f - (s2 / (2.0f * (s2 + 0.33f)));
-        const float orenB = 0.45f * s2 / (s2 + 0.09f);
-        const float sinV = sqrtf(smax(0.0f, 1.0f - nv * nv));
-        const float sinL = sqrtf(smax(0.0f, 1.0f - nl * nl));
-        const float sinAlpha = smax(sinV, sinL);
-        const float tanBeta = smin(sinV / smax(nv, 1.0e-6f), sinL / smax(nl, 1.0e-6f));
-        term = (orenA + orenB * smax(0.0f, cosPhi) * sinAlpha * tanBeta) * (wrapped / smax(nl, 1.0e-6f));
-    }
-    const DV3 diffuse = diffuse_color_d(m, p) * underCoat * underBase * (kInvPi * term);
-    const Dual baseRough = dclamp(p.rough + m.coat_affect_roughness * m.coat_weight * m.coat_roughness, 0.0f, 1.0f);
-    const Dual sr = roughness_for_d(baseRough, m.specular_anisotropy, m.specular_rotation, m, n, v, l);
-    DV3 spec = underCoat * spec_lobe_d(n, v, l, baseF0, sr);
-    if (m.thin_film_thickness > 0.0f) {
-        const V3 h = safe_normalized(v + l, n);
-        spec = underCoat * (spec_lobe_d(n, v, l, baseF0, sr) * film_color(m.thin_film_thickness, m.thin_film_ior,
-                                                                          sclamp(dot(v, h), 0.0f, 1.0f)));
-    }
-    const float cr = roughness_for(m.coat_roughness, m.coat_anisotropy, m.coat_rotation, m, cn, v, l);
-    const V3 coat = thin_film(spec_lobe(cn, v, l, cF0, cr), m, cn, v, l);
+    const DualR scale = ggx_scale_d(nh, nv, nl, r);
+    V3 film{1.0f, 1.0f, 1.0f};
+    if (m.thin_film_thickness > 0.0f) film = film_color(m.thin_film_thickness, m.thin_film_ior, vh);
+    // sheen scales the layer transmittance
     const float sw = sclamp(m.sheen, 0.0f, 1.0f);
-    float sf = 1.0f;
-    if (sw != 0.0f) {
-        const V3 h = safe_normalized(v + l, n);
-        const float lh = sclamp(dot(l, h), 0.0f, 1.0f);
-        sf = powf(1.0f - lh, 5.0f) * (1.0f - 0.5f * sclamp(m.sheen_roughness, 0.0f, 1.0f));
+    V3 sheen{0.0f, 0.0f, 0.0f};
+    if (sw != 0.0f)
+        sheen = ld3(m.sheen_color) * sw * (sheen_factor(l, h) * (1.0f - 0.5f * sclamp(m.sheen_roughness, 0.0f, 1.0f))) *
+                underCoat;
+    const float fv = schlick_weight(nv), fl = schlick_weight(nl), fh = schlick_weight(vh);
+    const float specWeight = sclamp(m.specular_weight, 0.0f, 1.0f) * f0_dielectric(m.ior);
+    const float uc[3] = {underCoat.x, underCoat.y, underCoat.z}, fc[3] = {film.x, film.y, film.z},
+                sh[3] = {sheen.x, sheen.y, sheen.z}, cf[3] = {coef.x, coef.y, coef.z};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float b = m.base_color[c], d = m.specular_color[c] * specWeight;
+        const DualBM f0{d * (1.0f - metal) + b * metal, metal, d * -dMetal + b * dMetal};
+        // 1 - (schlick(nv) + schlick(nl)) / 2, clamped
+        const DualBM s = (schlick_d(f0, fv) + schlick_d(f0, fl)) * 0.5f;
+        const float u = 1.0f - s.v;
+        const bool in = !(u < 0.0f || 1.0f < u);
+        const DualBM under{sclamp(u, 0.0f, 1.0f), in ? -s.b : 0.0f, in ? -s.m : 0.0f};
+        // DiffuseColor: lerp(base, lerp(base, subsurface colour, radius), sss) x scale
+        const float tint = b * (1.0f - radius) + m.subsurface_color[c] * radius;
+        const float color = b * (1.0f - sss) + tint * sss;
+        const float dColor = (1.0f - sss) + (1.0f - radius) * sss;
+        const DualBM dc{color * colorScale, dColor * colorScale, color * dColorScale};
+        const DualBM diffuse = dc * uc[c] * under * (kInvPi * term);
+        const DualBM fres = schlick_d(f0, fh) * (fc[c] * uc[c]);
+        out.base[c] = cf[c] * (diffuse.b + fres.b * scale.v + sh[c] * under.b);
+        out.metal += cf[c] * (diffuse.m + fres.m * scale.v + sh[c] * under.m);
+        out.rough += cf[c] * (fres.v * scale.r);
     }
-    const DV3 sheen = (ld3(m.sheen_color) * sw * sf * underCoat) * underBase;
-    return diffuse + spec + dv3(coat) + sheen;
+    return out;
 }
 
 }  // namespace shiro_gpu

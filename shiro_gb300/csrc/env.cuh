@@ -177,8 +177,10 @@ __device__ __forceinline__ size_t env_pick(const DevEnv& e, const V2& u, bool us
 }
 
 // EnvironmentMap::Sample (:109-163).  Returns the radiance; *pdf = 0 marks
-// a failed sample.
-__device__ __forceinline__ V3 env_sample(const DevEnv& e, const V2& u, bool useCdf, V3* dir, float* pdf) {
+// a failed sample.  *texel (may be NULL) is the texel picked, untouched for a
+// map without an importance table.
+__device__ __forceinline__ V3 env_sample(const DevEnv& e, const V2& u, bool useCdf, V3* dir, float* pdf,
+                                         uint32_t* texel = nullptr) {
     if (e.w == 0 || e.h == 0) {
         *dir = {0.0f, 1.0f, 0.0f};
         *pdf = 0.0f;
@@ -188,6 +190,7 @@ __device__ __forceinline__ V3 env_sample(const DevEnv& e, const V2& u, bool useC
         // the texel; its centre direction, pdf (mass rowMass * columnMass)
         // and radiance come from the per-texel sample records
         const size_t t = env_pick(e, u, useCdf);
+        if (texel) *texel = static_cast<uint32_t>(t);
         const float4 a = __ldg(&e.samples[2 * t]), b = __ldg(&e.samples[2 * t + 1]);
         *dir = V3{a.x, a.y, a.z};
         *pdf = a.w;

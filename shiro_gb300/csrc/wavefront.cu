@@ -135,14 +135,10 @@ struct AdjWave {
     const AdjView* view;  // device copy (gradient buffers, d_beauty, dome 0's texture), written per call
     float4* lrem;         // radiance of the path not yet accounted for
     float4* delta;        // d loss / d path radiance: d_beauty of its pixel / spp
-    float4* vtx;          // 3 per slot: (shading normal, material bits), (coat normal), (view direction)
-    float4* cont;         // 2 per slot: (continuation direction, 1 when its gradient is due), (its BSDF value)
-    float4* lgrad;        // 3 per light sample and slot, [k][P]: (L w s), (f R w s, 1 for dome 0's texture), (local dir)
     uint32_t on;          // replay stages follow the forward ones
     uint32_t pad;
 };
-constexpr size_t kAdjSlotFloat4 = 7;      // lrem, delta, vtx (3), cont (2)
-constexpr size_t kAdjLightFloat4 = 3;     // per light sample
+constexpr size_t kAdjSlotFloat4 = 2;      // lrem, delta
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
@@ -990,11 +986,12 @@ __global__ void __launch_bounds__(128) wf_resolve(WfView v) {
 
 // ---- adjoint replay stages ---------------------------------------------------
 // The estimator of adjoint.cu's path replay (adj_path with the scene's own
-// parameters), cut at the same seams as the forward stages: light samples and
-// continuation in wa_shade, their occlusion in wf_occlude, the gradients of
-// the visible samples and of the continuation in wa_shadow (they need the
-// radiance still to come, which is known once the vertex's direct light is),
-// the environment gradients of the misses in wa_miss.
+// parameters), cut at the forward stages' seams.  The forward stages logged
+// each bounce's hit and which light samples were visible, so nothing is traced
+// and a vertex's gradients are formed where its samples are: wa_shade replays
+// the visible light samples with theirs, which leaves the radiance still to
+// come for the continuation and its gradient in wa_continue.  wa_miss adds the
+// environment gradients of the paths that leave.
 
 __global__ void wa_begin(WfView v) {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
@@ -1089,59 +1086,54 @@ __global__ void __launch_bounds__(256) wa_hits(WfView v, uint32_t cur, uint32_t 
 // Light sample k of a vertex with the factors of its gradient: its clamped
 // contribution c, gL = L w s (material gradient = delta T gL . df) and
 // gE = f R w s (texel gradient of dome 0's texture = delta T gE at `local`),
-// with s the clamp scale held constant.  kExt: the scene has emitters or
+// with s the clamp scale held constant.  *texel is the texel drawn
+// (0xffffffff: no importance table).  kExt: the scene has emitters or
 // cut-outs (the replay stages are compiled for each kind of scene).
 template <bool kExt>
 __device__ __forceinline__ bool wa_light(const DevScene& s, const DevRequest& q, const AdjView& a, const Vertex& vx,
-                                         const Sampler& smp, uint32_t depth, uint32_t k, const float4* rec, const Mat& ms,
-                                         V3* ld, V3* c, V3* gL, V3* gE, V3* local, bool* envMark) {
-    V3 L, f, domeRad{0.0f, 0.0f, 0.0f};
-    float w;
+                                         const Sampler& smp, uint32_t depth, uint32_t k, V3* ld, V3* c, V3* gL, V3* gE,
+                                         V3* local, uint32_t* texel, bool* envMark) {
+    V3 L, domeRad{0.0f, 0.0f, 0.0f};
+    float nl, lp = 0.0f;
     int32_t envIdx = -1;
     *local = V3{0.0f, 0.0f, 0.0f};
+    *texel = 0xffffffffu;
+    const bool mis = k >= s.distantCount;
     if (kExt && k >= s.distantCount + s.domeCount * q.domeSamples) {  // the emissive-triangle sample
-        float lp, nl, reach;
+        float reach;
         if (!emissive_geometry(s, vx, smp, depth, ld, &L, &lp, &nl, &reach)) return false;
-        const float4 e = bsdf_eval_pdf_rec(rec, ms, vx.n, vx.cn, vx.view, *ld, true);
-        f = f4xyz(e);
-        w = nl * power_heuristic(lp, e.w) / lp;
-    } else if (k < s.distantCount) {
+    } else if (!mis) {
         const DevDistant l = s.distant[k];
         *ld = l.toLight;
-        const float nl = sclamp(dot(vx.n, *ld), 0.0f, 1.0f);
+        nl = sclamp(dot(vx.n, *ld), 0.0f, 1.0f);
         if (nl <= 0.0f) return false;
         L = l.radiance;
-        w = nl;
-        f = bsdf_eval_rec(rec, ms, vx.n, vx.cn, vx.view, *ld);
     } else {
         const uint32_t r = k - s.distantCount;
         const uint32_t li = r / q.domeSamples, jj = r - li * q.domeSamples;
         const DevDome& d = s.domes[li];
         const uint32_t dim = kDirectDimBase + depth * kDirectDepthStride + li * kDirectLightStride + jj * kDirectSampleStride;
         const V2 u = smp.next2d(dim);
-        float lp;
         if (d.env >= 0) {
-            env_sample(s.envs[d.env], u, (q.flags & SHIRO_RENDER_ENV_CDF) != 0u, local, &lp);
+            // (the replay's environment is the scene's: a sample's radiance is env_evaluate's there)
+            const V3 rad = env_sample(s.envs[d.env], u, (q.flags & SHIRO_RENDER_ENV_CDF) != 0u, local, &lp, texel);
             if (lp <= 0.0f) return false;
-            L = env_evaluate(env_for_eval(s, a, d.env), *local) * d.radiance;
+            L = rad * d.radiance;
             envIdx = d.env;
             domeRad = d.radiance;
         } else {
-            const float yy = 1.0f - 2.0f * u.y;
-            const float rr = sqrtf(smax(0.0f, 1.0f - yy * yy));
-            const float phi = 2.0f * kPi * u.x;
-            *local = V3{sinf(phi) * rr, yy, cosf(phi) * rr};
+            *local = sphere_direction(u);
             lp = kInvFourPi;
             L = V3{1.0f, 1.0f, 1.0f} * d.radiance;
         }
         *ld = light_to_world(d, *local);
-        const float nl = sclamp(dot(vx.n, *ld), 0.0f, 1.0f);
+        nl = sclamp(dot(vx.n, *ld), 0.0f, 1.0f);
         if (nl <= 0.0f) return false;
-        const float4 e = bsdf_eval_pdf_rec(rec, ms, vx.n, vx.cn, vx.view, *ld, true);
-        f = f4xyz(e);
-        const float mis = power_heuristic(lp, e.w);
-        w = nl * mis / lp;
     }
+    const float4 e =
+        bsdf_eval_pdf_rec(bsdf_rec(s, vx.hit.material), s.materials[vx.hit.material], vx.n, vx.cn, vx.view, *ld, mis);
+    const V3 f = f4xyz(e);
+    const float w = mis ? nl * power_heuristic(lp, e.w) / lp : nl;
     const V3 raw = f * L * w;
     *c = clamp24(q, raw);
     const float sc = clamp_scale(q, raw, kDirectSampleClamp);
@@ -1151,8 +1143,90 @@ __device__ __forceinline__ bool wa_light(const DevScene& s, const DevRequest& q,
     return true;
 }
 
+// Six blocks of 128 per SM for the two vertex stages (an 80-register cap, some
+// spills): they wait for path state and records, and for instructions; replay
+// of the 512x512 32-spp 256-material view 3.77 ms at four blocks, 3.65 at five,
+// 3.48 at six, 3.57 at eight (4.86 ms when light samples and continuations were
+// stored, with all their factors, for a gradient stage of their own).
+constexpr int kReplayBlocks = 6;
+
+// The replayed vertex of shade-queue entry `j` and its path's state; false when
+// the path passes through an opacity cut-out there (the forward's decision; no
+// media, transmission being refused).
 template <bool kExt>
-__global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw, uint32_t cur, uint32_t depth) {
+__device__ __forceinline__ bool wa_vertex(const WfView& v, const DevScene& s, uint32_t j, const Sampler& smp, uint32_t depth,
+                                          PathState& ps, Vertex& vx) {
+    const float4 o = v.ro[j], d = v.rd[j], t4 = v.T[j], h4 = v.hit[j];
+    const uint32_t bits = __float_as_uint(t4.w);
+    ps.ro = V3{o.x, o.y, o.z};
+    ps.rd = V3{d.x, d.y, d.z};
+    ps.prevPdf = d.w;
+    ps.T = V3{t4.x, t4.y, t4.z};
+    ps.radiance = V3{0.0f, 0.0f, 0.0f};
+    ps.diffDepth = bits & 0xffu;
+    ps.specDepth = (bits >> 8) & 0xffu;
+    ps.prevDelta = (bits & kFlagPrevDelta) != 0u;
+    ps.prevType = (bits >> kTypeShift) & 3u;
+    ps.inside = false;
+    ps.mediumActive = false;
+    HitRec h;
+    h.t = h4.x;
+    h.u = h4.y;
+    h.v = h4.z;
+    h.gid = __float_as_uint(h4.w);
+    vx = make_vertex(s, ps.ro, ps.rd, h);
+    return !kExt || enter_hit(s, smp, depth, vx, h.t, ps);
+}
+
+// Gradients of a vertex's visible light samples; the radiance still to come
+// past its direct (and emitted) light.
+template <bool kExt>
+__global__ void __launch_bounds__(128, kReplayBlocks) wa_shade(WfView v, DevScene s, AdjWave aw, uint32_t depth) {
+    const uint32_t count = v.counters[kHitCount];
+    const AdjView& a = *aw.view;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const uint32_t j = v.shadeQ[i];
+        // the samples the forward stages found taken and unoccluded at this vertex
+        const uint32_t seen = v.visLog[static_cast<size_t>(depth) * v.P + j];
+        if (!kExt && seen == 0u) continue;
+        const uint4 id = v.ident[j];
+        const DevRequest& q = v.reqs[id.w].q;
+        const Sampler smp{id.x, id.y, id.z, s.radical};
+        PathState ps;
+        Vertex vx;
+        if (!wa_vertex<kExt>(v, s, j, smp, depth, ps, vx)) continue;
+        const float4 dl4 = aw.delta[j], l4 = aw.lrem[j];
+        const uint32_t mat = vx.hit.material;
+        V3 lrem{l4.x, l4.y, l4.z};
+        if constexpr (kExt) {
+            // radiance emitted at this hit: no BSDF value of this vertex or a
+            // later one scales it, so it leaves the radiance still to come
+            add_emission(s, vx, depth, ps);
+            lrem = lrem - ps.radiance;
+        }
+        const V3 dT = V3{dl4.x, dl4.y, dl4.z} * ps.T;
+        const V3 direct = sum_direct<kExt>(s, q, [&](uint32_t k, V3* c) {
+            if (!((seen >> k) & 1u)) return false;
+            V3 ld, gL, gE, local;
+            uint32_t texel;
+            bool mark;
+            if (!wa_light<kExt>(s, q, a, vx, smp, depth, k, &ld, c, &gL, &gE, &local, &texel, &mark)) return false;
+            add_mat_grad(a, mat, bsdf_grad(s.materials[mat], vx.n, vx.cn, vx.view, ld, dT * gL));
+            if (mark) {
+                if (texel != 0xffffffffu) add_env_grad_texel(a, a.evalEnv, local, texel, dT * gE);
+                else add_env_grad(a, a.evalEnv, local, dT * gE);
+            }
+            return true;
+        });
+        lrem = lrem - ps.T * direct;
+        aw.lrem[j] = make_float4(lrem.x, lrem.y, lrem.z, 0.0f);
+    }
+}
+
+// Continuation of a vertex (the reflecting lobes of continue_path) and its
+// gradient, the radiance still to come being known.
+template <bool kExt>
+__global__ void __launch_bounds__(128, kReplayBlocks) wa_continue(WfView v, DevScene s, AdjWave aw, uint32_t cur, uint32_t depth) {
     const uint32_t count = v.counters[kHitCount];
     uint32_t* qout = cur ? v.rayQ0 : v.rayQ1;
     uint32_t* cout = &v.counters[cur ^ 1u];
@@ -1167,77 +1241,24 @@ __global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw
             j = v.shadeQ[i];
             const uint4 id = v.ident[j];
             const DevRequest& q = v.reqs[id.w].q;
-            const float4 o = v.ro[j], d = v.rd[j], t4 = v.T[j], h4 = v.hit[j];
-            const uint32_t bits = __float_as_uint(t4.w);
-            PathState ps;
-            ps.ro = V3{o.x, o.y, o.z};
-            ps.rd = V3{d.x, d.y, d.z};
-            ps.prevPdf = d.w;
-            ps.T = V3{t4.x, t4.y, t4.z};
-            ps.diffDepth = bits & 0xffu;
-            ps.specDepth = (bits >> 8) & 0xffu;
-            ps.prevDelta = (bits & kFlagPrevDelta) != 0u;
-            ps.prevType = (bits >> kTypeShift) & 3u;
-            ps.inside = false;
-            ps.mediumActive = false;
-            HitRec h;
-            h.t = h4.x;
-            h.u = h4.y;
-            h.v = h4.z;
-            h.gid = __float_as_uint(h4.w);
-            const Vertex vx = make_vertex(s, ps.ro, ps.rd, h);
-            const uint32_t mat = vx.hit.material;
-            const Mat& ms = s.materials[mat];
-            const float4* rec = bsdf_rec(s, mat);
-            aw.vtx[3 * static_cast<size_t>(j)] = make_float4(vx.n.x, vx.n.y, vx.n.z, __uint_as_float(mat));
-            aw.vtx[3 * static_cast<size_t>(j) + 1] = make_float4(vx.cn.x, vx.cn.y, vx.cn.z, 0.0f);
-            aw.vtx[3 * static_cast<size_t>(j) + 2] = make_float4(vx.view.x, vx.view.y, vx.view.z, 0.0f);
             const Sampler smp{id.x, id.y, id.z, s.radical};
-            // an opacity cut-out the path passes through (the forward's decision;
-            // no media, transmission being refused): the hit is not shaded
-            const bool shaded = !kExt || enter_hit(s, smp, depth, vx, h.t, ps);
-            if (kExt && shaded) {
-                // radiance emitted at this hit: no BSDF value of this vertex or a
-                // later one scales it, so it leaves the radiance still to come
-                ps.radiance = V3{0.0f, 0.0f, 0.0f};
-                add_emission(s, vx, depth, ps);
-                if (ps.radiance.x != 0.0f || ps.radiance.y != 0.0f || ps.radiance.z != 0.0f) {
-                    const float4 l4 = aw.lrem[j];
-                    aw.lrem[j] = make_float4(l4.x - ps.radiance.x, l4.y - ps.radiance.y, l4.z - ps.radiance.z, 0.0f);
-                }
-            }
-            const uint32_t nls = light_sample_count<kExt>(s, q);
-            // which samples the forward stages found taken and unoccluded at this vertex
-            const uint32_t seen = shaded ? v.visLog[static_cast<size_t>(depth) * v.P + j] : 0u;
-            for (uint32_t k = 0; k < nls; ++k) {
-                V3 ld{0.0f, 0.0f, 0.0f}, c{0.0f, 0.0f, 0.0f}, gL{0.0f, 0.0f, 0.0f}, gE{0.0f, 0.0f, 0.0f},
-                    local{0.0f, 0.0f, 0.0f};
-                bool mark = false;
-                const bool ok =
-                    shaded && wa_light<kExt>(s, q, a, vx, smp, depth, k, rec, ms, &ld, &c, &gL, &gE, &local, &mark);
-                const size_t e = static_cast<size_t>(k) * v.P + j;
-                v.shDir[e] = make_float4(ld.x, ld.y, ld.z, (ok && ((seen >> k) & 1u)) ? FLT_MAX : 0.0f);
-                v.shC[e] = make_float4(c.x, c.y, c.z, 0.0f);
-                aw.lgrad[3 * e] = make_float4(gL.x, gL.y, gL.z, 0.0f);
-                aw.lgrad[3 * e + 1] = make_float4(gE.x, gE.y, gE.z, mark ? 1.0f : 0.0f);
-                aw.lgrad[3 * e + 2] = make_float4(local.x, local.y, local.z, 0.0f);
-            }
-            v.shT[j] = make_float4(ps.T.x, ps.T.y, ps.T.z, 0.0f);
-            // continuation (the reflecting lobes of continue_path); past a cut-out
-            // the ray goes on unchanged, with no BSDF value to differentiate
-            bool alive = false, due = false, pass = false;
-            V3 next{0.0f, 0.0f, 0.0f}, f{0.0f, 0.0f, 0.0f};
+            PathState ps;
+            Vertex vx;
+            const bool shaded = wa_vertex<kExt>(v, s, j, smp, depth, ps, vx);
+            const Mat& ms = s.materials[vx.hit.material];
+            const float4* rec = bsdf_rec(s, vx.hit.material);
             const uint32_t base = depth * kPathDimStride;
             const float rw = vx.w.diffuse + vx.w.spec + vx.w.coat;
             const float tw = rw + 0.0f;
             do {
-                if (!shaded) {
-                    pass = depth + 1u < q.maxDepth;
+                if (!shaded) {  // past a cut-out the ray goes on unchanged, with no BSDF value to differentiate
+                    pushRay = depth + 1u < q.maxDepth;
                     break;
                 }
                 if (tw <= 0.0f) break;
                 const float sel = smp.next1d(base + 1u) * tw;
                 const V2 ds = smp.next2d(base + 2u);
+                V3 next;
                 float pdf = 0.0f;
                 bool delta2 = false, wantPdf = false;
                 const float rs = sel - 0.0f;
@@ -1264,7 +1285,7 @@ __global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw
                     delta2 = sr <= kDeltaRoughness;
                 }
                 const float4 ev = bsdf_eval_pdf_rec(rec, ms, vx.n, vx.cn, vx.view, next, wantPdf);
-                f = f4xyz(ev);
+                const V3 f = f4xyz(ev);
                 if (wantPdf) pdf = smax((rw / tw) * ev.w, 1.0e-6f);
                 const float cosT = sclamp(dot(vx.n, next), 0.0f, 1.0f);
                 if (cosT <= 0.0f) break;
@@ -1275,7 +1296,7 @@ __global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw
                 ps.prevDelta = delta2;
                 ps.prevPdf = pdf;
                 ps.prevType = type;
-                alive = true;
+                bool alive = true;
                 if (depth >= 2) {
                     const float cp = sclamp(maxc(ps.T), 0.05f, 0.95f);
                     if (smp.next1d(base + 4u) > cp) {
@@ -1284,63 +1305,21 @@ __global__ void __launch_bounds__(128) wa_shade(WfView v, DevScene s, AdjWave aw
                         ps.T = ps.T / cp;
                     }
                 }
-                due = alive && depth + 1u < q.maxDepth;
+                pushRay = alive && depth + 1u < q.maxDepth;
+                if (pushRay) {  // every later contribution scales with f (per channel)
+                    const float4 dl = aw.delta[j], l4 = aw.lrem[j];
+                    const V3 coef{f.x > 0.0f ? dl.x * l4.x / f.x : 0.0f, f.y > 0.0f ? dl.y * l4.y / f.y : 0.0f,
+                                  f.z > 0.0f ? dl.z * l4.z / f.z : 0.0f};
+                    add_mat_grad(a, vx.hit.material, bsdf_grad(ms, vx.n, vx.cn, vx.view, next, coef));
+                }
             } while (false);
-            aw.cont[2 * static_cast<size_t>(j)] = make_float4(next.x, next.y, next.z, due ? 1.0f : 0.0f);
-            aw.cont[2 * static_cast<size_t>(j) + 1] = make_float4(f.x, f.y, f.z, 0.0f);
-            if (due || pass) {
+            if (pushRay) {
                 v.T[j] = make_float4(ps.T.x, ps.T.y, ps.T.z, __uint_as_float(pack_state(ps)));
                 v.ro[j] = make_float4(ps.ro.x, ps.ro.y, ps.ro.z, 0.0f);
                 v.rd[j] = make_float4(ps.rd.x, ps.rd.y, ps.rd.z, ps.prevPdf);
-                pushRay = true;
             }
         }
         warp_push(cout, qout, pushRay, j);
-    }
-}
-
-// Gradients of a shaded vertex once its light samples' visibility is known.
-template <bool kExt>
-__global__ void __launch_bounds__(128, 4) wa_shadow(WfView v, DevScene s, AdjWave aw) {
-    const uint32_t count = v.counters[kHitCount];
-    const AdjView& a = *aw.view;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const uint32_t j = v.shadeQ[i];
-        const DevRequest& q = v.reqs[v.ident[j].w].q;
-        const float4 t4 = v.shT[j], dl4 = aw.delta[j], l4 = aw.lrem[j];
-        const float4 v0 = aw.vtx[3 * static_cast<size_t>(j)], v1 = aw.vtx[3 * static_cast<size_t>(j) + 1],
-                     v2 = aw.vtx[3 * static_cast<size_t>(j) + 2];
-        const V3 T0{t4.x, t4.y, t4.z}, dl{dl4.x, dl4.y, dl4.z};
-        const V3 n{v0.x, v0.y, v0.z}, cn{v1.x, v1.y, v1.z}, view{v2.x, v2.y, v2.z};
-        const uint32_t mat = __float_as_uint(v0.w);
-        const Mat& me = a.evalMats[mat];
-        const V3 dT = dl * T0;
-        const V3 direct = sum_direct<kExt>(s, q, [&](uint32_t k, V3* c) {
-            const size_t e = static_cast<size_t>(k) * v.P + j;
-            const float4 d4 = v.shDir[e];
-            if (d4.w == 0.0f) return false;
-            const float4 c4 = v.shC[e];
-            *c = V3{c4.x, c4.y, c4.z};
-            const float4 g0 = aw.lgrad[3 * e], g1 = aw.lgrad[3 * e + 1];
-            const DV3 fd = bsdf_eval_d(me, n, cn, view, V3{d4.x, d4.y, d4.z});
-            add_mat_grad(a, mat, fd, dT * V3{g0.x, g0.y, g0.z});
-            if (g1.w != 0.0f) {
-                const float4 g2 = aw.lgrad[3 * e + 2];
-                add_env_grad(a, a.evalEnv, V3{g2.x, g2.y, g2.z}, dT * V3{g1.x, g1.y, g1.z});
-            }
-            return true;
-        });
-        const V3 lrem = V3{l4.x, l4.y, l4.z} - T0 * direct;
-        const float4 c0 = aw.cont[2 * static_cast<size_t>(j)];
-        if (c0.w != 0.0f) {
-            const float4 f4 = aw.cont[2 * static_cast<size_t>(j) + 1];
-            const V3 f{f4.x, f4.y, f4.z};
-            const DV3 fd = bsdf_eval_d(me, n, cn, view, V3{c0.x, c0.y, c0.z});
-            const V3 coef{f.x > 0.0f ? dl.x * lrem.x / f.x : 0.0f, f.y > 0.0f ? dl.y * lrem.y / f.y : 0.0f,
-                          f.z > 0.0f ? dl.z * lrem.z / f.z : 0.0f};
-            add_mat_grad(a, mat, fd, coef);
-        }
-        aw.lrem[j] = make_float4(lrem.x, lrem.y, lrem.z, 0.0f);
     }
 }
 
@@ -1585,7 +1564,7 @@ struct Launch {
     int gBin;
     AdjWave aw;                   // aw.on: the adjoint replay follows the forward stages
     uint32_t replayOnly;          // the adjoint replay alone, of a kept forward wave
-    int gAdjShade, gAdjShadow, gAdjMiss, gAdjHits;
+    int gAdjShade, gAdjCont, gAdjMiss, gAdjHits;
     bool ext;  // the scene uses transmission, opacity or emitters
 };
 
@@ -1629,15 +1608,15 @@ void enqueue_replay(const Launch& L, cudaStream_t st) {
         const uint32_t cur = d & 1u;
         wa_hits<<<L.gAdjHits, 256, 0, st>>>(L.v, cur, d);  // no tracing: the forward stages' hits and visibility
         if (L.ext) {
-            wa_shade<true><<<L.gAdjShade, 128, 0, st>>>(L.v, L.s, L.aw, cur, d);
+            wa_shade<true><<<L.gAdjShade, 128, 0, st>>>(L.v, L.s, L.aw, d);
         } else {
-            wa_shade<false><<<L.gAdjShade, 128, 0, st>>>(L.v, L.s, L.aw, cur, d);
+            wa_shade<false><<<L.gAdjShade, 128, 0, st>>>(L.v, L.s, L.aw, d);
         }
         wa_miss<<<L.gAdjMiss, 256, 0, st>>>(L.v, L.s, L.aw, d);
         if (L.ext) {
-            wa_shadow<true><<<L.gAdjShadow, 128, 0, st>>>(L.v, L.s, L.aw);
+            wa_continue<true><<<L.gAdjCont, 128, 0, st>>>(L.v, L.s, L.aw, cur, d);
         } else {
-            wa_shadow<false><<<L.gAdjShadow, 128, 0, st>>>(L.v, L.s, L.aw);
+            wa_continue<false><<<L.gAdjCont, 128, 0, st>>>(L.v, L.s, L.aw, cur, d);
         }
         wf_end_bounce<<<1, 32, 0, st>>>(L.v, cur);
     }
@@ -1814,8 +1793,7 @@ int run_waves(ContextImpl* ctx, WavefrontState* wf, const ShiroWavefrontConfig& 
     if (adj) {  // per-slot replay state of each pool, and the parameter view on the device
         for (uint32_t k = 0; k < nl; ++k)
             if (!ensure_block(ctx, &wf->pools[k].adj,
-                              static_cast<size_t>(poolP[k]) * (kAdjSlotFloat4 + kAdjLightFloat4 * std::max(1u, lightSamples)) *
-                                  sizeof(float4), "adjoint replay state"))
+                              static_cast<size_t>(poolP[k]) * kAdjSlotFloat4 * sizeof(float4), "adjoint replay state"))
                 return SHIRO_ERR_OUT_OF_MEMORY;
         if (!ensure_block(ctx, &wf->adjView, sizeof(AdjView), "adjoint view")) return SHIRO_ERR_OUT_OF_MEMORY;
         adjCopy = *adj;
@@ -1882,7 +1860,7 @@ int run_waves(ContextImpl* ctx, WavefrontState* wf, const ShiroWavefrontConfig& 
     L.gRes = grid_for(wf_resolve, 128, wf->smCount);
     L.gBin = grid_for(wf_bin_scatter, 256, wf->smCount);
     L.gAdjShade = L.ext ? grid_for(wa_shade<true>, 128, wf->smCount) : grid_for(wa_shade<false>, 128, wf->smCount);
-    L.gAdjShadow = L.ext ? grid_for(wa_shadow<true>, 128, wf->smCount) : grid_for(wa_shadow<false>, 128, wf->smCount);
+    L.gAdjCont = L.ext ? grid_for(wa_continue<true>, 128, wf->smCount) : grid_for(wa_continue<false>, 128, wf->smCount);
     L.gAdjMiss = grid_for(wa_miss, 256, wf->smCount);
     L.gAdjHits = grid_for(wa_hits, 256, wf->smCount);
     L.binRays = cfg.bin_rays == 1 ? 1u : 0u;
@@ -1904,9 +1882,6 @@ int run_waves(ContextImpl* ctx, WavefrontState* wf, const ShiroWavefrontConfig& 
         aw.view = static_cast<const AdjView*>(wf->adjView.ptr);
         aw.lrem = b;
         aw.delta = b + p;
-        aw.vtx = b + 2 * p;
-        aw.cont = b + 5 * p;
-        aw.lgrad = b + 7 * p;
         aw.on = 1u;
         return aw;
     };
