@@ -81,20 +81,37 @@ constexpr uint32_t kHitCount = 8, kMissCount = 9;
 // do not queue behind one another (1080p field frame 96.5 -> 95.8 ms).
 constexpr uint32_t kCounters = 10, kCounterStride = 32;
 
+// Two float4 that the stages read and write together: one 32-byte sector, one
+// 256-bit access (sm_100 and later).  After the first bounce the queues are
+// sparse in the slots, and 16-byte arrays of their own fetched twice the bytes
+// used.
+struct alignas(32) F4Pair {
+    float4 a, b;
+};
+__device__ __forceinline__ F4Pair ld_pair(const F4Pair* p) {
+    F4Pair r;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+                 : "l"(p)
+                 : "memory");
+    return r;
+}
+__device__ __forceinline__ void st_pair(F4Pair* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 struct WfView {
     // path state, one entry per slot of the wave
-    float4* ro;      // ro.xyz, unused
-    float4* rd;      // rd.xyz, prevPdf
-    float4* T;       // T.xyz, bits: diffDepth | specDepth << 8 | flags
-    float4* rad;     // radiance.xyz, first-hit depth
+    F4Pair* ray;     // (ro.xyz, request), (rd.xyz, prevPdf)
+    F4Pair* st;      // (T.xyz, bits: diffDepth | specDepth << 8 | flags), (radiance.xyz, first-hit depth)
     uint4* ident;    // px, py, sample index, request
     float4* hit;     // t, u, v, global triangle index bits (0xffffffff: a miss)
     float4* medium;  // extinction of the medium the path is in (while it attenuates)
     // shadow records
-    float4* shOrigin;  // origin.xyz
-    float4* shT;       // throughput at the vertex
-    float4* shDir;     // [lightSamples][P]: dir.xyz, reach of the shadow ray (0: no sample / occluded)
-    float4* shC;       // [lightSamples][P]: contribution
+    F4Pair* shVtx;     // (origin.xyz, request), (throughput at the vertex, 1 when the path ends there)
+    F4Pair* shLight;   // [lightSamples][P]: (dir.xyz, reach of the shadow ray - 0: no sample / occluded), (contribution)
     uint32_t* rayQ0;
     uint32_t* rayQ1;
     uint32_t* shadowQ;     // paths with light samples to accumulate
@@ -214,9 +231,9 @@ __device__ __forceinline__ uint32_t bin_key(const WfView& v, const float4& o, co
 __device__ __forceinline__ void bin_item(const WfView& v, uint32_t which, uint32_t item, uint32_t* key) {
     if (which) {
         const uint32_t j = item >> 3, k = item & 7u;
-        *key = bin_key(v, v.shOrigin[j], v.shDir[static_cast<size_t>(k) * v.P + j], k);
+        *key = bin_key(v, v.shVtx[j].a, v.shLight[static_cast<size_t>(k) * v.P + j].a, k);
     } else {
-        *key = bin_key(v, v.ro[item], v.rd[item], 0u);
+        *key = bin_key(v, v.ray[item].a, v.ray[item].b, 0u);
     }
 }
 
@@ -308,6 +325,11 @@ __global__ void wf_begin(WfView v) {
     }
 }
 
+__device__ __forceinline__ void put_ray(const WfView& v, uint32_t j, const PathState& ps, uint32_t req) {
+    st_pair(&v.ray[j], make_float4(ps.ro.x, ps.ro.y, ps.ro.z, __uint_as_float(req)),
+            make_float4(ps.rd.x, ps.rd.y, ps.rd.z, ps.prevPdf));
+}
+
 __global__ void __launch_bounds__(128) wf_generate(WfView v) {
     const WaveDesc w = cur_wave(v);
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < w.paths; j += gridDim.x * blockDim.x) {
@@ -320,10 +342,9 @@ __global__ void __launch_bounds__(128) wf_generate(WfView v) {
         const Sampler smp{x, y, smpIdx, nullptr};
         PathState ps;
         init_path(q, smp, ps);
-        v.ro[j] = make_float4(ps.ro.x, ps.ro.y, ps.ro.z, 0.0f);
-        v.rd[j] = make_float4(ps.rd.x, ps.rd.y, ps.rd.z, ps.prevPdf);
-        v.T[j] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(kFlagPrevDelta));
-        v.rad[j] = make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0x7f800000));
+        put_ray(v, j, ps, sg.req);
+        st_pair(&v.st[j], make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(kFlagPrevDelta)),
+                make_float4(0.0f, 0.0f, 0.0f, __int_as_float(0x7f800000)));
         v.ident[j] = make_uint4(x, y, smpIdx, sg.req);
         v.rayQ0[j] = j;  // albedo / normal records are written by a first hit and read only after one
 
@@ -602,8 +623,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend(WfView v, DevScene 
             const uint32_t got = feed_lanes(feed, &counter(v, kFetchExtend), count, has, v.refillIdle);
             if (got != 0xffffffffu) {
                 j = q[got];
-                const float4 o = v.ro[j], d = v.rd[j];
-                wide_init(t, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, FLT_MAX);
+                const F4Pair r = ld_pair(&v.ray[j]);
+                wide_init(t, f4xyz(r.a), f4xyz(r.b), FLT_MAX);
                 has = true;
             }
             if (__ballot_sync(kFull, has) == 0u) break;
@@ -633,9 +654,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend(WfView v, DevScene 
         bool hit = false;
         if (valid) {
             j = q[i];
-            const float4 o = v.ro[j], d = v.rd[j];
+            const F4Pair r = ld_pair(&v.ray[j]);
             HitRec h;
-            trace_closest(s, V3{o.x, o.y, o.z}, V3{d.x, d.y, d.z}, &h, ctr);
+            trace_closest(s, f4xyz(r.a), f4xyz(r.b), &h, ctr);
             const float4 h4 = make_float4(h.t, h.u, h.v, __uint_as_float(h.gid));
             v.hit[j] = h4;
             if (kLog) log_hit(v, depth, j, h4);
@@ -705,7 +726,8 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
             float depth0 = 0.0f;
             bool shaded = false;  // false: an opacity cut-out the path passes through
             if (valid) {
-                const float4 o = v.ro[j], d = v.rd[j], t4 = v.T[j], r4 = v.rad[j], h4 = v.hit[j];
+                const F4Pair ry = ld_pair(&v.ray[j]), sp = ld_pair(&v.st[j]);
+                const float4 o = ry.a, d = ry.b, t4 = sp.a, r4 = sp.b, h4 = v.hit[j];
                 const uint32_t bits = __float_as_uint(t4.w);
                 ps.ro = V3{o.x, o.y, o.z};
                 ps.rd = V3{d.x, d.y, d.z};
@@ -753,8 +775,8 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
                     const bool ok = light_sample<kExt>(s, q, vx, smp, depth, k, &dir, &c, &reach, ctr);
                     lightMask |= ok ? (1u << k) : 0u;
                     const size_t e = static_cast<size_t>(k) * v.P + j;
-                    v.shDir[e] = make_float4(dir.x, dir.y, dir.z, ok ? reach : 0.0f);
-                    v.shC[e] = make_float4(c.x, c.y, c.z, 0.0f);
+                    st_pair(&v.shLight[e], make_float4(dir.x, dir.y, dir.z, ok ? reach : 0.0f),
+                            make_float4(c.x, c.y, c.z, 0.0f));
                 }
                 phase();
             }
@@ -762,8 +784,8 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
                 const bool anyLight = lightMask != 0u;
                 if (anyLight) {
                     const V3 org = shadow_origin(vx);
-                    v.shOrigin[j] = make_float4(org.x, org.y, org.z, 0.0f);
-                    v.shT[j] = make_float4(ps.T.x, ps.T.y, ps.T.z, 0.0f);
+                    st_pair(&v.shVtx[j], make_float4(org.x, org.y, org.z, __uint_as_float(id.w)),
+                            make_float4(ps.T.x, ps.T.y, ps.T.z, 0.0f));
                 }
                 const bool cont =
                     (!shaded || continue_path<kExt>(s, q, vx, smp, depth, ps, ctr)) && depth + 1u < q.maxDepth;
@@ -771,17 +793,16 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
                 uint32_t nb = pack_state(ps);
                 if (!cont && anyLight) {
                     nb |= kFlagDone;
-                    v.shT[j].w = 1.0f;  // read by wf_shadow with the throughput (no load of T for the flag)
+                    v.shVtx[j].b.w = 1.0f;  // read by wf_shadow with the throughput (no load of T for the flag)
                 }
-                v.T[j] = make_float4(ps.T.x, ps.T.y, ps.T.z, __uint_as_float(nb));
+                st_pair(&v.st[j], make_float4(ps.T.x, ps.T.y, ps.T.z, __uint_as_float(nb)),
+                        make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, depth0));
                 if (kExt && ps.mediumActive)
                     v.medium[j] = make_float4(ps.extinction.x, ps.extinction.y, ps.extinction.z, 0.0f);
                 if (cont) {
-                    v.ro[j] = make_float4(ps.ro.x, ps.ro.y, ps.ro.z, 0.0f);
-                    v.rd[j] = make_float4(ps.rd.x, ps.rd.y, ps.rd.z, ps.prevPdf);
+                    put_ray(v, j, ps, id.w);
                     pushRay = true;
                 }
-                v.rad[j] = make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, depth0);
                 if (!cont && !anyLight) write_record(v, j, ps.radiance, depth0);
             }
         }
@@ -804,8 +825,9 @@ __global__ void __launch_bounds__(256) wf_miss(WfView v, DevScene s, uint32_t de
     NullCounter ctr;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t j = v.shadeQ[v.P - 1u - i];
-        const DevRequest& q = v.reqs[v.ident[j].w].q;
-        const float4 d = v.rd[j], t4 = v.T[j], r4 = v.rad[j];
+        const F4Pair ry = ld_pair(&v.ray[j]), sp = ld_pair(&v.st[j]);
+        const DevRequest& q = v.reqs[__float_as_uint(ry.a.w)].q;
+        const float4 d = ry.b, t4 = sp.a, r4 = sp.b;
         const uint32_t bits = __float_as_uint(t4.w);
         PathState ps;
         ps.rd = V3{d.x, d.y, d.z};
@@ -844,13 +866,13 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_occlude(WfView v, DevScene
                 const uint32_t item = sq[got];
                 const uint32_t j = item >> 3, k = item & 7u;
                 e = static_cast<size_t>(k) * v.P + j;
-                const float4 o4 = v.shOrigin[j], d4 = v.shDir[e];
+                const float4 o4 = v.shVtx[j].a, d4 = v.shLight[e].a;
                 wide_init(t, V3{o4.x, o4.y, o4.z}, V3{d4.x, d4.y, d4.z}, d4.w);
             }
             if (__ballot_sync(kFull, t.node != kNoNode || wide_has_tri(t.tBits)) == 0u) break;
             const auto test = [&] {
                 if (wide_test_any(s, t)) {
-                    v.shDir[e].w = 0.0f;
+                    v.shLight[e].a.w = 0.0f;
                     t.node = kNoNode;
                     t.tBits = 0u;
                 }
@@ -877,7 +899,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_occlude(WfView v, DevScene
                 const uint32_t item = sq[i];
                 const uint32_t j = item >> 3, k = item & 7u;
                 e = static_cast<size_t>(k) * v.P + j;
-                const float4 o4 = v.shOrigin[j], d4 = v.shDir[e];
+                const float4 o4 = v.shVtx[j].a, d4 = v.shLight[e].a;
                 wide_init(t, V3{o4.x, o4.y, o4.z}, V3{d4.x, d4.y, d4.z}, d4.w);
             }
             bool occluded = false;
@@ -888,7 +910,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_occlude(WfView v, DevScene
                     t.node = kNoNode;
                 }
             }
-            if (occluded) v.shDir[e].w = 0.0f;
+            if (occluded) v.shLight[e].a.w = 0.0f;
         }
         return;
     }
@@ -900,8 +922,8 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_occlude(WfView v, DevScene
         const uint32_t item = sq[i];
         const uint32_t j = item >> 3, k = item & 7u;
         const size_t e = static_cast<size_t>(k) * v.P + j;
-        const float4 o4 = v.shOrigin[j], d4 = v.shDir[e];
-        if (trace_occluded(s, V3{o4.x, o4.y, o4.z}, V3{d4.x, d4.y, d4.z}, d4.w, ctr)) v.shDir[e].w = 0.0f;
+        const float4 o4 = v.shVtx[j].a, d4 = v.shLight[e].a;
+        if (trace_occluded(s, V3{o4.x, o4.y, o4.z}, V3{d4.x, d4.y, d4.z}, d4.w, ctr)) v.shLight[e].a.w = 0.0f;
     }
 }
 
@@ -910,20 +932,22 @@ __global__ void __launch_bounds__(256) wf_shadow(WfView v, DevScene s, uint32_t 
     const uint32_t count = counter(v, 2);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t j = v.shadowQ[i];
-        const DevRequest& q = v.reqs[v.ident[j].w].q;
-        const float4 t4 = v.shT[j], r4 = v.rad[j];
+        const F4Pair vt = ld_pair(&v.shVtx[j]);
+        const DevRequest& q = v.reqs[__float_as_uint(vt.a.w)].q;
+        const float4 t4 = vt.b, r4 = v.st[j].b;
         uint32_t visible = 0;
         const V3 direct = sum_direct<true>(s, q, [&](uint32_t k, V3* c) {
             const size_t e = static_cast<size_t>(k) * v.P + j;
-            if (v.shDir[e].w == 0.0f) return false;
-            const float4 c4 = v.shC[e];
+            const F4Pair sl = ld_pair(&v.shLight[e]);
+            if (sl.a.w == 0.0f) return false;
+            const float4 c4 = sl.b;
             *c = V3{c4.x, c4.y, c4.z};
             visible |= 1u << k;
             return true;
         });
         if (v.visLog) v.visLog[static_cast<size_t>(depth) * v.P + j] = static_cast<uint8_t>(visible);
         const V3 rad = V3{r4.x, r4.y, r4.z} + V3{t4.x, t4.y, t4.z} * direct;
-        v.rad[j] = make_float4(rad.x, rad.y, rad.z, r4.w);
+        v.st[j].b = make_float4(rad.x, rad.y, rad.z, r4.w);
         if (t4.w != 0.0f) write_record(v, j, rad, r4.w);  // the path ends here
     }
 }
@@ -1025,9 +1049,8 @@ __global__ void __launch_bounds__(128) wa_generate(WfView v, AdjWave aw) {
             const Sampler smp{x, y, smpIdx, nullptr};
             PathState ps;
             init_path(q, smp, ps);
-            v.ro[j] = make_float4(ps.ro.x, ps.ro.y, ps.ro.z, 0.0f);
-            v.rd[j] = make_float4(ps.rd.x, ps.rd.y, ps.rd.z, ps.prevPdf);
-            v.T[j] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(kFlagPrevDelta));
+            put_ray(v, j, ps, sg.req);
+            v.st[j].a = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(kFlagPrevDelta));
             v.ident[j] = make_uint4(x, y, smpIdx, sg.req);
             const float cnt = static_cast<float>(q.sampleCount);
             const float4 g = reinterpret_cast<const float4*>(a.dBeauty)[pix];
@@ -1161,7 +1184,8 @@ constexpr int kReplayBlocks = 6;
 template <bool kExt>
 __device__ __forceinline__ bool wa_vertex(const WfView& v, const DevScene& s, uint32_t j, const Sampler& smp, uint32_t depth,
                                           PathState& ps, Vertex& vx) {
-    const float4 o = v.ro[j], d = v.rd[j], t4 = v.T[j], h4 = v.hit[j];
+    const F4Pair ry = ld_pair(&v.ray[j]);
+    const float4 o = ry.a, d = ry.b, t4 = v.st[j].a, h4 = v.hit[j];
     const uint32_t bits = __float_as_uint(t4.w);
     ps.ro = V3{o.x, o.y, o.z};
     ps.rd = V3{d.x, d.y, d.z};
@@ -1319,9 +1343,8 @@ __global__ void __launch_bounds__(128, kReplayBlocks) wa_continue(WfView v, DevS
                 }
             } while (false);
             if (pushRay) {
-                v.T[j] = make_float4(ps.T.x, ps.T.y, ps.T.z, __uint_as_float(pack_state(ps)));
-                v.ro[j] = make_float4(ps.ro.x, ps.ro.y, ps.ro.z, 0.0f);
-                v.rd[j] = make_float4(ps.rd.x, ps.rd.y, ps.rd.z, ps.prevPdf);
+                v.st[j].a = make_float4(ps.T.x, ps.T.y, ps.T.z, __uint_as_float(pack_state(ps)));
+                put_ray(v, j, ps, id.w);
             }
         }
         warp_push(cout, qout, pushRay, j);
@@ -1335,9 +1358,10 @@ __global__ void __launch_bounds__(256) wa_miss(WfView v, DevScene s, AdjWave aw,
     if (a.env0 < 0 || !a.dEnv4) return;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const uint32_t j = v.shadeQ[v.P - 1u - i];
-        const DevRequest& q = v.reqs[v.ident[j].w].q;
+        const F4Pair ry = ld_pair(&v.ray[j]);
+        const DevRequest& q = v.reqs[__float_as_uint(ry.a.w)].q;
         if (!(depth > 0 || q.backgroundVisible)) continue;
-        const float4 d = v.rd[j], t4 = v.T[j], dl4 = aw.delta[j];
+        const float4 d = ry.b, t4 = v.st[j].a, dl4 = aw.delta[j];
         const V3 rd{d.x, d.y, d.z};
         const bool prevDelta = (__float_as_uint(t4.w) & kFlagPrevDelta) != 0u;
         const float mis = (s.domeCount == 0 || depth == 0 || prevDelta) ? 1.0f : env_miss_mis(s, d.w, rd);
@@ -1467,18 +1491,13 @@ WfView make_view(WavePool* wf, uint32_t P, uint32_t lightSamples, const WaveDesc
     std::memset(&v, 0, sizeof(v));  // padding too: the bytes key the graph cache
     const size_t p = P;
     char* st = static_cast<char*>(wf->state.ptr);
-    v.ro = reinterpret_cast<float4*>(st);
-    v.rd = v.ro + p;
-    v.T = v.rd + p;
-    v.rad = v.T + p;
-    v.ident = reinterpret_cast<uint4*>(v.rad + p);
+    v.ray = reinterpret_cast<F4Pair*>(st);
+    v.st = v.ray + p;
+    v.ident = reinterpret_cast<uint4*>(v.st + p);
     v.hit = reinterpret_cast<float4*>(v.ident + p);
     v.medium = v.hit + p;
-    float4* sh = static_cast<float4*>(wf->shadow.ptr);
-    v.shOrigin = sh;
-    v.shT = sh + p;
-    v.shDir = sh + 2 * p;
-    v.shC = sh + (2 + static_cast<size_t>(std::max(1u, lightSamples))) * p;
+    v.shVtx = static_cast<F4Pair*>(wf->shadow.ptr);
+    v.shLight = v.shVtx + p;
     uint32_t* qb = static_cast<uint32_t*>(wf->queues.ptr);
     v.counters = qb;
     v.rayQ0 = qb + kCounters * kCounterStride;
