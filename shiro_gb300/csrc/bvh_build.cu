@@ -831,14 +831,15 @@ __global__ void k_write_root(float4* out, float4 b0lo, float4 b0hi, int l0, floa
     } while (0)
 
 struct Scratch {
+    DevicePool& pool;
     std::vector<void*> ptrs;
     ~Scratch() {
-        for (void* p : ptrs) cudaFree(p);
+        for (void* p : ptrs) pool.put(p);
     }
     template <typename T>
     cudaError_t alloc(T** p, size_t count) {
         void* v = nullptr;
-        const cudaError_t e = cudaMalloc(&v, count * sizeof(T) + 16);
+        const cudaError_t e = pool.get(&v, count * sizeof(T) + 16);
         if (e == cudaSuccess) ptrs.push_back(v);
         *p = static_cast<T*>(v);
         return e;
@@ -990,7 +991,15 @@ static int sah_top(Scratch& sc, int m, int nInternal, int clusterSize, const uin
     return SHIRO_OK;
 }
 
-int build_bvh(const BvhInput& in, cudaStream_t stream, BvhOutput* out, std::string& err) {
+template <typename T>
+cudaError_t pool_get(DevicePool& pool, T** p, size_t bytes) {
+    void* v = nullptr;
+    const cudaError_t e = pool.get(&v, bytes);
+    *p = static_cast<T*>(v);
+    return e;
+}
+
+int build_bvh(const BvhInput& in, DevicePool& pool, cudaStream_t stream, BvhOutput* out, std::string& err) {
     const uint32_t m = in.smallCount;
     const uint32_t L = static_cast<uint32_t>(in.largeSlots.size());
     const uint32_t total = m + L;
@@ -1006,9 +1015,9 @@ int build_bvh(const BvhInput& in, cudaStream_t stream, BvhOutput* out, std::stri
         err = "leaf size out of range [1, 8]";
         return SHIRO_ERR_INVALID_ARGUMENT;
     }
-    Scratch sc;
+    Scratch sc{pool, {}};
     float4* triOut = nullptr;
-    BVH_CHECK(cudaMalloc(&triOut, 3 * sizeof(float4) * static_cast<size_t>(total)));
+    BVH_CHECK(pool_get(pool, &triOut, 3 * sizeof(float4) * static_cast<size_t>(total)));
     out->tris = triOut;
     out->triCount = total;
 
@@ -1140,7 +1149,7 @@ int build_bvh(const BvhInput& in, cudaStream_t stream, BvhOutput* out, std::stri
     const uint32_t offset = chain ? L : (needTop ? 1u : 0u);
     const uint32_t nodeCountOut = offset + (mortonTree ? emittedMorton : 0u);
     float4* nodes = nullptr;
-    BVH_CHECK(cudaMalloc(&nodes, 4 * sizeof(float4) * static_cast<size_t>(nodeCountOut)));
+    BVH_CHECK(pool_get(pool, &nodes, 4 * sizeof(float4) * static_cast<size_t>(nodeCountOut)));
     out->nodes = nodes;
     out->nodeCount = nodeCountOut;
     if (mortonTree) {
@@ -1484,9 +1493,9 @@ __global__ void k_collapse_wide(const float4* __restrict__ nodes2, const float4*
 
 }  // namespace
 
-int collapse_wide(const float4* nodes2, uint32_t nodeCount2, const float4* tris2, uint32_t triCount2, cudaStream_t stream,
-                  WideOutput* out, std::string& err) {
-    Scratch sc;
+int collapse_wide(const float4* nodes2, uint32_t nodeCount2, const float4* tris2, uint32_t triCount2, DevicePool& pool,
+                  cudaStream_t stream, WideOutput* out, std::string& err) {
+    Scratch sc{pool, {}};
     int2 *ta = nullptr, *tb = nullptr;
     unsigned int* cnt = nullptr;  // [0] node counter, [1] next task count, [2] triangle counter
     const uint32_t cap = std::max<uint32_t>(nodeCount2, 1);
@@ -1494,10 +1503,10 @@ int collapse_wide(const float4* nodes2, uint32_t nodeCount2, const float4* tris2
     BVH_CHECK(sc.alloc(&tb, cap));
     BVH_CHECK(sc.alloc(&cnt, 3));
     float4* nodes = nullptr;
-    BVH_CHECK(cudaMalloc(&nodes, 5 * sizeof(float4) * static_cast<size_t>(cap)));
+    BVH_CHECK(pool_get(pool, &nodes, 5 * sizeof(float4) * static_cast<size_t>(cap)));
     out->nodes = nodes;
     float4* tris = nullptr;
-    BVH_CHECK(cudaMalloc(&tris, 3 * sizeof(float4) * static_cast<size_t>(std::max<uint32_t>(triCount2, 1))));
+    BVH_CHECK(pool_get(pool, &tris, 3 * sizeof(float4) * static_cast<size_t>(std::max<uint32_t>(triCount2, 1))));
     out->tris = tris;
     // cost table of the slot assignment (bottom-up over the binary tree)
     WideDp dp;

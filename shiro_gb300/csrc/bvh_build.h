@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/shiro_gpu.h"
+#include "pool.h"
 
 namespace shiro_gpu {
 
@@ -30,9 +31,9 @@ struct BvhInput {
 };
 
 struct BvhOutput {
-    float4* nodes = nullptr;  // cudaMalloc'ed, owned by the caller afterwards
+    float4* nodes = nullptr;  // from the pool, owned by the caller afterwards
     uint32_t nodeCount = 0;
-    float4* tris = nullptr;   // cudaMalloc'ed, leaf order
+    float4* tris = nullptr;   // from the pool, leaf order
     uint32_t triCount = 0;
     uint32_t depth = 0;
     uint32_t maxLeaf = 0;
@@ -62,9 +63,9 @@ inline int leaf_link_host(int first, int count) { return ~((first << 3) | (count
 constexpr uint32_t kWideLeaf = 1;  // leaf size of the binary tree the wide BVH is collapsed from
 
 struct WideOutput {
-    float4* nodes = nullptr;  // cudaMalloc'ed, 5 float4 per node
+    float4* nodes = nullptr;  // from the pool, 5 float4 per node
     uint32_t nodeCount = 0;
-    float4* tris = nullptr;   // cudaMalloc'ed, 3 float4 per triangle, wide-leaf order
+    float4* tris = nullptr;   // from the pool, 3 float4 per triangle, wide-leaf order
     uint32_t triCount = 0;
     uint32_t depth = 0;
 };
@@ -73,9 +74,9 @@ struct WideOutput {
 // triangle in `tris2`) into compressed wide nodes; which binary nodes
 // become wide nodes minimises a surface-area cost (optimal collapse over
 // at most 8 slots per node, evaluated bottom-up on the device).
-int collapse_wide(const float4* nodes2, uint32_t nodeCount2, const float4* tris2, uint32_t triCount2, cudaStream_t stream,
-                  WideOutput* out, std::string& err);
+int collapse_wide(const float4* nodes2, uint32_t nodeCount2, const float4* tris2, uint32_t triCount2, DevicePool& pool,
+                  cudaStream_t stream, WideOutput* out, std::string& err);
 
-int build_bvh(const BvhInput& in, cudaStream_t stream, BvhOutput* out, std::string& err);
+int build_bvh(const BvhInput& in, DevicePool& pool, cudaStream_t stream, BvhOutput* out, std::string& err);
 
 }  // namespace shiro_gpu

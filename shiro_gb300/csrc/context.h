@@ -9,6 +9,7 @@
 
 #include "../../include/shiro_gpu.h"
 #include "kernels.h"
+#include "pool.h"
 #include "scene.cuh"
 
 namespace shiro_gpu {
@@ -41,10 +42,12 @@ struct ContextImpl {
     cudaStream_t stream = nullptr;
     std::string lastError;
 
+    DevicePool pool;  // blocks of the scene and of upload scratch
+
     // scene
     bool hasScene = false;
     DevScene scene{};
-    std::vector<DeviceBlock> sceneBlocks;  // geometry blocks first, then shading ones
+    std::vector<DeviceBlock> sceneBlocks;  // geometry blocks first, then shading ones (from the pool)
     size_t geomBlocks = 0;                 // sceneBlocks[0, geomBlocks): BVHs, triangles, shading records
     bool geomValid = false;                // geomSignature describes the resident geometry
     uint64_t geomSignature = 0;
@@ -104,6 +107,8 @@ struct ContextImpl {
 
 // Allocation helpers; on failure they set ctx->lastError and return false.
 bool ensure_block(ContextImpl* ctx, DeviceBlock* b, size_t bytes, const char* what);
+// A block from the context's pool (*b is empty before).
+bool pool_block(ContextImpl* ctx, DeviceBlock* b, size_t bytes, const char* what);
 int fail(ContextImpl* ctx, int code, const std::string& msg);
 int cuda_fail(ContextImpl* ctx, cudaError_t e, const char* what);
 

@@ -206,14 +206,15 @@ __global__ void k_alias_identity(uint2* __restrict__ alias, uint64_t n) {
 
 // Scratch of one build, freed when it goes out of scope.
 struct Scratch {
+    DevicePool& pool;
     std::vector<void*> blocks;
     ~Scratch() {
-        for (void* p : blocks) cudaFree(p);
+        for (void* b : blocks) pool.put(b);
     }
     template <typename T>
     cudaError_t get(T** p, size_t count) {
         void* v = nullptr;
-        const cudaError_t e = cudaMalloc(&v, std::max<size_t>(count * sizeof(T), 16));
+        const cudaError_t e = pool.get(&v, std::max<size_t>(count * sizeof(T), 16));
         if (e == cudaSuccess) blocks.push_back(v);
         *p = static_cast<T*>(v);
         return e;
@@ -241,7 +242,7 @@ int build_env_tables_device(ContextImpl* ctx, DevEnv& d) {
         const float theta = (static_cast<float>(y) + 0.5f) * kHostPi / static_cast<float>(h);
         sines[y] = std::max(std::sin(theta), 1.0e-6f);
     }
-    Scratch sc;
+    Scratch sc{ctx->pool, {}};
     float *dSin, *rowSum;
     u64 *q, *s, *gapD, *gapE, *ld, *heInc, *stats;
     uint32_t *lightFlag, *lpos, *lights, *heavies;

@@ -1,0 +1,83 @@
+// pool.h - device blocks kept by a context between uploads.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstddef>
+#include <map>
+#include <unordered_map>
+
+namespace shiro_gpu {
+
+// Scene uploads and importance-table builds take and give back up to 140
+// device blocks each (an upload of 327 k triangles spent 9 ms in cudaMalloc
+// and cudaFree).  A context keeps the blocks given back, up to kMaxIdle bytes,
+// and hands them out again; they return to the driver past that bound, when an
+// allocation fails, and with the context.  A block is used on the context's
+// stream alone, whose order makes the next use follow the last one; calls on
+// one context are serialised by the caller.
+class DevicePool {
+  public:
+    static constexpr size_t kMaxIdle = size_t(1) << 30;
+
+    DevicePool() = default;
+    DevicePool(const DevicePool&) = delete;
+    DevicePool& operator=(const DevicePool&) = delete;
+    ~DevicePool() { trim(0); }
+
+    cudaError_t get(void** out, size_t bytes) {
+        const size_t size = round(bytes);
+        auto it = idle_.lower_bound(size);
+        if (it != idle_.end() && it->first <= size + size / 4) {
+            *out = it->second;
+            live_[it->second] = it->first;
+            idleBytes_ -= it->first;
+            idle_.erase(it);
+            return cudaSuccess;
+        }
+        cudaError_t e = cudaMalloc(out, size);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            trim(0);
+            e = cudaMalloc(out, size);
+        }
+        if (e == cudaSuccess) live_[*out] = size;
+        else *out = nullptr;
+        return e;
+    }
+
+    void put(void* p) {
+        if (!p) return;
+        const auto it = live_.find(p);
+        if (it == live_.end()) return;
+        idle_.emplace(it->second, p);
+        idleBytes_ += it->second;
+        live_.erase(it);
+        trim(kMaxIdle);
+    }
+
+    // Returns idle blocks, largest first, until at most `keep` bytes are idle.
+    void trim(size_t keep) {
+        while (idleBytes_ > keep) {
+            const auto it = std::prev(idle_.end());
+            idleBytes_ -= it->first;
+            cudaFree(it->second);
+            idle_.erase(it);
+        }
+    }
+
+  private:
+    // 512-byte steps, then an eighth of the power of two below: blocks of
+    // similar size are interchangeable
+    static size_t round(size_t bytes) {
+        size_t step = 512;
+        while (step * 16 < bytes) step <<= 1;
+        return (std::max<size_t>(bytes, 16) + step - 1) / step * step;
+    }
+    std::multimap<size_t, void*> idle_;
+    std::unordered_map<void*, size_t> live_;
+    size_t idleBytes_ = 0;
+};
+
+}  // namespace shiro_gpu

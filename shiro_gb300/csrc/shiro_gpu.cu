@@ -44,7 +44,7 @@ template <typename T>
 int upload(ContextImpl* ctx, const std::vector<T>& v, const T** out, const char* what) {
     DeviceBlock b;
     const size_t bytes = std::max<size_t>(v.size() * sizeof(T), 16);
-    cudaError_t e = cudaMalloc(&b.ptr, bytes);
+    cudaError_t e = ctx->pool.get(&b.ptr, bytes);
     if (e != cudaSuccess) return cuda_fail(ctx, e, what);
     b.bytes = bytes;
     ctx->sceneBlocks.push_back(b);
@@ -98,7 +98,7 @@ ContextImpl::~ContextImpl() {
 }
 
 void ContextImpl::freeScene() {
-    for (auto& b : sceneBlocks) free_block(&b);
+    for (auto& b : sceneBlocks) pool.put(b.ptr);
     sceneBlocks.clear();
     geomBlocks = 0;
     geomValid = false;
@@ -112,7 +112,7 @@ void ContextImpl::freeScene() {
 }
 
 void ContextImpl::freeShading() {
-    for (size_t i = geomBlocks; i < sceneBlocks.size(); ++i) free_block(&sceneBlocks[i]);
+    for (size_t i = geomBlocks; i < sceneBlocks.size(); ++i) pool.put(sceneBlocks[i].ptr);
     sceneBlocks.resize(std::min(geomBlocks, sceneBlocks.size()));
     envDev.clear();
     envHost.clear();
@@ -146,7 +146,24 @@ size_t ContextImpl::deviceBytes() const {
 bool ensure_block(ContextImpl* ctx, DeviceBlock* b, size_t bytes, const char* what) {
     if (b->bytes >= bytes) return true;
     free_block(b);
-    const cudaError_t e = cudaMalloc(&b->ptr, bytes);
+    cudaError_t e = cudaMalloc(&b->ptr, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        ctx->pool.trim(0);  // idle upload blocks go first
+        e = cudaMalloc(&b->ptr, bytes);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        ctx->lastError = std::string(what) + ": cudaMalloc(" + std::to_string(bytes) + "): " + cudaGetErrorString(e);
+        b->ptr = nullptr;
+        return false;
+    }
+    b->bytes = bytes;
+    return true;
+}
+
+bool pool_block(ContextImpl* ctx, DeviceBlock* b, size_t bytes, const char* what) {
+    const cudaError_t e = ctx->pool.get(&b->ptr, bytes);
     if (e != cudaSuccess) {
         cudaGetLastError();
         ctx->lastError = std::string(what) + ": cudaMalloc(" + std::to_string(bytes) + "): " + cudaGetErrorString(e);
@@ -400,7 +417,7 @@ int build_bsdf_recs(ContextImpl* ctx) {
     const uint32_t n = ctx->materialCount + 1u;  // + the default material
     if (!ctx->scene.bsdfRecs) {
         DeviceBlock b;
-        if (!ensure_block(ctx, &b, kBsdfRec * sizeof(float4) * n, "BSDF records")) return SHIRO_ERR_OUT_OF_MEMORY;
+        if (!pool_block(ctx, &b, kBsdfRec * sizeof(float4) * n, "BSDF records")) return SHIRO_ERR_OUT_OF_MEMORY;
         ctx->sceneBlocks.push_back(b);
         ctx->scene.bsdfRecs = static_cast<const float4*>(b.ptr);
     }
@@ -417,7 +434,7 @@ int finish_env(ContextImpl* ctx, size_t k) {
     if (rc != SHIRO_OK) return rc;
     if (!d.samples) {
         DeviceBlock b;
-        if (!ensure_block(ctx, &b, 2 * n * sizeof(float4), "env sample records")) return SHIRO_ERR_OUT_OF_MEMORY;
+        if (!pool_block(ctx, &b, 2 * n * sizeof(float4), "env sample records")) return SHIRO_ERR_OUT_OF_MEMORY;
         ctx->sceneBlocks.push_back(b);
         d.samples = static_cast<const float4*>(b.ptr);
     }
@@ -441,8 +458,7 @@ int upload_envs(ContextImpl* ctx) {
         DeviceBlock& b;
         ContextImpl* ctx;
         ~Free() {
-            if (b.ptr) cudaStreamSynchronize(ctx->stream);  // the conversion read it
-            free_block(&b);
+            ctx->pool.put(b.ptr);  // (its next use follows the conversion on the stream)
         }
     } freeStage{rgbStage, ctx};
     for (size_t k = 0; k < ctx->envHost.size(); ++k) {
@@ -455,14 +471,14 @@ int upload_envs(ContextImpl* ctx) {
         d.hasTable = (e.latlong && n > 0) ? 1u : 0u;
         int rc;
         DeviceBlock tb;
-        if (!ensure_block(ctx, &tb, std::max<size_t>(n, 1) * sizeof(float4), "env texels")) return SHIRO_ERR_OUT_OF_MEMORY;
+        if (!pool_block(ctx, &tb, std::max<size_t>(n, 1) * sizeof(float4), "env texels")) return SHIRO_ERR_OUT_OF_MEMORY;
         ctx->sceneBlocks.push_back(tb);
         d.texels = static_cast<const float4*>(tb.ptr);
         if (n) {
-            if (rgbStage.bytes < 12 * n) {  // grown for the largest texture (a sync frees the old one)
-                if (rgbStage.ptr) cudaStreamSynchronize(ctx->stream);
-                free_block(&rgbStage);
-                if (!ensure_block(ctx, &rgbStage, 12 * n, "env texel staging")) return SHIRO_ERR_OUT_OF_MEMORY;
+            if (rgbStage.bytes < 12 * n) {  // grown for the largest texture
+                ctx->pool.put(rgbStage.ptr);
+                rgbStage = DeviceBlock{};
+                if (!pool_block(ctx, &rgbStage, 12 * n, "env texel staging")) return SHIRO_ERR_OUT_OF_MEMORY;
             }
             cudaError_t ce = cudaMemcpyAsync(rgbStage.ptr, e.rgb, 12 * n, cudaMemcpyHostToDevice, ctx->stream);
             if (ce != cudaSuccess) return cuda_fail(ctx, ce, "env texels");
@@ -472,10 +488,10 @@ int upload_envs(ContextImpl* ctx) {
         }
         if (d.hasTable) {
             DeviceBlock rb, cb, ab;
-            if (!ensure_block(ctx, &rb, (e.h + 1u) * sizeof(float), "env row cdf") ||
-                !ensure_block(ctx, &cb, static_cast<size_t>(e.h) * (e.w + 1u) * sizeof(float), "env conditional cdf") ||
-                !ensure_block(ctx, &ab, n * sizeof(uint2), "env alias")) {
-                for (DeviceBlock* x : {&rb, &cb, &ab}) free_block(x);
+            if (!pool_block(ctx, &rb, (e.h + 1u) * sizeof(float), "env row cdf") ||
+                !pool_block(ctx, &cb, static_cast<size_t>(e.h) * (e.w + 1u) * sizeof(float), "env conditional cdf") ||
+                !pool_block(ctx, &ab, n * sizeof(uint2), "env alias")) {
+                for (DeviceBlock* x : {&rb, &cb, &ab}) ctx->pool.put(x->ptr);
                 return SHIRO_ERR_OUT_OF_MEMORY;
             }
             for (DeviceBlock* x : {&rb, &cb, &ab}) ctx->sceneBlocks.push_back(*x);
@@ -748,7 +764,7 @@ int upload_shading(ContextImpl* ctx, const ShiroSceneDesc* sd) {
     // TriangleArea :198-222), float running sums in mesh / primitive order ----
     std::vector<float4> emissive;
     std::vector<float> emissiveCdf;
-    std::vector<int32_t> emissiveOf(ttotal, -1);
+    std::vector<int32_t> emissiveOf;  // sized by the first emitter
     float emissiveSum = 0.0f;
     {
         const ShiroMaterialDesc dflt = default_material();
@@ -777,6 +793,7 @@ int upload_shading(ContextImpl* ctx, const ShiroSceneDesc* sd) {
                 const float area = dbl * 0.5f;
                 const float sel = area * w;
                 emissiveSum += sel;
+                if (emissiveOf.empty()) emissiveOf.assign(ttotal, -1);
                 emissiveOf[g] = static_cast<int32_t>(emissiveCdf.size());
                 float gbits;
                 std::memcpy(&gbits, &g, 4);
@@ -1082,14 +1099,15 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
         std::memcpy(idx.data(), kPointIdx, sizeof(kPointIdx));
     }
     struct Temps {  // device scratch of the upload
+        DevicePool& pool;
         std::vector<void*> p;
         ~Temps() {
-            for (void* x : p) cudaFree(x);
+            for (void* x : p) pool.put(x);
         }
-    } temps;
+    } temps{ctx->pool, {}};
     auto scratch = [&](size_t bytes, auto** out) -> bool {
         void* v = nullptr;
-        if (cudaMalloc(&v, std::max<size_t>(bytes, 16)) != cudaSuccess) {
+        if (ctx->pool.get(&v, std::max<size_t>(bytes, 16)) != cudaSuccess) {
             cudaGetLastError();
             return false;
         }
@@ -1099,7 +1117,7 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
     };
     auto keep = [&](size_t bytes, auto** out) -> bool {  // geometry kept with the scene
         DeviceBlock blk;
-        if (!ensure_block(ctx, &blk, std::max<size_t>(bytes, 16), "scene geometry")) return false;
+        if (!pool_block(ctx, &blk, std::max<size_t>(bytes, 16), "scene geometry")) return false;
         ctx->sceneBlocks.push_back(blk);
         *out = static_cast<std::remove_pointer_t<decltype(out)>>(blk.ptr);
         return true;
@@ -1207,7 +1225,7 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
     bin.sahClusterSize = ctx->sahClusterSize;
     BvhOutput bout, bwide;
     std::string berr;
-    rc = build_bvh(bin, ctx->stream, &bout, berr);
+    rc = build_bvh(bin, ctx->pool, ctx->stream, &bout, berr);
     // the wide BVH is collapsed from a binary tree with small leaves (the
     // node's triangle bits bound the leaves it can hold); its box test folds
     // 2^23 * scale / direction into a bias, so it is built only while that
@@ -1216,11 +1234,11 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
     if (rc == SHIRO_OK && wideOk) {
         BvhInput small = bin;
         small.maxLeaf = kWideLeaf;
-        rc = build_bvh(small, ctx->stream, &bwide, berr);
+        rc = build_bvh(small, ctx->pool, ctx->stream, &bwide, berr);
     }
-    auto drop = [](BvhOutput& b) {
-        if (b.nodes) cudaFree(b.nodes);
-        if (b.tris) cudaFree(b.tris);
+    auto drop = [&](BvhOutput& b) {
+        ctx->pool.put(b.nodes);
+        ctx->pool.put(b.tris);
         b.nodes = nullptr;
         b.tris = nullptr;
     };
@@ -1237,15 +1255,15 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
     ctx->sceneBlocks.push_back({bout.nodes, 4 * sizeof(float4) * bout.nodeCount});
     ctx->sceneBlocks.push_back({bout.tris, 3 * sizeof(float4) * bout.triCount});
     WideOutput w8;
-    if (wideOk) rc = collapse_wide(bwide.nodes, bwide.nodeCount, bwide.tris, bwide.triCount, ctx->stream, &w8, berr);
+    if (wideOk) rc = collapse_wide(bwide.nodes, bwide.nodeCount, bwide.tris, bwide.triCount, ctx->pool, ctx->stream, &w8, berr);
     drop(bwide);
     if (rc == SHIRO_OK && w8.depth > static_cast<uint32_t>(kStackWide)) {
         rc = SHIRO_ERR_INVALID_ARGUMENT;
         berr = "deeper than the traversal stack";
     }
     if (rc != SHIRO_OK) {
-        if (w8.nodes) cudaFree(w8.nodes);
-        if (w8.tris) cudaFree(w8.tris);
+        ctx->pool.put(w8.nodes);
+        ctx->pool.put(w8.tris);
         return fail(ctx, rc, "wide BVH: " + berr);
     }
     if (w8.nodes) ctx->sceneBlocks.push_back({w8.nodes, 5 * sizeof(float4) * std::max<uint32_t>(bwide.nodeCount, 1)});
