@@ -23,7 +23,6 @@ struct BvhInput {
     const float4* centroids;  // device, 1 per small triangle
     uint32_t smallCount;
     std::vector<LargeTri> largeSlots;  // at most 8
-    uint32_t maxLeaf = 8;              // largest SAH leaf (1..8)
     // > 0: the Morton tree's subtrees of at most this many triangles are kept
     // as clusters and the tree above them is rebuilt by binned SAH; 0: the
     // Morton (LBVH) hierarchy throughout
@@ -33,7 +32,8 @@ struct BvhInput {
 struct BvhOutput {
     float4* nodes = nullptr;  // from the pool, owned by the caller afterwards
     uint32_t nodeCount = 0;
-    float4* tris = nullptr;   // from the pool, leaf order
+    float4* tris = nullptr;   // from the pool, leaf order (one array for all trees of a build)
+    bool ownsTris = false;    // the caller frees tris with this tree
     uint32_t triCount = 0;
     uint32_t depth = 0;
     uint32_t maxLeaf = 0;
@@ -60,7 +60,8 @@ inline int leaf_link_host(int first, int count) { return ~((first << 3) | (count
 // ((s & 1) ? -x : +x, (s & 2) ? -y : +y, (s & 4) ? -z : +z) from the node
 // centre, so a ray visits slots in the order of s ^ (7 ^ octant) to go
 // roughly front to back without sorting.
-constexpr uint32_t kWideLeaf = 1;  // leaf size of the binary tree the wide BVH is collapsed from
+constexpr uint32_t kBinaryLeaf = 8;  // largest SAH leaf of the binary BVH
+constexpr uint32_t kWideLeaf = 1;    // leaf size of the binary tree the wide BVH is collapsed from
 
 struct WideOutput {
     float4* nodes = nullptr;  // from the pool, 5 float4 per node
@@ -77,6 +78,13 @@ struct WideOutput {
 int collapse_wide(const float4* nodes2, uint32_t nodeCount2, const float4* tris2, uint32_t triCount2, DevicePool& pool,
                   cudaStream_t stream, WideOutput* out, std::string& err);
 
-int build_bvh(const BvhInput& in, DevicePool& pool, cudaStream_t stream, BvhOutput* out, std::string& err);
+// Builds one hierarchy and from it a tree per entry of `trees`, which differ in
+// their largest leaf (1..8) alone.
+struct BvhTree {
+    uint32_t maxLeaf;
+    BvhOutput* out;
+};
+int build_bvhs(const BvhInput& in, DevicePool& pool, cudaStream_t stream, const BvhTree* trees, uint32_t treeCount,
+               std::string& err);
 
 }  // namespace shiro_gpu

@@ -1225,20 +1225,16 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
     bin.sahClusterSize = ctx->sahClusterSize;
     BvhOutput bout, bwide;
     std::string berr;
-    rc = build_bvh(bin, ctx->pool, ctx->stream, &bout, berr);
     // the wide BVH is collapsed from a binary tree with small leaves (the
     // node's triangle bits bound the leaves it can hold); its box test folds
     // 2^23 * scale / direction into a bias, so it is built only while that
     // stays far from float overflow (coordinates below 1e9)
     const bool wideOk = mag < 1.0e9f;
-    if (rc == SHIRO_OK && wideOk) {
-        BvhInput small = bin;
-        small.maxLeaf = kWideLeaf;
-        rc = build_bvh(small, ctx->pool, ctx->stream, &bwide, berr);
-    }
+    const BvhTree trees[2] = {{kBinaryLeaf, &bout}, {kWideLeaf, &bwide}};
+    rc = build_bvhs(bin, ctx->pool, ctx->stream, trees, wideOk ? 2u : 1u, berr);
     auto drop = [&](BvhOutput& b) {
         ctx->pool.put(b.nodes);
-        ctx->pool.put(b.tris);
+        if (b.ownsTris) ctx->pool.put(b.tris);
         b.nodes = nullptr;
         b.tris = nullptr;
     };
