@@ -83,7 +83,7 @@ struct ContextImpl {
     DeviceBlock pathRecords;
     DeviceBlock aovScratch;
     DeviceBlock probeScratch;
-    uint32_t* errorWord = nullptr;
+    uint32_t* errorWord = nullptr;  // 16 bytes: the error word, the plain form's path counter
     float* radicalTable = nullptr;  // DevScene::radical, built when the context is created
     // device address of the static path-record array of shiro_gpu_render_static
     // (render_static.cu), looked up when the context is created; staticError

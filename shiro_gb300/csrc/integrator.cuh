@@ -557,7 +557,8 @@ __device__ __forceinline__ void init_path(const DevRequest& q, const Sampler& sm
     ps.extinction = V3{0.0f, 0.0f, 0.0f};
 }
 
-// The whole path in one thread (the plain form).
+// The whole path in one thread (the work-counting and per-path diagnostics; the
+// plain form takes the same steps warp by warp).
 template <bool kExt, typename Ctr>
 __device__ __forceinline__ PathResult trace_path(const DevScene& s, const DevRequest& q, uint32_t x, uint32_t y,
                                                  uint32_t sampleIndex, Ctr& ctr) {

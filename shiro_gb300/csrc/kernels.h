@@ -18,7 +18,7 @@ struct AovPtrs {
     float* depth;   // 1
 };
 
-// One thread per path: paths [pathBase, pathBase + count) of the request,
+// The plain form: paths [pathBase, pathBase + count) of the request,
 // path p = pixel * sampleCount + s (sample index sampleStart + s).
 void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBase, uint32_t count, float4* records,
                         cudaStream_t stream);

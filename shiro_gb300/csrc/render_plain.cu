@@ -1,37 +1,136 @@
-// render_plain.cu - the plain GPU form: one thread per path.
+// render_plain.cu - the plain GPU form: one launch follows every path to its end.
 //
 // CpuPathTracer::RenderSampleBatch (src/backend/cpu/CpuPathTracer.cpp:
 // 2043-2170) loops pixels on host threads and samples inside each pixel; here
-// every (pixel, sample) path is one CUDA thread running the whole estimator
-// (camera ray, traversal, shading, next-event estimation, Russian roulette)
-// to completion, and writes a 48-byte record.  A second kernel sums each
+// a lane runs the whole estimator of a (pixel, sample) path (camera ray,
+// traversal, shading, next-event estimation, Russian roulette), writes a
+// 48-byte record and takes the next path.  A second kernel sums each
 // pixel's records in sample order, so the batch average is formed with the
 // same additions, in the same order, as the reference.
+#include <algorithm>
+
 #include "integrator.cuh"
 #include "kernels.h"
+#include "lanes.cuh"
 
 namespace shiro_gpu {
 
 namespace {
 
-// Four blocks of 128 per SM (a 128-register cap, a few bytes of spills):
-// measured 11 % faster than the 165 registers the compiler otherwise takes.
-template <bool kExt>
-__global__ void __launch_bounds__(128, 4) k_plain_paths(const DevScene s, const DevRequest q, uint64_t pathBase,
-                                                     uint32_t count, float4* __restrict__ records) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const uint64_t path = pathBase + i;
-    const uint64_t pixel = path / q.sampleCount;
-    const uint32_t smp = static_cast<uint32_t>(path - pixel * q.sampleCount);
-    const uint32_t y = static_cast<uint32_t>(pixel / q.width);
-    const uint32_t x = static_cast<uint32_t>(pixel - static_cast<uint64_t>(y) * q.width);
+// A warp's lanes pass the steps of a bounce together: the lanes with a path
+// trace it to its next vertex, each light sample's shadow rays are traced side
+// by side (warp_closest, warp_occluded), and lanes whose path has ended take
+// the next path once kPlainRefill of them are idle.  With a thread per path
+// that ran on its own, warps came apart at the first branch and stayed apart
+// (7.3 of 32 lanes active on the 961x541 15-spp field frame); bound by the
+// latency of the tree's loads, the kernel then wants warps in flight rather
+// than registers: at 128, 80, 64, 48 and 40 registers a thread (4, 6, 8, 10,
+// 12 blocks of 128 per SM) that frame takes 18.6, 16.6, 14.9, 13.6 and 13.0 ms
+// (19.5 with a thread per path), the 1280x720 2-spp one 2.57, 2.37, 2.20, 2.09
+// and 2.06 (2.62), 640x480 8 spp with every lobe 10.5 (15.0); 32 registers
+// lose on small scenes again.  Lanes 1, 4, 8 idle: no difference; a warp that
+// waits for all its paths takes 15.0 instead of 13.8 ms.  Pieces of paths left
+// to be continued by whichever lanes stand at the same step were three times
+// slower: the light samples then run a few lanes at a time.
+//
+// A launch too small to fill kPlainBlocksSmall blocks per SM has no use for
+// more warps and keeps its registers (one path per lane, 96x64 pixels of a
+// sphere: 198 us, 224 with 48 registers; 256x256 303 and
+// 353 us).
+constexpr int kPlainBlocks = 12, kPlainBlocksSmall = 4, kPlainRefill = 4;
+constexpr uint32_t kPlainThreads = 128, kPlainChunk = 32;
+
+template <bool kExt, int kBlocks>
+__global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __grid_constant__ DevScene s,
+                                                                        const __grid_constant__ DevRequest q,
+                                                                        uint64_t pixelBase, uint32_t count,
+                                                                        uint32_t* __restrict__ next,
+                                                                        float4* __restrict__ records) {
     NullCounter ctr;
-    const PathResult r = trace_path<kExt>(s, q, x, y, q.sampleStart + smp, ctr);
-    float4* o = records + 3 * static_cast<size_t>(i);
-    o[0] = make_float4(r.radiance.x, r.radiance.y, r.radiance.z, r.depth);
-    o[1] = make_float4(r.albedo.x, r.albedo.y, r.albedo.z, 0.0f);
-    o[2] = make_float4(r.normal.x, r.normal.y, r.normal.z, 0.0f);
+    PathState ps;
+    Sampler smp{0u, 0u, 0u, s.radical};
+    bool alive = false;
+    uint32_t path = 0, depth = 0;
+    float depth0 = 0.0f;
+    const uint32_t nls = light_sample_count<kExt>(s, q), domeEnd = s.distantCount + s.domeCount * q.domeSamples;
+    const float domeDiv = static_cast<float>(q.domeSamples);
+    // the first path of a lane is its own index, the rest come from the queue
+    const uint32_t lanes = gridDim.x * kPlainThreads, queued = count > lanes ? count - lanes : 0u;
+    uint32_t got = blockIdx.x * kPlainThreads + threadIdx.x;
+    if (got >= count) got = 0xffffffffu;
+    LaneFeed feed;
+    for (;;) {
+        if (got != 0xffffffffu) {
+            path = got;
+            const uint32_t local = path / q.sampleCount;
+            const uint64_t pixel = pixelBase + local;
+            const uint64_t y = pixel / q.width;
+            smp.px = static_cast<uint32_t>(pixel - y * q.width);
+            smp.py = static_cast<uint32_t>(y);
+            smp.index = q.sampleStart + (path - local * q.sampleCount);
+            init_path(q, smp, ps);
+            depth = 0;
+            depth0 = __int_as_float(0x7f800000);
+            alive = true;
+        }
+        if (__ballot_sync(kFull, alive) == 0u) break;
+        bool on = alive && q.maxDepth != 0u;
+        HitRec h;
+        const bool found = warp_closest(s, on, ps.ro, ps.rd, &h);
+        __syncwarp();
+        bool shaded = false;
+        Vertex v;
+        if (on) {
+            if (!found) {
+                add_miss(s, q, ps, depth, ctr);
+                on = false;
+            } else {
+                v = make_vertex(s, ps.ro, ps.rd, h);
+                shaded = true;
+                if constexpr (kExt) shaded = enter_hit(s, smp, depth, v, h.t, ps);
+                if (shaded) {
+                    if (depth == 0) {
+                        const float4 dc = __ldg(bsdf_rec(s, v.hit.material) + 3);  // DiffuseColor
+                        const V3 nn = v.n * 0.5f + V3{0.5f, 0.5f, 0.5f};
+                        float4* o = records + 3 * static_cast<size_t>(path);
+                        o[1] = make_float4(dc.x, dc.y, dc.z, 0.0f);
+                        o[2] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+                        depth0 = h.t;
+                    }
+                    if constexpr (kExt) add_emission(s, v, depth, ps);
+                }
+            }
+        }
+        // sum_direct, its shadow rays a sample at a time for the whole warp
+        V3 out{0.0f, 0.0f, 0.0f}, acc{0.0f, 0.0f, 0.0f};
+        for (uint32_t k = 0;; ++k) {
+            if (k > s.distantCount && k <= domeEnd && (k - s.distantCount) % q.domeSamples == 0u) {
+                out = out + acc / domeDiv;
+                acc = V3{0.0f, 0.0f, 0.0f};
+            }
+            if (k >= nls) break;
+            V3 dir, c;
+            float reach = 0.0f;
+            const bool lit = shaded && light_sample<kExt>(s, q, v, smp, depth, k, &dir, &c, &reach, ctr);
+            __syncwarp();
+            const bool blocked = warp_occluded(s, lit, shadow_origin(v), dir, reach);
+            if (lit && !blocked) {
+                if (k >= s.distantCount && k < domeEnd) acc = acc + c;
+                else out = out + c;
+            }
+        }
+        __syncwarp();
+        if (shaded) {
+            ps.radiance = ps.radiance + ps.T * out;
+            on = continue_path<kExt>(s, q, v, smp, depth, ps, ctr);
+        }
+        if (on) on = ++depth < q.maxDepth;
+        if (alive && !on)
+            records[3 * static_cast<size_t>(path)] = make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, depth0);
+        alive = on;
+        got = feed_lanes<kPlainChunk>(feed, next, queued, alive, kPlainRefill);
+        if (got != 0xffffffffu) got += lanes;
+    }
 }
 
 __global__ void k_resolve(const DevRequest q, uint64_t pixelBase, uint32_t count, const float4* __restrict__ records,
@@ -44,13 +143,17 @@ __global__ void k_resolve(const DevRequest q, uint64_t pixelBase, uint32_t count
     float depth = __int_as_float(0x7f800000);
     const float4* r = records + 3 * static_cast<size_t>(i) * n;
     for (uint32_t k = 0; k < n; ++k) {
-        const float4 a = r[3 * k], b = r[3 * k + 1], c = r[3 * k + 2];
+        const float4 a = r[3 * k];
         b0 = b0 + a.x;
         b1 = b1 + a.y;
         b2 = b2 + a.z;
-        b3 = b3 + (a.w < __int_as_float(0x7f800000) ? 1.0f : 0.0f);
-        alb = alb + V3{b.x, b.y, b.z};
-        nrm = nrm + V3{c.x, c.y, c.z};
+        const bool hit = a.w < __int_as_float(0x7f800000);
+        b3 = b3 + (hit ? 1.0f : 0.0f);
+        if (hit) {  // without a shaded first hit albedo and normal are zero (and not in the record)
+            const float4 b = r[3 * k + 1], c = r[3 * k + 2];
+            alb = alb + V3{b.x, b.y, b.z};
+            nrm = nrm + V3{c.x, c.y, c.z};
+        }
         if (a.w < depth) depth = a.w;
     }
     const float cnt = static_cast<float>(n);
@@ -192,10 +295,25 @@ void launch_qmc_table(float* table, cudaStream_t stream) {
 void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBase, uint32_t count, float4* records,
                         cudaStream_t stream) {
     if (count == 0) return;
+    int device = 0, sms = 1;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const unsigned blocks = grid(count, kPlainThreads);
+    const uint64_t pixelBase = pathBase / q.sampleCount;
+    uint32_t* next = s.error + 1;  // the path queue's counter
+    if (blocks <= static_cast<unsigned>(kPlainBlocksSmall * sms)) {
+        if (s.extended)
+            k_plain_paths<true, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
+        else
+            k_plain_paths<false, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
+        return;
+    }
+    const unsigned resident = std::min(blocks, static_cast<unsigned>(kPlainBlocks * sms));
+    if (resident < blocks) cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
     if (s.extended)
-        k_plain_paths<true><<<grid(count, 128), 128, 0, stream>>>(s, q, pathBase, count, records);
+        k_plain_paths<true, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
     else
-        k_plain_paths<false><<<grid(count, 128), 128, 0, stream>>>(s, q, pathBase, count, records);
+        k_plain_paths<false, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
 }
 
 void launch_render_paths(const DevScene& s, const DevRequest& q, const uint32_t* pixels, const uint32_t* sampleIdx,
@@ -215,8 +333,10 @@ void launch_env_pick(const DevEnv& e, const float2* u, uint32_t n, bool useCdf, 
 
 cudaError_t preload_plain_kernels() {
     cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, k_plain_paths<false>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_paths<true>);
+    cudaError_t e = cudaFuncGetAttributes(&a, k_plain_paths<false, kPlainBlocks>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_paths<true, kPlainBlocks>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_paths<false, kPlainBlocksSmall>);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_paths<true, kPlainBlocksSmall>);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_resolve);
     return e;
 }

@@ -17,6 +17,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "lanes.cuh"
 #include "scene.cuh"
 
 namespace shiro_gpu {
@@ -335,6 +336,36 @@ __device__ __forceinline__ bool wide_test_any(const DevScene& s, WideTrav& t) {
     return tri_test(t.o, t.d, kRayEpsilon, t.tmax, ta, tb, tc, &tt, &u, &v);
 }
 
+// One step of a warp's wide-BVH traversal: every lane that has a node and no
+// triangle pending visits it; pending triangles wait until kTriLanes lanes
+// hold some (or no lane has a node to visit) and are then tested by those
+// lanes together until fewer than kTriStop hold any (postponed leaves, Ylitie,
+// Karras and Laine 2017).  Tested as soon as a lane finds them, a warp ran its
+// triangle tests for the one or two lanes that had just reached a leaf; on the
+// 1080p field frame nodes are now visited by 24.5 of 32 lanes and triangles
+// tested by 10.4, and the frame takes 112.3 ms instead of 117.9 (kTriLanes 5:
+// 113.3, 12: 113.6, 16: 116.1, 20: 120.1; kTriStop 4: 116.4, 8: 127.9 - lanes
+// left with triangles visit no node).  Holding a second node's triangles per
+// lane, so that fewer wait, costs more registers than it gains (110 against
+// 107.9 ms).  False when no lane has anything left.  Warp-uniform call.
+constexpr int kTriLanes = 8;
+constexpr int kTriStop = 2;
+
+template <typename Visit, typename Test>
+__device__ __forceinline__ bool trav_step(WideTrav& t, Visit&& visit, Test&& test) {
+    if (t.node != kNoNode && !wide_has_tri(t.tBits)) visit();
+    uint32_t pend = __ballot_sync(kFull, wide_has_tri(t.tBits));
+    const uint32_t run = __ballot_sync(kFull, t.node != kNoNode && !wide_has_tri(t.tBits));
+    if (run == 0u && pend == 0u) return false;
+    if (__popc(pend) >= kTriLanes || run == 0u) {
+        do {
+            if (wide_has_tri(t.tBits)) test();
+            pend = __ballot_sync(kFull, wide_has_tri(t.tBits));
+        } while (__popc(pend) >= kTriStop);
+    }
+    return true;
+}
+
 // The one-thread forms test a node's triangles before they move on: with the
 // move first, lanes without triangles ran ahead of the others and the warp
 // fell apart (90 instead of 31 ms for the 961x541 15-spp field frame).
@@ -527,6 +558,153 @@ __device__ __noinline__ bool trace_occluded(const DevScene& s, const V3 o, const
         if (sp == 0) return false;
         node = stackNode[--sp];
     }
+}
+
+// ---- warp forms ----
+//
+// A warp's rays traced side by side: all 32 lanes call, `on` marks the lanes
+// that have a ray, and the results are those of trace_closest and
+// trace_occluded (a lane takes the same steps in the same order).  Left to the
+// compiler, lanes whose traversals take different branches stay apart and the
+// warp runs them one by one; here the ballots of every step bring the lanes
+// together again.  Binary leaves wait until kBinLeafLanes lanes have reached
+// one or no lane has a node left (1: 18.8 ms for the 961x541 15-spp field frame
+// in the plain form, 4: 18.6, 8: 18.7).  The two trees have functions of their
+// own: one function with both keeps the registers and the stack of the larger,
+// 15.8 instead of 13.6 ms.
+constexpr int kBinLeafLanes = 4;
+constexpr int kBinDone = static_cast<int>(0x80000000u);  // no node (no leaf is encoded so)
+
+template <bool kAny>
+__device__ __forceinline__ uint32_t warp_binary(const DevScene& s, bool on, const V3& o, const V3& d, float maxDist,
+                                                HitRec* out) {
+    const RayInv r = ray_inv(o, d);
+    float bestT = maxDist;
+    uint32_t bestGid = 0xffffffffu;
+    float bu = 0.0f, bv = 0.0f;
+    int stackNode[kStack];
+    float stackT[kAny ? 1 : kStack];
+    int sp = 0;
+    int node = on ? 0 : kBinDone;
+    uint32_t visits = 0;
+    for (;;) {
+        const uint32_t leaves = __ballot_sync(kFull, node < 0 && node != kBinDone);
+        const uint32_t inner = __ballot_sync(kFull, node >= 0);
+        if ((leaves | inner) == 0u) break;
+        const bool testLeaves = __popc(leaves) >= kBinLeafLanes || inner == 0u;
+        bool pop = false;
+        if (node >= 0) {
+            if (++visits > kMaxVisits) {
+                atomicOr(s.error, kErrTraversalLimit);
+                bestGid = 0xffffffffu;
+                node = kBinDone;
+            } else {
+                const float4* np = s.nodes + 4 * static_cast<size_t>(node);
+                const float4 n0 = __ldg(np), n1 = __ldg(np + 1), n2 = __ldg(np + 2), n3 = __ldg(np + 3);
+                float t0, t1;
+                bool h0, h1;
+                node_boxes(n0, n1, n2, r, bestT, &t0, &t1, &h0, &h1);
+                const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
+                const bool swap = h1 && (!h0 || t1 < t0);
+                node = swap ? c1 : c0;
+                if (h0 && h1) {
+                    if (sp < kStack) {
+                        stackNode[sp] = swap ? c0 : c1;
+                        if constexpr (!kAny) stackT[sp] = swap ? t0 : t1;
+                        ++sp;
+                    } else {
+                        atomicOr(s.error, kErrStackOverflow);
+                        bestGid = 0xffffffffu;
+                        node = kBinDone;
+                    }
+                }
+                pop = !(h0 || h1);
+            }
+        } else if (testLeaves && node != kBinDone) {
+            const uint32_t enc = ~static_cast<uint32_t>(node);
+            const uint32_t first = enc >> 3, cnt = (enc & 7u) + 1u;
+            pop = true;
+            for (uint32_t k = first; k < first + cnt; ++k) {
+                const float4* tp = s.tris + 3 * static_cast<size_t>(k);
+                const float4 a = __ldg(tp), b = __ldg(tp + 1), c = __ldg(tp + 2);
+                float t, u, v;
+                if (!tri_test(o, d, kRayEpsilon, kAny ? maxDist : FLT_MAX, a, b, c, &t, &u, &v)) continue;
+                if constexpr (kAny) {
+                    bestGid = 0u;
+                    sp = 0;
+                    break;
+                } else {
+                    const uint32_t gid = __float_as_uint(a.w);
+                    if (t < bestT || (t == bestT && gid < bestGid)) {
+                        bestT = t;
+                        bestGid = gid;
+                        bu = u;
+                        bv = v;
+                    }
+                }
+            }
+        }
+        if (pop) {  // the next entry still in range
+            node = kBinDone;
+            while (sp > 0) {
+                --sp;
+                if (kAny || stackT[kAny ? 0 : sp] <= bestT) {
+                    node = stackNode[sp];
+                    break;
+                }
+            }
+        }
+    }
+    if constexpr (!kAny) *out = HitRec{bestT, bu, bv, bestGid};
+    return bestGid;
+}
+
+static __device__ __noinline__ bool warp_closest_wide(const DevScene& s, bool on, const V3 o, const V3 d, HitRec* out) {
+    WideTrav t;
+    uint2 stack[kStackWide];
+    wide_init(t, o, d, FLT_MAX);
+    if (!on) t.node = kNoNode;
+    while (trav_step(t, [&] { wide_visit(s, t, stack); }, [&] { wide_test_closest(s, t); })) {
+    }
+    *out = HitRec{t.tmax, t.bu, t.bv, t.bestGid};
+    return t.bestGid != 0xffffffffu;
+}
+
+static __device__ __noinline__ bool warp_occluded_wide(const DevScene& s, bool on, const V3 o, const V3 d, float maxDist) {
+    WideTrav t;
+    uint2 stack[kStackWide];
+    wide_init(t, o, d, maxDist);
+    if (!on) t.node = kNoNode;
+    bool hit = false;
+    const auto test = [&] {
+        if (!wide_test_any(s, t)) return;
+        hit = true;
+        t.node = kNoNode;
+        t.tBits = 0u;
+    };
+    while (trav_step(t, [&] { wide_visit(s, t, stack); }, test)) {
+    }
+    return hit;
+}
+
+static __device__ __noinline__ bool warp_closest_binary(const DevScene& s, bool on, const V3 o, const V3 d, HitRec* out) {
+    return warp_binary<false>(s, on, o, d, FLT_MAX, out) != 0xffffffffu;
+}
+
+static __device__ __noinline__ bool warp_occluded_binary(const DevScene& s, bool on, const V3 o, const V3 d, float maxDist) {
+    return warp_binary<true>(s, on, o, d, maxDist, nullptr) != 0xffffffffu;
+}
+
+// trace_closest of the lanes with `on`; the others get false.
+__device__ __forceinline__ bool warp_closest(const DevScene& s, bool on, const V3& o, const V3& d, HitRec* out) {
+    __syncwarp();
+    return s.nodes8 ? warp_closest_wide(s, on, o, d, out) : warp_closest_binary(s, on, o, d, out);
+}
+
+// trace_occluded of the lanes with `on`; the others get false.
+__device__ __forceinline__ bool warp_occluded(const DevScene& s, bool on, const V3& o, const V3& d, float maxDist) {
+    __syncwarp();
+    return s.nodes8 ? warp_occluded_wide(s, on, o, d, maxDist) : warp_occluded_binary(s, on, o, d, maxDist);
 }
 
 }  // namespace shiro_gpu

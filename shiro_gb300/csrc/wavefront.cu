@@ -34,6 +34,7 @@
 #include "adjoint.cuh"
 #include "context.h"
 #include "integrator.cuh"
+#include "lanes.cuh"
 
 namespace shiro_gpu {
 
@@ -159,8 +160,6 @@ struct AdjWave {
     uint32_t pad;
 };
 constexpr size_t kAdjSlotFloat4 = 2;      // lrem, delta
-
-__device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
 // Appends `item` to a queue when `pred`; one atomicAdd per warp.
 __device__ __forceinline__ void warp_push(uint32_t* counter, uint32_t* queue, bool pred, uint32_t item) {
@@ -369,48 +368,7 @@ __device__ __forceinline__ uint32_t warp_claim(uint32_t* counter, bool pred) {
     return base + __popc(ballot & ((1u << lane_id()) - 1u));
 }
 
-// Lane-level work distribution for the wide-BVH traversal.  A warp claims
-// kFetchChunk queue entries with one atomicAdd and hands them to its lanes;
-// once `refillIdle` lanes have finished their rays they take the next
-// entries, so a warp is not held back by its slowest ray.  Between refills a
-// busy lane visits up to `travSteps` wide nodes (each visit is the same
-// 8-child test for every lane, so lanes at different depths still run it
-// together).
-constexpr uint32_t kFull = 0xffffffffu;
-constexpr uint32_t kFetchChunk = 64;
-
-struct LaneFeed {
-    uint32_t next = 0, end = 0;  // the warp's claimed entries [next, end)
-    bool exhausted = false;
-};
-
-// Assigns queue entries to idle lanes (`has` false); warp-uniform call.
-// Returns the entry index this lane received, or 0xffffffff.
-__device__ __forceinline__ uint32_t feed_lanes(LaneFeed& f, uint32_t* counter, uint32_t count, bool has, int refillIdle) {
-    const uint32_t lane = lane_id();
-    uint32_t got = 0xffffffffu;
-    uint32_t idle = __ballot_sync(kFull, !has);
-    if (f.exhausted || __popc(idle) < refillIdle) return got;
-    while (idle != 0u) {
-        if (f.next >= f.end) {
-            uint32_t b = 0;
-            if (lane == 0) b = atomicAdd(counter, kFetchChunk);
-            b = __shfl_sync(kFull, b, 0);
-            if (b >= count) {
-                f.exhausted = true;
-                break;
-            }
-            f.next = b;
-            f.end = min(b + kFetchChunk, count);
-        }
-        const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
-        const uint32_t take = min(f.end - f.next, static_cast<uint32_t>(__popc(idle)));
-        if (((idle >> lane) & 1u) && rank < take) got = f.next + rank;
-        f.next += take;
-        idle = __ballot_sync(kFull, !has && got == 0xffffffffu);
-    }
-    return got;
-}
+constexpr uint32_t kFetchChunk = 64;  // queue entries a warp of the traversal stages claims at a time
 
 // Per-warp staging of finished rays for the shade queue: entries collect in
 // shared memory and leave `cnt` at a time with one atomicAdd.
@@ -433,36 +391,6 @@ __device__ __forceinline__ void flush_stage(uint32_t* buf, uint32_t& n, uint32_t
 
 __device__ __forceinline__ void log_hit(const WfView& v, uint32_t depth, uint32_t j, const float4& h) {
     if (v.hitLog) v.hitLog[static_cast<size_t>(depth) * v.P + j] = h;
-}
-
-// One step of a warp's wide-BVH traversal: every lane that has a node and no
-// triangle pending visits it; pending triangles wait until kTriLanes lanes
-// hold some (or no lane has a node to visit) and are then tested by those
-// lanes together until fewer than kTriStop hold any (postponed leaves, Ylitie,
-// Karras and Laine 2017).  Tested as soon as a lane finds them, a warp ran its
-// triangle tests for the one or two lanes that had just reached a leaf; on the
-// 1080p field frame nodes are now visited by 24.5 of 32 lanes and triangles
-// tested by 10.4, and the frame takes 112.3 ms instead of 117.9 (kTriLanes 5:
-// 113.3, 12: 113.6, 16: 116.1, 20: 120.1; kTriStop 4: 116.4, 8: 127.9 - lanes
-// left with triangles visit no node).  Holding a second node's triangles per
-// lane, so that fewer wait, costs more registers than it gains (110 against
-// 107.9 ms).  False when no lane has anything left.  Warp-uniform call.
-constexpr int kTriLanes = 8;
-constexpr int kTriStop = 2;
-
-template <typename Visit, typename Test>
-__device__ __forceinline__ bool trav_step(WideTrav& t, Visit&& visit, Test&& test) {
-    if (t.node != kNoNode && !wide_has_tri(t.tBits)) visit();
-    uint32_t pend = __ballot_sync(kFull, wide_has_tri(t.tBits));
-    const uint32_t run = __ballot_sync(kFull, t.node != kNoNode && !wide_has_tri(t.tBits));
-    if (run == 0u && pend == 0u) return false;
-    if (__popc(pend) >= kTriLanes || run == 0u) {
-        do {
-            if (wide_has_tri(t.tBits)) test();
-            pend = __ballot_sync(kFull, wide_has_tri(t.tBits));
-        } while (__popc(pend) >= kTriStop);
-    }
-    return true;
 }
 
 // ---- warp-cooperative triangle tests ----------------------------------------
@@ -620,7 +548,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend(WfView v, DevScene 
             __syncwarp();
             if (hc >= 32u) flush_stage(hb, hc, 32u, &counter(v, kHitCount), v.shadeQ, v.P, false);
             if (mc >= 32u) flush_stage(mb, mc, 32u, &counter(v, kMissCount), v.shadeQ, v.P, true);
-            const uint32_t got = feed_lanes(feed, &counter(v, kFetchExtend), count, has, v.refillIdle);
+            const uint32_t got = feed_lanes<kFetchChunk>(feed, &counter(v, kFetchExtend), count, has, v.refillIdle);
             if (got != 0xffffffffu) {
                 j = q[got];
                 const F4Pair r = ld_pair(&v.ray[j]);
@@ -861,7 +789,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_occlude(WfView v, DevScene
         size_t e = 0;
         for (;;) {
             const bool has = t.node != kNoNode || wide_has_tri(t.tBits);
-            const uint32_t got = feed_lanes(feed, &counter(v, kFetchOcclude), count, has, v.refillIdle);
+            const uint32_t got = feed_lanes<kFetchChunk>(feed, &counter(v, kFetchOcclude), count, has, v.refillIdle);
             if (got != 0xffffffffu) {
                 const uint32_t item = sq[got];
                 const uint32_t j = item >> 3, k = item & 7u;
