@@ -12,6 +12,7 @@
 #include "integrator.cuh"
 #include "kernels.h"
 #include "lanes.cuh"
+#include "resolve.cuh"
 
 namespace shiro_gpu {
 
@@ -133,44 +134,14 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
     }
 }
 
-__global__ void k_resolve(const DevRequest q, uint64_t pixelBase, uint32_t count, const float4* __restrict__ records,
-                          AovPtrs aov) {
+__global__ void __launch_bounds__(128) k_resolve(const DevRequest q, uint64_t pixelBase, uint32_t count,
+                                                 const float4* __restrict__ records, AovPtrs aov) {
+    __shared__ float stage[4][96];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    const uint32_t n = q.sampleCount;
-    float b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f;
-    V3 alb{0.0f, 0.0f, 0.0f}, nrm{0.0f, 0.0f, 0.0f};
-    float depth = __int_as_float(0x7f800000);
-    const float4* r = records + 3 * static_cast<size_t>(i) * n;
-    for (uint32_t k = 0; k < n; ++k) {
-        const float4 a = r[3 * k];
-        b0 = b0 + a.x;
-        b1 = b1 + a.y;
-        b2 = b2 + a.z;
-        const bool hit = a.w < __int_as_float(0x7f800000);
-        b3 = b3 + (hit ? 1.0f : 0.0f);
-        if (hit) {  // without a shaded first hit albedo and normal are zero (and not in the record)
-            const float4 b = r[3 * k + 1], c = r[3 * k + 2];
-            alb = alb + V3{b.x, b.y, b.z};
-            nrm = nrm + V3{c.x, c.y, c.z};
-        }
-        if (a.w < depth) depth = a.w;
-    }
-    const float cnt = static_cast<float>(n);
-    const float inv = 1.0f / cnt;
-    const size_t p = static_cast<size_t>(pixelBase + i);
-    aov.beauty[4 * p + 0] = b0 / cnt;
-    aov.beauty[4 * p + 1] = b1 / cnt;
-    aov.beauty[4 * p + 2] = b2 / cnt;
-    aov.beauty[4 * p + 3] = b3 / cnt;
-    const V3 a = alb * inv, nn = nrm * inv;
-    aov.albedo[3 * p + 0] = a.x;
-    aov.albedo[3 * p + 1] = a.y;
-    aov.albedo[3 * p + 2] = a.z;
-    aov.normal[3 * p + 0] = nn.x;
-    aov.normal[3 * p + 1] = nn.y;
-    aov.normal[3 * p + 2] = nn.z;
-    aov.depth[p] = depth;
+    const bool on = i < count;
+    PixelAov px;
+    if (on) px = resolve_pixel(records + 3 * static_cast<size_t>(i) * q.sampleCount, q.sampleCount);
+    store_pixels(aov, __all_sync(kFull, on) != 0, on, static_cast<size_t>(pixelBase + i), px, stage[threadIdx.x >> 5]);
 }
 
 __global__ void k_primary_hits(const DevScene s, const DevRequest q, uint32_t* __restrict__ prim, float* __restrict__ tout) {

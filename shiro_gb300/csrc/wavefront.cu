@@ -35,6 +35,7 @@
 #include "context.h"
 #include "integrator.cuh"
 #include "lanes.cuh"
+#include "resolve.cuh"
 
 namespace shiro_gpu {
 
@@ -895,49 +896,21 @@ __global__ void wf_end_bounce(WfView v, uint32_t cur) {
 
 // Per-pixel average of the wave's records, same additions as k_resolve.
 __global__ void __launch_bounds__(128) wf_resolve(WfView v) {
+    __shared__ float stage[4][96];
     const WaveDesc w = cur_wave(v);
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < w.pixels; p += gridDim.x * blockDim.x) {
+    const uint32_t lane = lane_id();
+    for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x - lane; base < w.pixels; base += gridDim.x * blockDim.x) {
+        const uint32_t p = base + lane;
+        const bool on = p < w.pixels;
         const WaveSeg& sg = find_seg(v, w, p, true);
         const WfRequest& r = v.reqs[sg.req];
         const uint32_t n = r.q.sampleCount;
         const uint32_t lp = p - sg.pixelOffset;
-        const float4* rec = v.records + 3 * (static_cast<size_t>(sg.pathOffset) + static_cast<size_t>(lp) * n);
-        float b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f;
-        V3 alb{0.0f, 0.0f, 0.0f}, nrm{0.0f, 0.0f, 0.0f};
-        float depth = __int_as_float(0x7f800000);
-        for (uint32_t k = 0; k < n; ++k) {
-            const float4 a = rec[3 * k];
-            b0 = b0 + a.x;
-            b1 = b1 + a.y;
-            b2 = b2 + a.z;
-            const bool hit = a.w < __int_as_float(0x7f800000);
-            b3 = b3 + (hit ? 1.0f : 0.0f);
-            if (hit) {  // albedo and normal of a path whose first ray missed are zero (adding them changes nothing)
-                const float4 b = rec[3 * k + 1], c = rec[3 * k + 2];
-                alb = alb + V3{b.x, b.y, b.z};
-                nrm = nrm + V3{c.x, c.y, c.z};
-            }
-            if (a.w < depth) depth = a.w;
-        }
-        const float cnt = static_cast<float>(n);
-        const float inv = 1.0f / cnt;
-        const size_t px = static_cast<size_t>(sg.pixelStart) + lp;
-        if ((reinterpret_cast<uintptr_t>(r.aov.beauty) & 15u) == 0u) {  // one 16-byte store (host planes too)
-            reinterpret_cast<float4*>(r.aov.beauty)[px] = make_float4(b0 / cnt, b1 / cnt, b2 / cnt, b3 / cnt);
-        } else {
-            r.aov.beauty[4 * px + 0] = b0 / cnt;
-            r.aov.beauty[4 * px + 1] = b1 / cnt;
-            r.aov.beauty[4 * px + 2] = b2 / cnt;
-            r.aov.beauty[4 * px + 3] = b3 / cnt;
-        }
-        const V3 a = alb * inv, nn = nrm * inv;
-        r.aov.albedo[3 * px + 0] = a.x;
-        r.aov.albedo[3 * px + 1] = a.y;
-        r.aov.albedo[3 * px + 2] = a.z;
-        r.aov.normal[3 * px + 0] = nn.x;
-        r.aov.normal[3 * px + 1] = nn.y;
-        r.aov.normal[3 * px + 2] = nn.z;
-        r.aov.depth[px] = depth;
+        PixelAov px;
+        if (on) px = resolve_pixel(v.records + 3 * (static_cast<size_t>(sg.pathOffset) + static_cast<size_t>(lp) * n), n);
+        const uint32_t firstSeg = __shfl_sync(kFull, sg.pixelOffset, 0);
+        const bool together = __all_sync(kFull, on && sg.pixelOffset == firstSeg) != 0;
+        store_pixels(r.aov, together, on, static_cast<size_t>(sg.pixelStart) + lp, px, stage[threadIdx.x >> 5]);
     }
 }
 
