@@ -3,9 +3,9 @@
 // 1. The reference table (EnvironmentMap::BuildImportanceTable,
 //    src/render/EnvironmentMap.cpp:185-236) in the reference's float
 //    arithmetic and order: per row a running sum of
-//    max(0, luminance) * sin(theta_centre) (one thread per row, so each row's
-//    conditional CDF is summed left to right exactly as the reference does),
-//    the rows' normalisation, the row CDF (one thread: H additions in order),
+//    max(0, luminance) * sin(theta_centre) (each row's conditional CDF is
+//    summed left to right exactly as the reference does), the rows'
+//    normalisation, the row CDF (H additions in order),
 //    then the texel masses rowMass * columnMass (LatLongPdf, :302-313).  Only
 //    the H per-row sines come from the host, from the same std::sin the
 //    reference calls, so the tables equal the reference's bit for bit.
@@ -30,6 +30,7 @@
 //    GPU forms them in (the oracle's sequential sweep checks it bit for bit).
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -45,23 +46,47 @@ constexpr double kMassScale = 1152921504606846976.0;  // 2^60
 
 inline unsigned grid_of(uint64_t n, unsigned b) { return static_cast<unsigned>((n + b - 1) / b); }
 
-// Row sums and unnormalised conditional CDFs, one thread per row.
-__global__ void k_env_rows(const float4* __restrict__ tex, const float* __restrict__ sines, uint32_t w, uint32_t h,
-                           float* __restrict__ cond, float* __restrict__ rowSum) {
-    const uint32_t y = blockIdx.x * blockDim.x + threadIdx.x;
+// The running sum `sum` of a warp's 32 values, added in lane order (every lane
+// forms the same sums); returns the lane's own partial sum.
+__device__ __forceinline__ float warp_running_sum(float v, float& sum) {
+    const uint32_t lane = threadIdx.x & 31u;
+    float mine = 0.0f;
+#pragma unroll
+    for (uint32_t j = 0; j < 32; ++j) {
+        sum += __shfl_sync(0xffffffffu, v, j);
+        if (j == lane) mine = sum;
+    }
+    return mine;
+}
+
+// Row sums and unnormalised conditional CDFs, a warp per row: the additions
+// must go left to right, so a row takes its width's worth of them one after
+// another, but the texels come and the partial sums go 32 side by side, the
+// next 32 while these are added.  A thread per row loaded and stored at a
+// row's stride: 288 us for 2048x1024, now 20.
+__global__ void __launch_bounds__(128) k_env_rows(const float4* __restrict__ tex, const float* __restrict__ sines,
+                                                  uint32_t w, uint32_t h, float* __restrict__ cond,
+                                                  float* __restrict__ rowSum) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t y = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (y >= h) return;
     const float sinT = sines[y];
-    const size_t off = static_cast<size_t>(y) * (w + 1u);
     const float4* t = tex + static_cast<size_t>(y) * w;
+    float* out = cond + static_cast<size_t>(y) * (w + 1u);
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     float row = 0.0f;
-    cond[off] = 0.0f;
-    for (uint32_t x = 0; x < w; ++x) {
-        const float4 c = t[x];
+    if (lane == 0) out[0] = 0.0f;
+    float4 next = lane < w ? t[lane] : none;
+    for (uint32_t x0 = 0; x0 < w; x0 += 32u) {
+        const float4 c = next;
+        const uint32_t x = x0 + lane, ahead = x + 32u;  // w < 2^31
+        next = ahead < w ? t[ahead] : none;
         const float lum = c.x * 0.2126f + c.y * 0.7152f + c.z * 0.0722f;
-        row += (0.0f < lum ? lum : 0.0f) * sinT;  // std::max(0.0f, lum)
-        cond[off + x + 1u] = row;
+        const float v = (0.0f < lum ? lum : 0.0f) * sinT;  // std::max(0.0f, lum); past the row 0, which adds nothing
+        const float mine = warp_running_sum(v, row);
+        if (x < w) out[x + 1u] = mine;
     }
-    rowSum[y] = row;
+    if (lane == 0) rowSum[y] = row;
 }
 
 __global__ void k_env_cond_normalize(float* __restrict__ cond, const float* __restrict__ rowSum, uint32_t w,
@@ -74,45 +99,72 @@ __global__ void k_env_cond_normalize(float* __restrict__ cond, const float* __re
     c = row > 0.0f ? c / row : static_cast<float>(x) / static_cast<float>(w);
 }
 
-// Row CDF: H additions in row order (a row without weight counts 1), then
-// the normalisation - one thread, as the reference's loop.
-__global__ void k_env_row_cdf(const float* __restrict__ rowSum, uint32_t h, float* __restrict__ rowCdf) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    float total = 0.0f;
-    rowCdf[0] = 0.0f;
-    for (uint32_t y = 0; y < h; ++y) {
-        const float r = rowSum[y];
-        total += r > 0.0f ? r : 1.0f;
-        rowCdf[y + 1u] = total;
+// Row CDF: H additions in row order (a row without weight counts 1) by the
+// block's first warp, as in k_env_rows, then the normalisation by all of it.
+// One thread for all of it: 114 us for 1024 rows, now 17.
+__global__ void __launch_bounds__(1024) k_env_row_cdf(const float* __restrict__ rowSum, uint32_t h,
+                                                      float* __restrict__ rowCdf) {
+    __shared__ float all;
+    if (threadIdx.x < 32u) {
+        const uint32_t lane = threadIdx.x;
+        float total = 0.0f, next = lane < h ? rowSum[lane] : 1.0f;
+        for (uint32_t y0 = 0; y0 < h; y0 += 32u) {
+            const float r = next;
+            const uint32_t y = y0 + lane;
+            next = y + 32u < h ? rowSum[y + 32u] : 1.0f;
+            const float mine = warp_running_sum(y < h ? (r > 0.0f ? r : 1.0f) : 0.0f, total);
+            if (y < h) rowCdf[y + 1u] = mine;
+        }
+        if (lane == 0) {
+            rowCdf[0] = 0.0f;
+            all = total;
+        }
     }
-    for (uint32_t y = 1; y <= h; ++y)
+    __syncthreads();
+    const float total = all;
+    for (uint32_t y = 1u + threadIdx.x; y <= h; y += blockDim.x)
         rowCdf[y] = total <= 0.0f ? static_cast<float>(y) / static_cast<float>(h) : rowCdf[y] / total;
 }
 
 // Texel masses (into texels.w) and their fixed-point weights; stats[0] +=
-// weights, stats[1] = max weight.
-__global__ void k_env_mass(float4* __restrict__ tex, const float* __restrict__ rowCdf, const float* __restrict__ cond,
-                           uint32_t w, uint32_t h, u64* __restrict__ q, u64* __restrict__ stats) {
-    const uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+// weights, stats[1] = max weight.  Whole numbers, so the order in which the
+// blocks add theirs does not matter; with two atomics a warp on the same two
+// words the 2048x1024 texels took 87 us, with two a block of a resident grid
+// 14.
+__global__ void __launch_bounds__(256) k_env_mass(float4* __restrict__ tex, const float* __restrict__ rowCdf,
+                                                  const float* __restrict__ cond, uint32_t w, uint32_t h,
+                                                  u64* __restrict__ q, u64* __restrict__ stats) {
+    __shared__ u64 sums[8], maxima[8];
     const uint64_t n = static_cast<uint64_t>(w) * h;
-    u64 v = 0;
-    if (i < n) {
-        const uint32_t y = static_cast<uint32_t>(i / w), x = static_cast<uint32_t>(i - static_cast<uint64_t>(y) * w);
+    u64 sum = 0, mx = 0;
+    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
+         i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+        const uint32_t y = static_cast<uint32_t>(i) / w, x = static_cast<uint32_t>(i) - y * w;  // n < 2^31
         const float rowMass = rowCdf[y + 1u] - rowCdf[y];
         const size_t off = static_cast<size_t>(y) * (w + 1u);
         const float colMass = cond[off + x + 1u] - cond[off + x];
         const float m = rowMass * colMass;
         tex[i].w = m;
-        v = m > 0.0f ? static_cast<u64>(static_cast<double>(m) * kMassScale) : 0ull;
+        const u64 v = m > 0.0f ? static_cast<u64>(static_cast<double>(m) * kMassScale) : 0ull;
         q[i] = v;
+        sum += v;
+        mx = v > mx ? v : mx;
     }
-    u64 sum = v, mx = v;
     for (int o = 16; o > 0; o >>= 1) {
         sum += __shfl_xor_sync(0xffffffffu, sum, o);
         const u64 other = __shfl_xor_sync(0xffffffffu, mx, o);
         mx = other > mx ? other : mx;
     }
     if ((threadIdx.x & 31u) == 0u) {
+        sums[threadIdx.x >> 5] = sum;
+        maxima[threadIdx.x >> 5] = mx;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) {
+            sum += sums[k];
+            mx = maxima[k] > mx ? maxima[k] : mx;
+        }
         if (sum) atomicAdd(&stats[0], sum);
         atomicMax(&stats[1], mx);
     }
@@ -270,10 +322,12 @@ int build_env_tables_device(ContextImpl* ctx, DevEnv& d) {
     ENV_CHECK(cudaMemcpyAsync(dSin, sines.data(), h * sizeof(float), cudaMemcpyHostToDevice, st));
     ENV_CHECK(cudaMemsetAsync(stats, 0, 2 * sizeof(u64), st));
     ENV_CHECK(cudaMemsetAsync(first, 0xff, sizeof(unsigned int), st));
-    k_env_rows<<<grid_of(h, 128), 128, 0, st>>>(tex, dSin, w, h, cond, rowSum);
+    k_env_rows<<<grid_of(h, 4), 128, 0, st>>>(tex, dSin, w, h, cond, rowSum);
     k_env_cond_normalize<<<grid_of(n, 256), 256, 0, st>>>(cond, rowSum, w, h);
-    k_env_row_cdf<<<1, 32, 0, st>>>(rowSum, h, rowCdf);
-    k_env_mass<<<grid_of(n, 256), 256, 0, st>>>(tex, rowCdf, cond, w, h, q, stats);
+    k_env_row_cdf<<<1, 1024, 0, st>>>(rowSum, h, rowCdf);
+    int sms = 1;
+    ENV_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+    k_env_mass<<<std::min(grid_of(n, 256), static_cast<unsigned>(8 * sms)), 256, 0, st>>>(tex, rowCdf, cond, w, h, q, stats);
     k_env_first_max<<<grid_of(n, 256), 256, 0, st>>>(q, n, stats, first);
     ENV_CHECK(cudaGetLastError());
     u64 hs[2];
