@@ -35,9 +35,10 @@ namespace {
 // slower: the light samples then run a few lanes at a time.
 //
 // A launch too small to fill kPlainBlocksSmall blocks per SM has no use for
-// more warps and keeps its registers (one path per lane, 96x64 pixels of a
-// sphere: 198 us, 224 with 48 registers; 256x256 303 and
-// 353 us).
+// more warps and keeps its registers (256x256 pixels of a sphere: 303 us, 353
+// with 48 registers); its paths spread over all of those blocks' warps, a few
+// lanes of each (96x64 pixels: 134 us, with 32 a warp 199; 160x120 of every
+// lobe 614 and 738).
 constexpr int kPlainBlocks = 12, kPlainBlocksSmall = 4, kPlainRefill = 4;
 constexpr uint32_t kPlainThreads = 128, kPlainChunk = 32;
 
@@ -45,7 +46,7 @@ template <bool kExt, int kBlocks>
 __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __grid_constant__ DevScene s,
                                                                         const __grid_constant__ DevRequest q,
                                                                         uint64_t pixelBase, uint32_t count,
-                                                                        uint32_t* __restrict__ next,
+                                                                        uint32_t perWarp, uint32_t* __restrict__ next,
                                                                         float4* __restrict__ records) {
     NullCounter ctr;
     PathState ps;
@@ -55,10 +56,11 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
     float depth0 = 0.0f;
     const uint32_t nls = light_sample_count<kExt>(s, q), domeEnd = s.distantCount + s.domeCount * q.domeSamples;
     const float domeDiv = static_cast<float>(q.domeSamples);
-    // the first path of a lane is its own index, the rest come from the queue
-    const uint32_t lanes = gridDim.x * kPlainThreads, queued = count > lanes ? count - lanes : 0u;
-    uint32_t got = blockIdx.x * kPlainThreads + threadIdx.x;
-    if (got >= count) got = 0xffffffffu;
+    // the first perWarp paths of a warp have its own indices, the rest come from the queue
+    const uint32_t warp = (blockIdx.x * kPlainThreads + threadIdx.x) >> 5;
+    const uint32_t first = gridDim.x * (kPlainThreads >> 5) * perWarp, queued = count > first ? count - first : 0u;
+    uint32_t got = warp * perWarp + lane_id();
+    if (lane_id() >= perWarp || got >= count) got = 0xffffffffu;
     LaneFeed feed;
     for (;;) {
         if (got != 0xffffffffu) {
@@ -129,8 +131,8 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
         if (alive && !on)
             records[3 * static_cast<size_t>(path)] = make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, depth0);
         alive = on;
-        got = feed_lanes<kPlainChunk>(feed, next, queued, alive, kPlainRefill);
-        if (got != 0xffffffffu) got += lanes;
+        got = feed_lanes(feed, next, queued, kPlainChunk, alive, kPlainRefill);
+        if (got != 0xffffffffu) got += first;
     }
 }
 
@@ -269,22 +271,25 @@ void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBas
     int device = 0, sms = 1;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const unsigned blocks = grid(count, kPlainThreads);
+    constexpr unsigned kWarps = kPlainThreads / 32;
     const uint64_t pixelBase = pathBase / q.sampleCount;
     uint32_t* next = s.error + 1;  // the path queue's counter
-    if (blocks <= static_cast<unsigned>(kPlainBlocksSmall * sms)) {
+    const unsigned smallWarps = static_cast<unsigned>(kPlainBlocksSmall * sms) * kWarps;
+    if (count <= 32u * smallWarps) {
+        const uint32_t perWarp = (count + smallWarps - 1u) / smallWarps;
+        const unsigned blocks = grid(count, perWarp * kWarps);
         if (s.extended)
-            k_plain_paths<true, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
+            k_plain_paths<true, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, perWarp, next, records);
         else
-            k_plain_paths<false, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
+            k_plain_paths<false, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, perWarp, next, records);
         return;
     }
-    const unsigned resident = std::min(blocks, static_cast<unsigned>(kPlainBlocks * sms));
+    const unsigned blocks = grid(count, kPlainThreads), resident = std::min(blocks, static_cast<unsigned>(kPlainBlocks * sms));
     if (resident < blocks) cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
     if (s.extended)
-        k_plain_paths<true, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
+        k_plain_paths<true, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, 32u, next, records);
     else
-        k_plain_paths<false, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, next, records);
+        k_plain_paths<false, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, 32u, next, records);
 }
 
 void launch_render_paths(const DevScene& s, const DevRequest& q, const uint32_t* pixels, const uint32_t* sampleIdx,

@@ -369,8 +369,6 @@ __device__ __forceinline__ uint32_t warp_claim(uint32_t* counter, bool pred) {
     return base + __popc(ballot & ((1u << lane_id()) - 1u));
 }
 
-constexpr uint32_t kFetchChunk = 64;  // queue entries a warp of the traversal stages claims at a time
-
 // Per-warp staging of finished rays for the shade queue: entries collect in
 // shared memory and leave `cnt` at a time with one atomicAdd.
 __device__ __forceinline__ void flush_stage(uint32_t* buf, uint32_t& n, uint32_t cnt, uint32_t* counter, uint32_t* shadeQ,
@@ -528,6 +526,9 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend(WfView v, DevScene 
         WideTrav t;
         t.node = kNoNode;
         t.tBits = 0u;
+        const WarpShare share = warp_share(count);
+        const bool spare = lane_id() >= share.lanes;
+        const int refill = min(v.refillIdle, static_cast<int>(share.lanes));
         LaneFeed feed;
         bool has = false;
         uint32_t j = 0, hc = 0, mc = 0;
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend(WfView v, DevScene 
             __syncwarp();
             if (hc >= 32u) flush_stage(hb, hc, 32u, &counter(v, kHitCount), v.shadeQ, v.P, false);
             if (mc >= 32u) flush_stage(mb, mc, 32u, &counter(v, kMissCount), v.shadeQ, v.P, true);
-            const uint32_t got = feed_lanes<kFetchChunk>(feed, &counter(v, kFetchExtend), count, has, v.refillIdle);
+            const uint32_t got = feed_lanes(feed, &counter(v, kFetchExtend), count, share.chunk, has || spare, refill);
             if (got != 0xffffffffu) {
                 j = q[got];
                 const F4Pair r = ld_pair(&v.ray[j]);
@@ -786,11 +787,14 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_occlude(WfView v, DevScene
         WideTrav t;
         t.node = kNoNode;
         t.tBits = 0u;
+        const WarpShare share = warp_share(count);
+        const bool spare = lane_id() >= share.lanes;
+        const int refill = min(v.refillIdle, static_cast<int>(share.lanes));
         LaneFeed feed;
         size_t e = 0;
         for (;;) {
             const bool has = t.node != kNoNode || wide_has_tri(t.tBits);
-            const uint32_t got = feed_lanes<kFetchChunk>(feed, &counter(v, kFetchOcclude), count, has, v.refillIdle);
+            const uint32_t got = feed_lanes(feed, &counter(v, kFetchOcclude), count, share.chunk, has || spare, refill);
             if (got != 0xffffffffu) {
                 const uint32_t item = sq[got];
                 const uint32_t j = item >> 3, k = item & 7u;
