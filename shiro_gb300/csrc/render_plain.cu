@@ -160,19 +160,35 @@ __global__ void k_primary_hits(const DevScene s, const DevRequest q, uint32_t* _
     tout[i] = hit ? h.t : FLT_MAX;
 }
 
-__global__ void k_trace_rays(const DevScene s, const float* __restrict__ o, const float* __restrict__ d,
-                             const float* __restrict__ tmax, uint32_t n, uint32_t* __restrict__ prim,
-                             float* __restrict__ tout, uint32_t* __restrict__ occ) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// The closest hit (blockIdx.y 0) and the occlusion of listed rays, perWarp rays a
+// warp: fewer than 32 where the rays would leave SMs without a warp.  Bound by
+// the latency of each ray's chain of node loads: with both queries one after
+// the other in a thread, 32 rays a warp and 89 registers, 1003, 10007, 200003
+// and a million rays at a sphere took 50, 58, 141 and 493 us; as two halves of
+// the grid, spread, at 48 registers 19, 30, 112 and 449 (at 59 registers, 8
+// blocks per SM, 18, 31, 115 and 488; at 40, 12 blocks, 20, 34, 113 and 458).
+// Traced warp by warp (warp_closest) they were slower: 164 for 200003.
+constexpr int kRayBlocks = 10;
+constexpr uint32_t kRayWarpsPerSm = 16;
+
+__global__ void __launch_bounds__(128, kRayBlocks) k_trace_rays(const DevScene s, const float* __restrict__ o,
+                                                                const float* __restrict__ d,
+                                                                const float* __restrict__ tmax, uint32_t n,
+                                                                uint32_t perWarp, uint32_t* __restrict__ prim,
+                                                                float* __restrict__ tout, uint32_t* __restrict__ occ) {
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, i = warp * perWarp + lane_id();
+    if (lane_id() >= perWarp || i >= n) return;
     const V3 ro{o[3 * i], o[3 * i + 1], o[3 * i + 2]};
     const V3 rd{d[3 * i], d[3 * i + 1], d[3 * i + 2]};
-    HitRec h;
     NullCounter ctr;
-    const bool hit = trace_closest(s, ro, rd, &h, ctr);
-    prim[i] = hit ? h.gid : 0xffffffffu;
-    tout[i] = hit ? h.t : FLT_MAX;
-    occ[i] = trace_occluded(s, ro, rd, tmax[i], ctr) ? 1u : 0u;
+    if (blockIdx.y == 0) {
+        HitRec h;
+        const bool hit = trace_closest(s, ro, rd, &h, ctr);
+        prim[i] = hit ? h.gid : 0xffffffffu;
+        tout[i] = hit ? h.t : FLT_MAX;
+    } else {
+        occ[i] = trace_occluded(s, ro, rd, tmax[i], ctr) ? 1u : 0u;
+    }
 }
 
 // Work-counting variant: every `stride`-th path of the request, same
@@ -340,7 +356,12 @@ void launch_count_paths(const DevScene& s, const DevRequest& q, uint32_t stride,
 void launch_trace_rays(const DevScene& s, const float* o, const float* d, const float* tmax, uint32_t n, uint32_t* prim,
                        float* t, uint32_t* occ, cudaStream_t stream) {
     if (n == 0) return;
-    k_trace_rays<<<grid(n, 128), 128, 0, stream>>>(s, o, d, tmax, n, prim, t, occ);
+    int device = 0, sms = 1;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const uint32_t warps = static_cast<uint32_t>(sms) * kRayWarpsPerSm;
+    const uint32_t perWarp = std::min(32u, n / warps + 1u);
+    k_trace_rays<<<dim3(grid(n, 4 * perWarp), 2), 128, 0, stream>>>(s, o, d, tmax, n, perWarp, prim, t, occ);
 }
 
 }  // namespace shiro_gpu
