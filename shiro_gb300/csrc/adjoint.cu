@@ -31,6 +31,7 @@
 #include "bsdf_diff.cuh"
 #include "context.h"
 #include "integrator.cuh"
+#include "resolve.cuh"
 
 namespace shiro_gpu {
 
@@ -301,10 +302,9 @@ __global__ void __launch_bounds__(128) k_frozen(const __grid_constant__ DevScene
     const uint32_t x = static_cast<uint32_t>(pixel - static_cast<uint64_t>(y) * q.width);
     float depth0;
     const V3 L = adj_path(s, q, a, x, y, q.sampleStart + smp, V3{0, 0, 0}, V3{0, 0, 0}, &depth0, false);
-    float4* o = records + 3 * static_cast<size_t>(i);
-    o[0] = make_float4(L.x, L.y, L.z, depth0);
-    o[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    o[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const PathRecords rec(records, count);
+    rec.radiance[i] = make_float4(L.x, L.y, L.z, depth0);
+    st_pair(rec.first + i, make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
 }
 
 __global__ void k_scatter_params(Mat* mats, uint32_t n, const float* base, const float* rough, const float* metal) {

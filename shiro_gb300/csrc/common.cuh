@@ -77,4 +77,25 @@ constexpr uint32_t kErrStackOverflow = 2u;
 constexpr uint32_t kErrBadIndex = 4u;
 constexpr uint32_t kErrQueueOverflow = 8u;
 
+// Two float4 that are read and written together: one 32-byte sector, one
+// 256-bit access (sm_100 and later).  After the first bounce the queues are
+// sparse in the slots, and 16-byte arrays of their own fetched twice the bytes
+// used.
+struct alignas(32) F4Pair {
+    float4 a, b;
+};
+__device__ __forceinline__ F4Pair ld_pair(const F4Pair* p) {
+    F4Pair r;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+                 : "l"(p)
+                 : "memory");
+    return r;
+}
+__device__ __forceinline__ void st_pair(F4Pair* p, const float4& a, const float4& b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 }  // namespace shiro_gpu

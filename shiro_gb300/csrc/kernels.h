@@ -7,8 +7,8 @@
 
 namespace shiro_gpu {
 
-// Per-path result in the scratch buffer: 3 x float4 =
-// (radiance rgb, depth), (albedo rgb, 0), (normal rgb, 0).
+// Per-path result in the scratch buffer: (albedo rgb, 0), (normal rgb, 0) and
+// (radiance rgb, depth), laid out as resolve.cuh's PathRecords.
 constexpr size_t kPathRecordBytes = 3 * sizeof(float4);
 
 struct AovPtrs {
@@ -25,7 +25,7 @@ void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBas
 // One thread per pixel of [pixelBase, pixelBase + count): averages the
 // pixel's sampleCount records in sample order into the AOV planes
 // (CpuPathTracer.cpp:2093-2137).
-void launch_resolve_pixels(const DevRequest& q, uint64_t pixelBase, uint32_t count, const float4* records, AovPtrs aov,
+void launch_resolve_pixels(const DevRequest& q, uint64_t pixelBase, uint32_t count, float4* records, AovPtrs aov,
                            cudaStream_t stream);
 // Diagnostics: listed paths of the plain form (10 floats each: radiance,
 // albedo, normal, depth), and the texel a dome texture's sampler picks for

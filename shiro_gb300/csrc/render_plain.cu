@@ -47,13 +47,14 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
                                                                         const __grid_constant__ DevRequest q,
                                                                         uint64_t pixelBase, uint32_t count,
                                                                         uint32_t perWarp, uint32_t* __restrict__ next,
-                                                                        float4* __restrict__ records) {
+                                                                        float4* records) {
     NullCounter ctr;
     PathState ps;
     Sampler smp{0u, 0u, 0u, s.radical};
     bool alive = false;
     uint32_t path = 0, depth = 0;
     float depth0 = 0.0f;
+    const PathRecords rec(records, count);
     const uint32_t nls = light_sample_count<kExt>(s, q), domeEnd = s.distantCount + s.domeCount * q.domeSamples;
     const float domeDiv = static_cast<float>(q.domeSamples);
     // the first perWarp paths of a warp have its own indices, the rest come from the queue
@@ -95,9 +96,7 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
                     if (depth == 0) {
                         const float4 dc = __ldg(bsdf_rec(s, v.hit.material) + 3);  // DiffuseColor
                         const V3 nn = v.n * 0.5f + V3{0.5f, 0.5f, 0.5f};
-                        float4* o = records + 3 * static_cast<size_t>(path);
-                        o[1] = make_float4(dc.x, dc.y, dc.z, 0.0f);
-                        o[2] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+                        st_pair(rec.first + path, make_float4(dc.x, dc.y, dc.z, 0.0f), make_float4(nn.x, nn.y, nn.z, 0.0f));
                         depth0 = h.t;
                     }
                     if constexpr (kExt) add_emission(s, v, depth, ps);
@@ -129,7 +128,7 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
         }
         if (on) on = ++depth < q.maxDepth;
         if (alive && !on)
-            records[3 * static_cast<size_t>(path)] = make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, depth0);
+            rec.radiance[path] = make_float4(ps.radiance.x, ps.radiance.y, ps.radiance.z, depth0);
         alive = on;
         got = feed_lanes(feed, next, queued, kPlainChunk, alive, kPlainRefill);
         if (got != 0xffffffffu) got += first;
@@ -137,12 +136,13 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
 }
 
 __global__ void __launch_bounds__(128) k_resolve(const DevRequest q, uint64_t pixelBase, uint32_t count,
-                                                 const float4* __restrict__ records, AovPtrs aov) {
+                                                 float4* records, AovPtrs aov) {
     __shared__ float stage[4][96];
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool on = i < count;
     PixelAov px;
-    if (on) px = resolve_pixel(records + 3 * static_cast<size_t>(i) * q.sampleCount, q.sampleCount);
+    if (on) px = resolve_pixel(PathRecords(records, static_cast<uint64_t>(count) * q.sampleCount),
+                               static_cast<uint64_t>(i) * q.sampleCount, q.sampleCount);
     store_pixels(aov, __all_sync(kFull, on) != 0, on, static_cast<size_t>(pixelBase + i), px, stage[threadIdx.x >> 5]);
 }
 
@@ -333,7 +333,7 @@ cudaError_t preload_plain_kernels() {
     return e;
 }
 
-void launch_resolve_pixels(const DevRequest& q, uint64_t pixelBase, uint32_t count, const float4* records, AovPtrs aov,
+void launch_resolve_pixels(const DevRequest& q, uint64_t pixelBase, uint32_t count, float4* records, AovPtrs aov,
                            cudaStream_t stream) {
     if (count == 0) return;
     k_resolve<<<grid(count, 128), 128, 0, stream>>>(q, pixelBase, count, records, aov);

@@ -13,6 +13,19 @@
 
 namespace shiro_gpu {
 
+// The records of `paths` paths in one block: the (albedo, 0), (normal, 0) pairs
+// of all, then the (radiance, depth) of all.  Most paths write the two parts in
+// different stages, and averaging reads the second alone of paths that hit
+// nothing: as three float4 a path, each end of a path wrote half a sector.
+// (1080p x64 field frame 90.7 -> 89.7 ms, 24 uneven frames 30.6 -> 30.1, the
+// plain form's 961x541 15-spp frame 13.1 -> 12.95.)
+struct PathRecords {
+    F4Pair* first;
+    float4* radiance;
+    __device__ __forceinline__ PathRecords(float4* base, uint64_t paths)
+        : first(reinterpret_cast<F4Pair*>(base)), radiance(base + 2 * paths) {}
+};
+
 struct PixelAov {
     float4 beauty;
     V3 albedo, normal;
@@ -41,36 +54,34 @@ struct PixelSum {
 };
 
 // The average of a pixel's n records, the loads of kResolveBatch records in
-// flight at a time (one at a time: 304 and 399 us where four take 297 and 379,
-// a 1279x719 4-spp frame and a wave of uneven frames; eight: 288 and 369, but
-// 25 instead of 17 us for two samples a pixel).
+// flight at a time (measured with records of three float4: one at a time 304
+// and 399 us where four took 297 and 379, a 1279x719 4-spp frame and a wave of
+// uneven frames; eight 288 and 369, but 25 instead of 17 us for two samples a
+// pixel).
 constexpr uint32_t kResolveBatch = 4;
 
-__device__ __forceinline__ PixelAov resolve_pixel(const float4* __restrict__ rec, uint32_t n) {
+__device__ __forceinline__ PixelAov resolve_pixel(const PathRecords& r, uint64_t path, uint32_t n) {
+    const float4* __restrict__ rad = r.radiance + path;
+    const F4Pair* first = r.first + path;
     PixelSum s;
     uint32_t k = 0;
     for (; k + kResolveBatch <= n; k += kResolveBatch) {
-        float4 a[kResolveBatch], b[kResolveBatch], c[kResolveBatch];
+        float4 a[kResolveBatch];
+        F4Pair f[kResolveBatch];
 #pragma unroll
-        for (uint32_t j = 0; j < kResolveBatch; ++j) a[j] = rec[3 * static_cast<size_t>(k + j)];
+        for (uint32_t j = 0; j < kResolveBatch; ++j) a[j] = rad[k + j];
 #pragma unroll
         for (uint32_t j = 0; j < kResolveBatch; ++j) {
-            if (PixelSum::hit(a[j])) {
-                b[j] = rec[3 * static_cast<size_t>(k + j) + 1];
-                c[j] = rec[3 * static_cast<size_t>(k + j) + 2];
-            }
+            if (PixelSum::hit(a[j])) f[j] = ld_pair(first + k + j);
         }
 #pragma unroll
-        for (uint32_t j = 0; j < kResolveBatch; ++j) s.add(a[j], b[j], c[j]);
+        for (uint32_t j = 0; j < kResolveBatch; ++j) s.add(a[j], f[j].a, f[j].b);
     }
     for (; k < n; ++k) {
-        const float4 a = rec[3 * static_cast<size_t>(k)];
-        float4 b{}, c{};
-        if (PixelSum::hit(a)) {
-            b = rec[3 * static_cast<size_t>(k) + 1];
-            c = rec[3 * static_cast<size_t>(k) + 2];
-        }
-        s.add(a, b, c);
+        const float4 a = rad[k];
+        F4Pair f{};
+        if (PixelSum::hit(a)) f = ld_pair(first + k);
+        s.add(a, f.a, f.b);
     }
     const float cnt = static_cast<float>(n);
     const float inv = 1.0f / cnt;
@@ -96,7 +107,7 @@ __device__ __forceinline__ void store_plane3(float* __restrict__ plane, size_t f
 // warp's pixels follow one another, the three-float planes are written through
 // it, 32 consecutive floats a store: the planes may lie in page-locked host
 // memory, and a lane's three floats at a stride of twelve bytes crossed the
-// link as three partial lines (the 40 MB of a 1279x719 frame: 571 us, now 297;
+// link as three partial lines (the 40 MB of a 1279x719 frame: 571 us, now 291;
 // a device-to-host copy of as many bytes takes 208).
 __device__ __forceinline__ void store_pixels(const AovPtrs& aov, bool together, bool on, size_t px, const PixelAov& r,
                                              float* stage) {

@@ -83,27 +83,6 @@ constexpr uint32_t kHitCount = 8, kMissCount = 9;
 // do not queue behind one another (1080p field frame 96.5 -> 95.8 ms).
 constexpr uint32_t kCounters = 10, kCounterStride = 32;
 
-// Two float4 that the stages read and write together: one 32-byte sector, one
-// 256-bit access (sm_100 and later).  After the first bounce the queues are
-// sparse in the slots, and 16-byte arrays of their own fetched twice the bytes
-// used.
-struct alignas(32) F4Pair {
-    float4 a, b;
-};
-__device__ __forceinline__ F4Pair ld_pair(const F4Pair* p) {
-    F4Pair r;
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
-                 : "l"(p)
-                 : "memory");
-    return r;
-}
-__device__ __forceinline__ void st_pair(F4Pair* p, const float4& a, const float4& b) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
-                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
-                 : "memory");
-}
-
 struct WfView {
     // path state, one entry per slot of the wave
     F4Pair* ray;     // (ro.xyz, request), (rd.xyz, prevPdf)
@@ -121,7 +100,8 @@ struct WfView {
     uint32_t* shadeQ;      // rays after extend: hits from the front, misses from the back
     uint32_t* counters;  // 0: ray count A, 1: ray count B, 2: shadow paths, 3: wave index, 4: shadow rays,
                          // 5-7: work fetch, 8: hits, 9: misses
-    float4* records;     // 3 per slot
+    F4Pair* firstHit;    // path records (PathRecords): (albedo, 0), (normal, 0)
+    float4* radiance;    // (radiance, first-hit depth)
     const WaveDesc* waves;
     const WaveSeg* segs;
     const WfRequest* reqs;
@@ -599,7 +579,7 @@ __global__ void __launch_bounds__(256, kMinBlocks) wf_extend(WfView v, DevScene 
 }
 
 __device__ __forceinline__ void write_record(const WfView& v, uint32_t j, const V3& rad, float depth0) {
-    v.records[3 * static_cast<size_t>(j)] = make_float4(rad.x, rad.y, rad.z, depth0);
+    v.radiance[j] = make_float4(rad.x, rad.y, rad.z, depth0);
 }
 
 // Shade stage, compiled with several register caps (the autotuner picks) and
@@ -688,8 +668,7 @@ __global__ void __maxnreg__(kRegs) wf_shade(WfView v, DevScene s, uint32_t cur, 
                         const float4 dc = __ldg(bsdf_rec(s, vx.hit.material) + 3);  // DiffuseColor
                         const V3 alb{dc.x, dc.y, dc.z};
                         const V3 nn = vx.n * 0.5f + V3{0.5f, 0.5f, 0.5f};
-                        v.records[3 * static_cast<size_t>(j) + 1] = make_float4(alb.x, alb.y, alb.z, 0.0f);
-                        v.records[3 * static_cast<size_t>(j) + 2] = make_float4(nn.x, nn.y, nn.z, 0.0f);
+                        st_pair(&v.firstHit[j], make_float4(alb.x, alb.y, alb.z, 0.0f), make_float4(nn.x, nn.y, nn.z, 0.0f));
                         depth0 = h.t;
                     }
                     if constexpr (kExt) add_emission(s, vx, depth, ps);
@@ -911,7 +890,7 @@ __global__ void __launch_bounds__(128) wf_resolve(WfView v) {
         const uint32_t n = r.q.sampleCount;
         const uint32_t lp = p - sg.pixelOffset;
         PixelAov px;
-        if (on) px = resolve_pixel(v.records + 3 * (static_cast<size_t>(sg.pathOffset) + static_cast<size_t>(lp) * n), n);
+        if (on) px = resolve_pixel(PathRecords(reinterpret_cast<float4*>(v.firstHit), v.P), static_cast<uint64_t>(sg.pathOffset) + static_cast<uint64_t>(lp) * n, n);
         const uint32_t firstSeg = __shfl_sync(kFull, sg.pixelOffset, 0);
         const bool together = __all_sync(kFull, on && sg.pixelOffset == firstSeg) != 0;
         store_pixels(r.aov, together, on, static_cast<size_t>(sg.pixelStart) + lp, px, stage[threadIdx.x >> 5]);
@@ -962,7 +941,7 @@ __global__ void __launch_bounds__(128) wa_generate(WfView v, AdjWave aw) {
             v.ident[j] = make_uint4(x, y, smpIdx, sg.req);
             const float cnt = static_cast<float>(q.sampleCount);
             const float4 g = reinterpret_cast<const float4*>(a.dBeauty)[pix];
-            const float4 r = v.records[3 * static_cast<size_t>(j)];
+            const float4 r = v.radiance[j];
             aw.delta[j] = make_float4(g.x / cnt, g.y / cnt, g.z / cnt, 0.0f);
             aw.lrem[j] = make_float4(r.x, r.y, r.z, 0.0f);
             push = g.x != 0.0f || g.y != 0.0f || g.z != 0.0f;
@@ -1301,7 +1280,7 @@ __global__ void __launch_bounds__(128) wf_records_out(WfView v) {
         const WaveSeg& sg = find_seg(v, w, j, false);
         const uint32_t spp = v.reqs[sg.req].q.sampleCount;
         const size_t path = static_cast<size_t>(sg.pixelStart) * spp + (j - sg.pathOffset);
-        v.recordsOut[path] = v.records[3 * static_cast<size_t>(j)];
+        v.recordsOut[path] = v.radiance[j];
     }
 }
 
@@ -1426,7 +1405,8 @@ WfView make_view(WavePool* wf, uint32_t P, uint32_t lightSamples, const WaveDesc
     v.shadeQ = v.shadowRayQ + p * static_cast<size_t>(std::max(1u, lightSamples));
     v.sortedQ = v.shadeQ + p;
     v.binCount = v.sortedQ + p * static_cast<size_t>(std::max(1u, lightSamples));
-    v.records = static_cast<float4*>(wf->records.ptr);
+    v.firstHit = static_cast<F4Pair*>(wf->records.ptr);
+    v.radiance = reinterpret_cast<float4*>(v.firstHit + p);
     v.waves = waves;
     v.segs = segs;
     v.reqs = reqs;
