@@ -23,27 +23,41 @@ namespace {
 // by side (warp_closest, warp_occluded), and lanes whose path has ended take
 // the next path once kPlainRefill of them are idle.  With a thread per path
 // that ran on its own, warps came apart at the first branch and stayed apart
-// (7.3 of 32 lanes active on the 961x541 15-spp field frame); bound by the
-// latency of the tree's loads, the kernel then wants warps in flight rather
-// than registers: at 128, 80, 64, 48 and 40 registers a thread (4, 6, 8, 10,
-// 12 blocks of 128 per SM) that frame takes 18.6, 16.6, 14.9, 13.6 and 13.0 ms
-// (19.5 with a thread per path), the 1280x720 2-spp one 2.57, 2.37, 2.20, 2.09
-// and 2.06 (2.62), 640x480 8 spp with every lobe 10.5 (15.0); 32 registers
-// lose on small scenes again.  Lanes 1, 4, 8 idle: no difference; a warp that
-// waits for all its paths takes 15.0 instead of 13.8 ms.  Pieces of paths left
-// to be continued by whichever lanes stand at the same step were three times
-// slower: the light samples then run a few lanes at a time.
+// (7.3 of 32 lanes active on the 961x541 15-spp field frame, now 11.8); bound
+// by the latency of the tree's loads, the kernel then wants warps in flight
+// rather than registers: at 128, 80, 64, 48 and 40 registers a thread (4, 6, 8,
+// 10, 12 blocks of 128 per SM) that frame takes 18.6, 16.6, 14.9, 13.6 and 13.0
+// ms (19.5 with a thread per path).  Lanes 1, 4, 8 idle: no difference; a warp
+// that waits for all its paths takes 15.0 instead of 13.8 ms.  Paths in any
+// phase side by side were three times slower: the light samples then run a few
+// lanes at a time.
 //
-// A launch too small to fill kPlainBlocksSmall blocks per SM has no use for
-// more warps and keeps its registers (256x256 pixels of a sphere: 303 us, 353
-// with 48 registers); its paths spread over all of those blocks' warps, a few
-// lanes of each (96x64 pixels: 134 us, with 32 a warp 199; 160x120 of every
-// lobe 614 and 738).
-constexpr int kPlainBlocks = 12, kPlainBlocksSmall = 4, kPlainRefill = 4;
-constexpr uint32_t kPlainThreads = 128, kPlainChunk = 32;
+// The next limit was instruction fetch (8.4 stall cycles per issue, 7.4 for
+// loads): 48 warps at 48 places of a long program.  So the warps of larger
+// blocks meet at the starts of a bounce, of its shading and of its
+// continuation, and - where the program is longest, with every lobe in - of
+// each light sample.  Field frame, 1280x720 2-spp field frame, 640x480 8-spp
+// frame with every lobe, 512x512 4-spp sphere: 12.96, 2.08, 10.55 and 1.09 ms
+// without; 12.4, 2.00, 8.7 and 0.87 in 5 blocks of 256; 12.7, 2.13, 7.5 and 0.87
+// in 3 of 512; there with the light samples 13.3, 2.22, 6.3 and 0.88.
+//
+// A launch too small to fill kPlainSmall has no use for more warps and keeps
+// its registers (256x256 pixels of a sphere: 303 us, 353 with 48 registers); its
+// paths spread over all of those blocks' warps, a few lanes of each (96x64
+// pixels: 134 us, with 32 a warp 199; 160x120 of every lobe 614 and 738).
+enum { kSyncBounce = 1, kSyncHit = 2, kSyncContinue = 4, kSyncLight = 8 };
+struct PlainShape {
+    uint32_t threads;
+    int blocks, sync;
+};
+constexpr PlainShape kPlainLean{256, 5, kSyncBounce | kSyncHit | kSyncContinue};
+constexpr PlainShape kPlainExt{512, 3, kSyncBounce | kSyncHit | kSyncContinue | kSyncLight};
+constexpr PlainShape kPlainSmall{128, 4, 0};
+constexpr int kPlainRefill = 4;
+constexpr uint32_t kPlainChunk = 32;
 
-template <bool kExt, int kBlocks>
-__global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __grid_constant__ DevScene s,
+template <bool kExt, uint32_t kThreads, int kBlocks, int kSync>
+__global__ void __launch_bounds__(kThreads, kBlocks) k_plain_paths(const __grid_constant__ DevScene s,
                                                                         const __grid_constant__ DevRequest q,
                                                                         uint64_t pixelBase, uint32_t count,
                                                                         uint32_t perWarp, uint32_t* __restrict__ next,
@@ -58,8 +72,8 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
     const uint32_t nls = light_sample_count<kExt>(s, q), domeEnd = s.distantCount + s.domeCount * q.domeSamples;
     const float domeDiv = static_cast<float>(q.domeSamples);
     // the first perWarp paths of a warp have its own indices, the rest come from the queue
-    const uint32_t warp = (blockIdx.x * kPlainThreads + threadIdx.x) >> 5;
-    const uint32_t first = gridDim.x * (kPlainThreads >> 5) * perWarp, queued = count > first ? count - first : 0u;
+    const uint32_t warp = (blockIdx.x * kThreads + threadIdx.x) >> 5;
+    const uint32_t first = gridDim.x * (kThreads >> 5) * perWarp, queued = count > first ? count - first : 0u;
     uint32_t got = warp * perWarp + lane_id();
     if (lane_id() >= perWarp || got >= count) got = 0xffffffffu;
     LaneFeed feed;
@@ -77,11 +91,16 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
             depth0 = __int_as_float(0x7f800000);
             alive = true;
         }
-        if (__ballot_sync(kFull, alive) == 0u) break;
+        if constexpr (kSync & kSyncBounce) {
+            if (!__syncthreads_or(alive)) break;
+        } else {
+            if (__ballot_sync(kFull, alive) == 0u) break;
+        }
         bool on = alive && q.maxDepth != 0u;
         HitRec h;
         const bool found = warp_closest(s, on, ps.ro, ps.rd, &h);
-        __syncwarp();
+        if constexpr (kSync & kSyncHit) __syncthreads();
+        else __syncwarp();
         bool shaded = false;
         Vertex v;
         if (on) {
@@ -113,6 +132,7 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
             if (k >= nls) break;
             V3 dir, c;
             float reach = 0.0f;
+            if constexpr (kSync & kSyncLight) __syncthreads();
             const bool lit = shaded && light_sample<kExt>(s, q, v, smp, depth, k, &dir, &c, &reach, ctr);
             __syncwarp();
             const bool blocked = warp_occluded(s, lit, shadow_origin(v), dir, reach);
@@ -121,7 +141,8 @@ __global__ void __launch_bounds__(kPlainThreads, kBlocks) k_plain_paths(const __
                 else out = out + c;
             }
         }
-        __syncwarp();
+        if constexpr (kSync & kSyncContinue) __syncthreads();
+        else __syncwarp();
         if (shaded) {
             ps.radiance = ps.radiance + ps.T * out;
             on = continue_path<kExt>(s, q, v, smp, depth, ps, ctr);
@@ -281,31 +302,33 @@ void launch_qmc_table(float* table, cudaStream_t stream) {
     k_qmc_table<<<grid(24u * kQmcTable, 256), 256, 0, stream>>>(table);
 }
 
+template <bool kExt, const PlainShape& kShape>
+static void launch_plain(const DevScene& s, const DevRequest& q, uint64_t pixelBase, uint32_t count, uint32_t perWarp,
+                         unsigned maxBlocks, float4* records, cudaStream_t stream) {
+    const unsigned blocks = grid(count, kShape.threads / 32u * perWarp), resident = std::min(blocks, maxBlocks);
+    uint32_t* next = s.error + 1;  // the path queue's counter
+    if (resident < blocks) cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
+    k_plain_paths<kExt, kShape.threads, kShape.blocks, kShape.sync>
+        <<<resident, kShape.threads, 0, stream>>>(s, q, pixelBase, count, perWarp, next, records);
+}
+
 void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBase, uint32_t count, float4* records,
                         cudaStream_t stream) {
     if (count == 0) return;
     int device = 0, sms = 1;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    constexpr unsigned kWarps = kPlainThreads / 32;
     const uint64_t pixelBase = pathBase / q.sampleCount;
-    uint32_t* next = s.error + 1;  // the path queue's counter
-    const unsigned smallWarps = static_cast<unsigned>(kPlainBlocksSmall * sms) * kWarps;
+    const auto resident = [&](const PlainShape& p) { return static_cast<unsigned>(p.blocks * sms); };
+    const uint32_t smallWarps = resident(kPlainSmall) * kPlainSmall.threads / 32u;
+    const uint32_t perWarp = std::min(32u, (count + smallWarps - 1u) / smallWarps);
     if (count <= 32u * smallWarps) {
-        const uint32_t perWarp = (count + smallWarps - 1u) / smallWarps;
-        const unsigned blocks = grid(count, perWarp * kWarps);
-        if (s.extended)
-            k_plain_paths<true, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, perWarp, next, records);
-        else
-            k_plain_paths<false, kPlainBlocksSmall><<<blocks, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, perWarp, next, records);
-        return;
+        if (s.extended) launch_plain<true, kPlainSmall>(s, q, pixelBase, count, perWarp, ~0u, records, stream);
+        else launch_plain<false, kPlainSmall>(s, q, pixelBase, count, perWarp, ~0u, records, stream);
+    } else {
+        if (s.extended) launch_plain<true, kPlainExt>(s, q, pixelBase, count, 32u, resident(kPlainExt), records, stream);
+        else launch_plain<false, kPlainLean>(s, q, pixelBase, count, 32u, resident(kPlainLean), records, stream);
     }
-    const unsigned blocks = grid(count, kPlainThreads), resident = std::min(blocks, static_cast<unsigned>(kPlainBlocks * sms));
-    if (resident < blocks) cudaMemsetAsync(next, 0, sizeof(uint32_t), stream);
-    if (s.extended)
-        k_plain_paths<true, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, 32u, next, records);
-    else
-        k_plain_paths<false, kPlainBlocks><<<resident, kPlainThreads, 0, stream>>>(s, q, pixelBase, count, 32u, next, records);
 }
 
 void launch_render_paths(const DevScene& s, const DevRequest& q, const uint32_t* pixels, const uint32_t* sampleIdx,
@@ -323,12 +346,17 @@ void launch_env_pick(const DevEnv& e, const float2* u, uint32_t n, bool useCdf, 
     k_env_pick<<<grid(n, 256), 256, 0, stream>>>(e, u, n, useCdf ? 1u : 0u, texel, pdf);
 }
 
+template <bool kExt, const PlainShape& kShape>
+static cudaError_t preload_plain(cudaFuncAttributes* a) {
+    return cudaFuncGetAttributes(a, k_plain_paths<kExt, kShape.threads, kShape.blocks, kShape.sync>);
+}
+
 cudaError_t preload_plain_kernels() {
     cudaFuncAttributes a;
-    cudaError_t e = cudaFuncGetAttributes(&a, k_plain_paths<false, kPlainBlocks>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_paths<true, kPlainBlocks>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_paths<false, kPlainBlocksSmall>);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_plain_paths<true, kPlainBlocksSmall>);
+    cudaError_t e = preload_plain<false, kPlainLean>(&a);
+    if (e == cudaSuccess) e = preload_plain<true, kPlainExt>(&a);
+    if (e == cudaSuccess) e = preload_plain<false, kPlainSmall>(&a);
+    if (e == cudaSuccess) e = preload_plain<true, kPlainSmall>(&a);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_resolve);
     return e;
 }
