@@ -5,7 +5,7 @@ consecutive sample indices starting at `sampleStart` and the batches are
 averaged per pixel (Renderer.cpp:47-110, CpuPathTracer.cpp:2093-2137).  A
 converged image here is the same estimator run for many samples per pixel:
 `converged` renders batches of `batch_spp` consecutive sample indices with the
-plain GPU form (one CUDA thread per path) and accumulates the batch means in
+plain GPU form (a path per lane) and accumulates the batch means in
 float64 on the device.  The spread of the batch means estimates the per-pixel
 variance of one sample, which turns the difference between an image and the
 converged one into z-scores.
