@@ -514,14 +514,12 @@ int shiro_gpu_render_paths(ShiroGpuContext* ctx, const ShiroRenderDesc* request,
  * with sample_count > 1 048 576 is refused (SHIRO_ERR_INVALID_ARGUMENT);
  * all calls share the array, so calls that overlap on the GPU race and must be
  * serialised by the caller.  shiro_gpu_create sets the array up for its device
- * (looks its address up and loads its module and the plain-form kernels), so
- * the device memory this entry point relies on is taken when the context is
- * made, before a caller's allocator claims the rest; if that set-up failed,
- * this entry point returns SHIRO_ERR_CUDA with the reason.  The thread-local
- * memory the kernels use is sized by the CUDA driver at the first launch of a
- * kernel that needs it: a caller that must see no allocation at all renders
- * once with shiro_gpu_render (or this entry point) before claiming the
- * device's memory. */
+ * (looks its address up, loads its module and the plain-form kernels and
+ * launches each of them once over no paths, which has the CUDA driver size
+ * its thread-local memory for them), so the device memory this entry point
+ * relies on is taken when the context is made, before a caller's allocator
+ * claims the rest; if that set-up failed, this entry point returns
+ * SHIRO_ERR_CUDA with the reason. */
 int shiro_gpu_render_static(ShiroGpuContext* ctx, const ShiroRenderDesc* request, const volatile int* cancel,
                             ShiroAovs* out);
 

@@ -34,10 +34,12 @@ void launch_render_paths(const DevScene& s, const DevRequest& q, const uint32_t*
                          uint32_t n, float* out, cudaStream_t stream);
 void launch_env_pick(const DevEnv& e, const float2* u, uint32_t n, bool useCdf, uint32_t* texel, float* pdf,
                      cudaStream_t stream);
-// Loads the plain-form kernels (both k_plain_paths variants and k_resolve)
-// into the current device's context now: under CUDA's lazy module loading a
-// kernel's code is otherwise placed in device memory at its first launch.
-cudaError_t preload_plain_kernels();
+// Loads the plain-form kernels (every k_plain_paths variant and k_resolve) into
+// the current device's context now and has the driver size its thread-local
+// memory for them: under CUDA's lazy module loading a kernel's code, and what
+// thread-local memory it needs beyond that of kernels before it, is otherwise
+// placed in device memory at its first launch.
+cudaError_t preload_plain_kernels(cudaStream_t stream);
 // out[2k], out[2k+1] = Sampler{px, py, index}.next2d(branch) of tuple k
 // (tuples packed as uint4 px, py, index, branch).
 void launch_sample_probe(const uint4* tuples, uint32_t n, const float* table, float* out, cudaStream_t stream);

@@ -346,18 +346,26 @@ void launch_env_pick(const DevEnv& e, const float2* u, uint32_t n, bool useCdf, 
     k_env_pick<<<grid(n, 256), 256, 0, stream>>>(e, u, n, useCdf ? 1u : 0u, texel, pdf);
 }
 
+// Loads an instance and launches it over no paths (it reads no scene then), so
+// that the driver has sized its thread-local memory for it.
 template <bool kExt, const PlainShape& kShape>
-static cudaError_t preload_plain(cudaFuncAttributes* a) {
-    return cudaFuncGetAttributes(a, k_plain_paths<kExt, kShape.threads, kShape.blocks, kShape.sync>);
+static cudaError_t preload_plain(cudaStream_t stream) {
+    k_plain_paths<kExt, kShape.threads, kShape.blocks, kShape.sync>
+        <<<1, kShape.threads, 0, stream>>>(DevScene{}, DevRequest{}, 0, 0u, 32u, nullptr, nullptr);
+    return cudaGetLastError();
 }
 
-cudaError_t preload_plain_kernels() {
+// The shapes keep 960 to 1440 bytes a thread (their registers differ), and the
+// size of a launch chooses one: without this the first large frame after a
+// small one took 65 (lean) to 120 MB (extended) of device memory more.
+cudaError_t preload_plain_kernels(cudaStream_t stream) {
     cudaFuncAttributes a;
-    cudaError_t e = preload_plain<false, kPlainLean>(&a);
-    if (e == cudaSuccess) e = preload_plain<true, kPlainExt>(&a);
-    if (e == cudaSuccess) e = preload_plain<false, kPlainSmall>(&a);
-    if (e == cudaSuccess) e = preload_plain<true, kPlainSmall>(&a);
+    cudaError_t e = preload_plain<false, kPlainLean>(stream);
+    if (e == cudaSuccess) e = preload_plain<true, kPlainExt>(stream);
+    if (e == cudaSuccess) e = preload_plain<false, kPlainSmall>(stream);
+    if (e == cudaSuccess) e = preload_plain<true, kPlainSmall>(stream);
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_resolve);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     return e;
 }
 

@@ -19,8 +19,9 @@
 //    by the caller.  Every record a launch reads was written by the same call,
 //    so nothing needs clearing between calls;
 //  * shiro_gpu_create sets the array up for its device (static_scratch_setup
-//    below): it looks the array's device address up and loads this module and
-//    the plain-form kernels, so the device memory they take is taken then,
+//    below): it looks the array's device address up, loads this module and
+//    the plain-form kernels and launches each of those once over no paths, so
+//    the device memory they take, thread-local memory included, is taken then,
 //    not at the first shiro_gpu_render_static call.  A context made after a
 //    cudaDeviceReset looks the address up again.
 #include <cuda_runtime.h>
@@ -48,9 +49,9 @@ __global__ void k_fill(float* __restrict__ p, uint64_t n, float v) {
 // Called by shiro_gpu_create with the context's device current.  In host code
 // gStaticRecords names a host-side stand-in, so the array's device address is
 // looked up here (which also loads this module, allocating the array); the
-// kernels the static path launches are loaded too, because CUDA's lazy
-// loading would otherwise place their code in device memory at their first
-// launch.  A failure leaves the context usable for every other entry point;
+// kernels the static path launches are loaded and launched too, because CUDA's
+// lazy loading would otherwise place their code, and the driver their
+// thread-local memory, in device memory at their first launch.  A failure leaves the context usable for every other entry point;
 // shiro_gpu_render_static then reports it.
 void static_scratch_setup(ContextImpl* ctx) {
     void* p = nullptr;
@@ -58,7 +59,7 @@ void static_scratch_setup(ContextImpl* ctx) {
     if (e == cudaSuccess && !p) e = cudaErrorInvalidSymbol;
     cudaFuncAttributes a;
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, k_fill);
-    if (e == cudaSuccess) e = preload_plain_kernels();
+    if (e == cudaSuccess) e = preload_plain_kernels(ctx->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         ctx->staticRecords = nullptr;
