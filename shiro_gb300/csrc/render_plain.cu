@@ -44,7 +44,9 @@ namespace {
 // A launch too small to fill kPlainSmall has no use for more warps and keeps
 // its registers (256x256 pixels of a sphere: 303 us, 353 with 48 registers); its
 // paths spread over all of those blocks' warps, a few lanes of each (96x64
-// pixels: 134 us, with 32 a warp 199; 160x120 of every lobe 614 and 738).
+// pixels: 134 us, with 32 a warp 199; 160x120 of every lobe 614 and 738).  How
+// far past its resident lanes (77 824 on 152 SMs) that shape stays the better
+// one is small_paths below.
 enum { kSyncBounce = 1, kSyncHit = 2, kSyncContinue = 4, kSyncLight = 8 };
 struct PlainShape {
     uint32_t threads;
@@ -312,6 +314,32 @@ static void launch_plain(const DevScene& s, const DevRequest& q, uint64_t pixelB
         <<<resident, kShape.threads, 0, stream>>>(s, q, pixelBase, count, perWarp, next, records);
 }
 
+// Launches of at most this many paths take kPlainSmall, a path per lane and as
+// many blocks as that makes; `lanes` are its resident ones.  With few paths per
+// resident lane the larger shapes have no queue to refill lanes from, and what
+// is left is each path's own latency, which fewer registers and the meetings of
+// a block lengthen, the more the deeper the paths and the less of their time is
+// the traversal of a large tree.  Kernel us, kPlainSmall and
+// the larger shape, four samples a pixel: field of 256 objects, depth 3, 100
+// thousand paths 502 and 606, 140 thousand 694 and 662, 180 thousand 770 and 743;
+// field of 16, depth 4, 140 thousand 316 and 359, 180 thousand 351 and 406;
+// sphere, depth 4, 140 thousand 260 and 288, 200 thousand 297 and 308; depth 12,
+// field of 256, 200 thousand 1035 and 1079, 230 thousand 1045 and 976; field of
+// 16, 200 thousand 427 and 515; sphere, 200 thousand 374 and 431.
+// With the extended lobes in, the larger shape pays early where shading is most
+// of the work (every lobe in 36 thousand triangles, depth 4: of the time of a
+// thread per path, 100 thousand paths 0.70 and 0.79, 135 thousand 0.66 and 0.66,
+// 175 thousand 0.70 and 0.61; depth 12: 0.87 and 1.07, 0.74 and 0.88, 0.77 and
+// 0.78) and late in larger scenes (a field of 64 objects, one of them emitting:
+// 100 thousand 0.95 and 1.46, 195 thousand 0.95 and 1.17, 270 thousand 0.93 and
+// 1.06; a transmitting one in a field of 256: 100 thousand 0.91 and 1.23, 195
+// thousand 0.88 and 0.85).
+static uint64_t small_paths(const DevScene& s, const DevRequest& q, uint64_t lanes) {
+    const bool large = s.triCount >= (s.extended ? 1u << 16 : 1u << 18), deep = q.maxDepth > (!s.extended && !large ? 4u : 6u);
+    if (s.extended) return large ? lanes * 3u : lanes * (deep ? 4u : 3u) / 2u;
+    return deep ? lanes * 3u : large ? lanes * 2u : lanes * 5u / 2u;
+}
+
 void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBase, uint32_t count, float4* records,
                         cudaStream_t stream) {
     if (count == 0) return;
@@ -321,8 +349,8 @@ void launch_plain_paths(const DevScene& s, const DevRequest& q, uint64_t pathBas
     const uint64_t pixelBase = pathBase / q.sampleCount;
     const auto resident = [&](const PlainShape& p) { return static_cast<unsigned>(p.blocks * sms); };
     const uint32_t smallWarps = resident(kPlainSmall) * kPlainSmall.threads / 32u;
-    const uint32_t perWarp = std::min(32u, (count + smallWarps - 1u) / smallWarps);
-    if (count <= 32u * smallWarps) {
+    if (count <= small_paths(s, q, 32ull * smallWarps)) {
+        const uint32_t perWarp = std::min(32u, (count + smallWarps - 1u) / smallWarps);
         if (s.extended) launch_plain<true, kPlainSmall>(s, q, pixelBase, count, perWarp, ~0u, records, stream);
         else launch_plain<false, kPlainSmall>(s, q, pixelBase, count, perWarp, ~0u, records, stream);
     } else {
