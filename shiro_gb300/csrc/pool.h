@@ -42,8 +42,12 @@ class DevicePool {
             trim(0);
             e = cudaMalloc(out, size);
         }
-        if (e == cudaSuccess) live_[*out] = size;
-        else *out = nullptr;
+        if (e == cudaSuccess) {
+            live_[*out] = size;
+        } else {
+            cudaGetLastError();  // reported by the return value alone: a later launch's check must not find it
+            *out = nullptr;
+        }
         return e;
     }
 

@@ -1,0 +1,87 @@
+"""Device memory of scene uploads, over a CUDA runtime without a device
+(tests/cpp/fake_cuda.cpp): any allocation may fail."""
+import ctypes as C
+import glob
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from shiro_gb300 import build
+
+    build.build()
+    cuda = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(build.nvcc()))), "include")
+    out = os.path.join(HERE, "cpp", "_build", "libshiro_gpu_fake.so")
+    os.makedirs(os.path.dirname(out), exist_ok=True)
+    objs = sorted(glob.glob(os.path.join(build.BUILD, "*.o")))
+    r = subprocess.run([os.environ.get("CXX", "g++"), "-O1", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", cuda,
+                        "-o", out, os.path.join(HERE, "cpp", "fake_cuda.cpp")] + objs + ["-pthread", "-ldl"],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr[-3000:]
+    so = C.CDLL(out)
+    p, u = C.c_void_p, C.c_size_t
+    for name, args, res in (("fake_reset", [C.c_long, u], None), ("fake_mallocs", [], C.c_long),
+                            ("fake_live_bytes", [], u), ("fake_busy_streams", [], C.c_int), ("fake_pool_new", [], p),
+                            ("fake_pool_delete", [p], None), ("fake_pool_get", [p, u], p), ("fake_pool_put", [p, p], None),
+                            ("shiro_gpu_create", [C.c_int, p], C.c_int), ("shiro_gpu_destroy", [p], None),
+                            ("shiro_gpu_upload_scene", [p, p], C.c_int), ("shiro_gpu_set_bvh_build", [p, C.c_uint32], C.c_int),
+                            ("shiro_gpu_set_params", [p] * 5, C.c_int), ("shiro_gpu_last_error", [p], C.c_char_p),
+                            ("shiro_gpu_last_stats", [p, p], C.c_int)):
+        f = getattr(so, name)
+        f.argtypes, f.restype = args, res
+    return so
+
+
+ANY = (1 << 64) - 1
+
+
+@pytest.fixture
+def context(lib):
+    lib.fake_reset(-1, ANY)
+    ctx = C.c_void_p()
+    assert lib.shiro_gpu_create(0, C.byref(ctx)) == 0
+    assert lib.shiro_gpu_set_bvh_build(ctx, 0) == 0
+    yield ctx
+    lib.fake_reset(-1, ANY)
+    lib.shiro_gpu_destroy(ctx)
+    assert lib.fake_live_bytes() == 0
+
+
+def scene():
+    from shiro_gb300 import scenes
+    from shiro_gb300.abi import MarshalledScene
+
+    sc = scenes.sphere_scene(16, 8, segments=8, rings=6)
+    sc.materials[1].emission_strength, sc.materials[1].emission_color = 2.0, (1.0, 1.0, 1.0)
+    return MarshalledScene(sc)
+
+
+def test_an_upload_succeeds_after_one_that_ran_out_of_memory(lib):
+    from shiro_gb300.abi import SHIRO_ERR_OUT_OF_MEMORY as OUT_OF_MEMORY
+
+    ms = scene()
+    total, failed = 1, 0
+    k = 1
+    while k <= total:
+        lib.fake_reset(-1, ANY)
+        ctx = C.c_void_p()
+        assert lib.shiro_gpu_create(0, C.byref(ctx)) == 0
+        lib.shiro_gpu_set_bvh_build(ctx, 0)
+        lib.fake_reset(k, ANY)
+        rc = lib.shiro_gpu_upload_scene(ctx, ms.ref())
+        if rc != 0:
+            failed += 1
+            total = k + 1
+            assert rc == OUT_OF_MEMORY, (k, rc, lib.shiro_gpu_last_error(ctx))
+        lib.fake_reset(-1, ANY)
+        assert lib.shiro_gpu_upload_scene(ctx, ms.ref()) == 0, (k, lib.shiro_gpu_last_error(ctx))
+        lib.shiro_gpu_destroy(ctx)
+        assert lib.fake_live_bytes() == 0
+        k += 1
+    assert failed > 40
