@@ -14,9 +14,13 @@ namespace shiro_gpu {
 // device blocks each (an upload of 327 k triangles spent 9 ms in cudaMalloc
 // and cudaFree).  A context keeps the blocks given back, up to kMaxIdle bytes,
 // and hands them out again; they return to the driver past that bound, when an
-// allocation fails, and with the context.  A block is used on the context's
-// stream alone, whose order makes the next use follow the last one; calls on
-// one context are serialised by the caller.
+// allocation fails, and with the context.  Within a
+// call a block is used on the context's stream alone, whose order makes the
+// next use follow the last one.  Between calls, which the caller serialises, the
+// stream may become another one (shiro_gpu_set_stream): so every call that
+// takes blocks or gives some back, or reads the scene's, has waited for its
+// stream when it returns, also when it failed, and no block that is idle or
+// replaced by the next upload is still in use.
 class DevicePool {
   public:
     static constexpr size_t kMaxIdle = size_t(1) << 30;

@@ -181,6 +181,8 @@ int fail(ContextImpl* ctx, int code, const std::string& msg) {
 
 int cuda_fail(ContextImpl* ctx, cudaError_t e, const char* what) {
     cudaGetLastError();
+    if (ctx) cudaStreamSynchronize(ctx->stream);  // what the call had queued reads the scene (DevicePool)
+    cudaGetLastError();
     return fail(ctx, e == cudaErrorMemoryAllocation ? SHIRO_ERR_OUT_OF_MEMORY : SHIRO_ERR_CUDA,
                 std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -863,6 +865,13 @@ int upload_shading(ContextImpl* ctx, const ShiroSceneDesc* sd) {
     return SHIRO_OK;
 }
 
+// The status of a call that uses the block pool: one that failed waits for what
+// it had queued (one that succeeded has waited), see DevicePool.
+int settled(ContextImpl* ctx, int rc) {
+    if (rc != SHIRO_OK) cudaStreamSynchronize(ctx->stream);
+    return rc;
+}
+
 int finish_upload(ContextImpl* ctx) {
     DevScene& s = ctx->scene;
     s.error = ctx->errorWord;
@@ -1024,10 +1033,7 @@ int shiro_gpu_supports_scene(const ShiroSceneDesc* scene, char* reason, size_t r
     return ok;
 }
 
-int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
-    if (!handle || !sd) return SHIRO_ERR_INVALID_ARGUMENT;
-    ContextImpl* ctx = &handle->impl;
-    cudaSetDevice(ctx->device);
+static int upload_scene(ContextImpl* ctx, const ShiroSceneDesc* sd) {
     std::string why;
     if (!supports(sd, &why)) return fail(ctx, SHIRO_ERR_UNSUPPORTED_SCENE, "unsupported scene: " + why);
     if (sd->mesh_count && !sd->meshes) return fail(ctx, SHIRO_ERR_INVALID_ARGUMENT, "null mesh array");
@@ -1295,6 +1301,12 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
     return finish_upload(ctx);
 }
 
+int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
+    if (!handle || !sd) return SHIRO_ERR_INVALID_ARGUMENT;
+    cudaSetDevice(handle->impl.device);
+    return settled(&handle->impl, upload_scene(&handle->impl, sd));
+}
+
 int shiro_gpu_render(ShiroGpuContext* handle, const ShiroRenderDesc* req, const volatile int* cancel, ShiroAovs* out) {
     if (!handle || !req || !out) return SHIRO_ERR_INVALID_ARGUMENT;
     ContextImpl* ctx = &handle->impl;
@@ -1460,7 +1472,7 @@ int shiro_gpu_autotune(ShiroGpuContext* ctx, const ShiroRenderDesc* req, ShiroWa
 int shiro_gpu_set_params(ShiroGpuContext* ctx, const float* base, const float* rough, const float* metal, const float* env) {
     if (!ctx) return SHIRO_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->impl.device);
-    return adjoint_set_params(&ctx->impl, base, rough, metal, env);
+    return settled(&ctx->impl, adjoint_set_params(&ctx->impl, base, rough, metal, env));
 }
 
 int shiro_gpu_adjoint(ShiroGpuContext* ctx, const ShiroRenderDesc* req, const float* dBeauty, float* dBase, float* dRough,

@@ -1,10 +1,12 @@
 """Device memory of scene uploads, over a CUDA runtime without a device
-(tests/cpp/fake_cuda.cpp): any allocation may fail."""
+(tests/cpp/fake_cuda.cpp): any allocation may fail, and a call that fails leaves
+nothing queued behind it."""
 import ctypes as C
 import glob
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -79,9 +81,21 @@ def test_an_upload_succeeds_after_one_that_ran_out_of_memory(lib):
             failed += 1
             total = k + 1
             assert rc == OUT_OF_MEMORY, (k, rc, lib.shiro_gpu_last_error(ctx))
+        assert lib.fake_busy_streams() == 0, (k, rc)
         lib.fake_reset(-1, ANY)
         assert lib.shiro_gpu_upload_scene(ctx, ms.ref()) == 0, (k, lib.shiro_gpu_last_error(ctx))
         lib.shiro_gpu_destroy(ctx)
         assert lib.fake_live_bytes() == 0
         k += 1
     assert failed > 40
+
+
+def test_a_refused_parameter_update_leaves_nothing_queued(lib, context):
+    """The materials are written before the missing texture is noticed."""
+    ms = scene()
+    ms.desc.dome_light_count = 0
+    assert lib.shiro_gpu_upload_scene(context, ms.ref()) == 0
+    rough, env = np.full(2, 0.5, np.float32), np.ones((8, 16, 3), np.float32)
+    assert lib.shiro_gpu_set_params(context, None, rough.ctypes.data, None, env.ctypes.data) == -1
+    assert b"no environment texture" in lib.shiro_gpu_last_error(context)
+    assert lib.fake_busy_streams() == 0
