@@ -31,7 +31,8 @@ class DevicePool {
     ~DevicePool() { trim(0); }
 
     cudaError_t get(void** out, size_t bytes) {
-        const size_t size = round(bytes);
+        const size_t exact = steps(bytes, 512);
+        size_t size = exact > kMaxIdle ? exact : round(bytes);  // what is never kept needs no common size
         auto it = idle_.lower_bound(size);
         if (it != idle_.end() && it->first <= size + size / 4) {
             *out = it->second;
@@ -44,6 +45,7 @@ class DevicePool {
         if (e != cudaSuccess) {
             cudaGetLastError();
             trim(0);
+            size = exact;
             e = cudaMalloc(out, size);
         }
         if (e == cudaSuccess) {
@@ -76,12 +78,13 @@ class DevicePool {
     }
 
   private:
+    static size_t steps(size_t bytes, size_t step) { return (std::max<size_t>(bytes, 16) + step - 1) / step * step; }
     // 512-byte steps, then an eighth of the power of two below: blocks of
     // similar size are interchangeable
     static size_t round(size_t bytes) {
         size_t step = 512;
         while (step * 16 < bytes) step <<= 1;
-        return (std::max<size_t>(bytes, 16) + step - 1) / step * step;
+        return steps(bytes, step);
     }
     std::multimap<size_t, void*> idle_;
     std::unordered_map<void*, size_t> live_;

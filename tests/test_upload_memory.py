@@ -99,3 +99,49 @@ def test_a_refused_parameter_update_leaves_nothing_queued(lib, context):
     assert lib.shiro_gpu_set_params(context, None, rough.ctypes.data, None, env.ctypes.data) == -1
     assert b"no environment texture" in lib.shiro_gpu_last_error(context)
     assert lib.fake_busy_streams() == 0
+
+
+def test_pool_takes_no_more_than_asked_where_that_decides(lib):
+    """Blocks of common sizes are up to an eighth larger than asked; not those
+    too large to be kept, nor where only the size asked for is left."""
+    pool = lib.fake_pool_new()
+    lib.fake_reset(-1, ANY)
+    large = (5 << 30) + 512  # past the pool's bound of idle bytes
+    p = lib.fake_pool_get(pool, large)
+    assert p and lib.fake_live_bytes() == large
+    lib.fake_pool_put(pool, p)
+    assert lib.fake_live_bytes() == 0
+    asked = (64 << 20) + 512
+    lib.fake_reset(-1, asked)
+    p = lib.fake_pool_get(pool, asked)
+    assert p and lib.fake_live_bytes() == asked
+    lib.fake_pool_put(pool, p)
+    lib.fake_reset(-1, ANY)
+    lib.fake_pool_delete(pool)
+    assert lib.fake_live_bytes() == 0
+
+
+def test_pool_reuses_bounds_and_retries(lib):
+    pool = lib.fake_pool_new()
+    lib.fake_reset(-1, ANY)
+    a = lib.fake_pool_get(pool, 1000)
+    lib.fake_pool_put(pool, a)
+    assert lib.fake_pool_get(pool, 900) == a and lib.fake_mallocs() == 1  # the same block for a similar size
+    b = lib.fake_pool_get(pool, 1000)
+    assert b != a  # the first is in use
+    lib.fake_pool_put(pool, b)
+    c = lib.fake_pool_get(pool, 100)
+    assert c != b  # the idle one is too large for this
+    lib.fake_pool_put(pool, a)
+    lib.fake_pool_put(pool, c)
+    big = [lib.fake_pool_get(pool, 400 << 20) for _ in range(3)]
+    for p in big:
+        lib.fake_pool_put(pool, p)
+    assert lib.fake_live_bytes() <= 1 << 30  # 1.2 GB given back: the bound's worth is kept
+    lib.fake_reset(-1, 900 << 20)
+    p = lib.fake_pool_get(pool, 850 << 20)  # fits only once the idle ones are gone
+    assert p and lib.fake_live_bytes() <= 900 << 20
+    lib.fake_pool_put(pool, p)
+    lib.fake_reset(-1, ANY)
+    lib.fake_pool_delete(pool)
+    assert lib.fake_live_bytes() == 0
