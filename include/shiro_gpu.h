@@ -337,8 +337,15 @@ void shiro_hdri_free(float* pixels);
  * per-triangle records are kept and only what derives from materials, lights
  * and environments is replaced.  A scene without triangles is accepted and
  * renders as the CPU tracer renders it: every ray misses (the environment,
- * unoccluded lights). */
+ * unoccluded lights).  The context keeps up to 1 GiB of the device memory that
+ * an upload, and the importance tables shiro_gpu_set_params rebuilds, no longer
+ * need, for the next ones; it goes back when an allocation of this context
+ * fails, with the context, or by shiro_gpu_trim. */
 int shiro_gpu_upload_scene(ShiroGpuContext* ctx, const ShiroSceneDesc* scene);
+
+/* Returns the idle device memory kept from uploads to the driver, for another
+ * context or allocator of the device.  The scene stays as it is. */
+int shiro_gpu_trim(ShiroGpuContext* ctx);
 
 /* FrameBuffer RenderSampleBatch(const RenderRequest&)
  * (RenderBackend.h:33; CpuPathTracer.cpp:2043-2170) with the plain
@@ -534,7 +541,8 @@ typedef struct ShiroRenderStats {
     uint64_t triangles;         /* triangles of the uploaded scene */
     uint32_t bvh_depth;
     uint32_t bvh_max_leaf;
-    uint64_t device_bytes;      /* device memory held by the context */
+    uint64_t device_bytes;      /* device memory held by the context: the scene, idle blocks kept from
+                                   uploads, the plain form's and the probes' scratch */
     /* wavefront stages (filled by an event-timed run, use_graph = 0):
      * 0 generate, 1 extend (closest hit), 2 shade, 3 occlusion rays,
      * 4 resolve, 5 light-sample accumulation and queue bookkeeping */

@@ -80,6 +80,7 @@ def load_library(path: str = LIB_PATH):
         "shiro_gpu_set_stream": ([_P, _P], C.c_int),
         "shiro_gpu_supports_scene": ([_P, C.c_char_p, C.c_size_t], C.c_int),
         "shiro_gpu_upload_scene": ([_P, _P], C.c_int),
+        "shiro_gpu_trim": ([_P], C.c_int),
         "shiro_gpu_render": ([_P, _P, _P, _P], C.c_int),
         "shiro_gpu_render_batch": ([_P, _P, _U, _P, _P], C.c_int),
         "shiro_gpu_render_batch_ready": ([_P, _P, _U, _P, _P, abi.PixelsReady, _P], C.c_int),
@@ -220,6 +221,13 @@ class GpuBackend:
             self._scene_key = None
             raise self._err(rc)
         self._scene_key = key
+
+    def trim(self):
+        """Returns the device memory the context keeps from uploads (1 GiB at
+        most) to the driver, for another allocator; the scene stays."""
+        rc = self.lib.shiro_gpu_trim(self._ctx)
+        if rc != 0:
+            raise self._err(rc)
 
     def render(self, scene: Scene, camera: Camera, settings: RenderSettings, sample_start: int = 0,
                sample_count: Optional[int] = None, flags: int = 0, cancel: Optional[C.c_int] = None,

@@ -14,9 +14,9 @@ namespace shiro_gpu {
 // device blocks each (an upload of 327 k triangles spent 9 ms in cudaMalloc
 // and cudaFree).  A context keeps the blocks given back, up to kMaxIdle bytes,
 // and hands them out again; they return to the driver past that bound, when an
-// allocation fails, and with the context.  Within a
-// call a block is used on the context's stream alone, whose order makes the
-// next use follow the last one.  Between calls, which the caller serialises, the
+// allocation of the context fails, at shiro_gpu_trim, and with the context.
+// Within a call a block is used on the context's stream alone, whose order
+// makes the next use follow the last one.  Between calls, which the caller serialises, the
 // stream may become another one (shiro_gpu_set_stream): so every call that
 // takes blocks or gives some back, or reads the scene's, has waited for its
 // stream when it returns, also when it failed, and no block that is idle or
@@ -37,6 +37,7 @@ class DevicePool {
         if (it != idle_.end() && it->first <= size + size / 4) {
             *out = it->second;
             live_[it->second] = it->first;
+            liveBytes_ += it->first;
             idleBytes_ -= it->first;
             idle_.erase(it);
             return cudaSuccess;
@@ -50,6 +51,7 @@ class DevicePool {
         }
         if (e == cudaSuccess) {
             live_[*out] = size;
+            liveBytes_ += size;
         } else {
             cudaGetLastError();  // reported by the return value alone: a later launch's check must not find it
             *out = nullptr;
@@ -63,6 +65,7 @@ class DevicePool {
         if (it == live_.end()) return;
         idle_.emplace(it->second, p);
         idleBytes_ += it->second;
+        liveBytes_ -= it->second;
         live_.erase(it);
         trim(kMaxIdle);
     }
@@ -77,6 +80,9 @@ class DevicePool {
         }
     }
 
+    // Device bytes of the blocks handed out and of the idle ones.
+    size_t bytes() const { return liveBytes_ + idleBytes_; }
+
   private:
     static size_t steps(size_t bytes, size_t step) { return (std::max<size_t>(bytes, 16) + step - 1) / step * step; }
     // 512-byte steps, then an eighth of the power of two below: blocks of
@@ -88,7 +94,7 @@ class DevicePool {
     }
     std::multimap<size_t, void*> idle_;
     std::unordered_map<void*, size_t> live_;
-    size_t idleBytes_ = 0;
+    size_t idleBytes_ = 0, liveBytes_ = 0;
 };
 
 }  // namespace shiro_gpu

@@ -138,9 +138,8 @@ void ContextImpl::freeShading() {
 }
 
 size_t ContextImpl::deviceBytes() const {
-    size_t n = pathRecords.bytes + aovScratch.bytes + probeScratch.bytes;
-    for (const auto& b : sceneBlocks) n += b.bytes;
-    return n;
+    // the scene's blocks and the idle ones are the pool's; error words, table of radical inverses
+    return pathRecords.bytes + aovScratch.bytes + probeScratch.bytes + pool.bytes() + 16 + 24u * kQmcTable * sizeof(float);
 }
 
 bool ensure_block(ContextImpl* ctx, DeviceBlock* b, size_t bytes, const char* what) {
@@ -1305,6 +1304,14 @@ int shiro_gpu_upload_scene(ShiroGpuContext* handle, const ShiroSceneDesc* sd) {
     if (!handle || !sd) return SHIRO_ERR_INVALID_ARGUMENT;
     cudaSetDevice(handle->impl.device);
     return settled(&handle->impl, upload_scene(&handle->impl, sd));
+}
+
+int shiro_gpu_trim(ShiroGpuContext* ctx) {
+    if (!ctx) return SHIRO_ERR_INVALID_ARGUMENT;
+    cudaSetDevice(ctx->impl.device);
+    ctx->impl.pool.trim(0);
+    ctx->impl.stats.device_bytes = ctx->impl.deviceBytes();
+    return SHIRO_OK;
 }
 
 int shiro_gpu_render(ShiroGpuContext* handle, const ShiroRenderDesc* req, const volatile int* cancel, ShiroAovs* out) {

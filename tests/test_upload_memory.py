@@ -34,7 +34,7 @@ def lib():
                             ("shiro_gpu_create", [C.c_int, p], C.c_int), ("shiro_gpu_destroy", [p], None),
                             ("shiro_gpu_upload_scene", [p, p], C.c_int), ("shiro_gpu_set_bvh_build", [p, C.c_uint32], C.c_int),
                             ("shiro_gpu_set_params", [p] * 5, C.c_int), ("shiro_gpu_last_error", [p], C.c_char_p),
-                            ("shiro_gpu_last_stats", [p, p], C.c_int)):
+                            ("shiro_gpu_last_stats", [p, p], C.c_int), ("shiro_gpu_trim", [p], C.c_int)):
         f = getattr(so, name)
         f.argtypes, f.restype = args, res
     return so
@@ -145,3 +145,26 @@ def test_pool_reuses_bounds_and_retries(lib):
     lib.fake_reset(-1, ANY)
     lib.fake_pool_delete(pool)
     assert lib.fake_live_bytes() == 0
+
+
+def test_device_bytes_and_trim(lib, context):
+    """What a context says it holds is what is allocated; trimming gives back
+    what its scene does not need, and the next upload takes it again."""
+    from shiro_gb300.abi import RenderStats
+
+    ms, st = scene(), RenderStats()
+
+    def held():
+        assert lib.shiro_gpu_last_stats(context, C.byref(st)) == 0
+        assert st.device_bytes == lib.fake_live_bytes()
+        return st.device_bytes
+
+    assert lib.shiro_gpu_upload_scene(context, ms.ref()) == 0
+    whole = held()
+    assert lib.shiro_gpu_trim(context) == 0
+    assert held() < whole
+    assert lib.shiro_gpu_upload_scene(context, ms.ref()) == 0  # the geometry stays: shading blocks alone
+    held()
+    lib.fake_reset(1, ANY)  # no new memory: the idle blocks serve
+    assert lib.shiro_gpu_upload_scene(context, ms.ref()) == 0
+    assert lib.shiro_gpu_trim(None) == -1
