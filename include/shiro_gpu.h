@@ -376,7 +376,9 @@ int shiro_gpu_render_batch(ShiroGpuContext* ctx, const ShiroRenderDesc* requests
 typedef struct ShiroWavefrontConfig {
     uint32_t paths_in_flight;
     uint32_t extend_block;
-    uint32_t shade_block;
+    uint32_t shade_block;   /* scenes without transmission, opacity cut-outs and emitters; with them the shade
+                               stage takes 768, 640 or 512 threads by shade_regs (80, 96, 128), and the
+                               autotuner leaves this field as it is */
     uint32_t shadow_block;
     uint32_t use_graph;
     uint32_t shade_regs;    /* register cap of the shade stage: 128, 96 or 80 */

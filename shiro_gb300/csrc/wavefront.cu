@@ -2289,10 +2289,12 @@ int wavefront_autotune(ContextImpl* ctx, const ShiroRenderDesc* req, ShiroWavefr
         c.extend_block = blk;
         if ((rc = trial(c)) != SHIRO_OK) return rc;
     }
-    for (uint32_t blk : {64u, 128u, 256u}) {
-        ShiroWavefrontConfig c = best;
-        c.shade_block = blk;
-        if ((rc = trial(c)) != SHIRO_OK) return rc;
+    if (!ctx->extendedMaterials) {  // (the extended shade stage sizes its own blocks)
+        for (uint32_t blk : {64u, 128u, 256u}) {
+            ShiroWavefrontConfig c = best;
+            c.shade_block = blk;
+            if ((rc = trial(c)) != SHIRO_OK) return rc;
+        }
     }
     for (uint32_t blk : {64u, 128u, 256u}) {
         ShiroWavefrontConfig c = best;
