@@ -85,26 +85,6 @@ __device__ __forceinline__ float ggx_vis(float nDotV, float nDotL, float r) {
     const float a2 = a * a;
     return 1.0f / (1.0f + ggx_lambda(nDotV, a2) + ggx_lambda(nDotL, a2));
 }
-__device__ __forceinline__ V3 spec_lobe(const V3& n, const V3& v, const V3& l, const V3& f0, float r) {
-    const float nv = sclamp(dot(n, v), 0.0f, 1.0f);
-    const float nl = sclamp(dot(n, l), 0.0f, 1.0f);
-    if (nv <= 0.0f || nl <= 0.0f) return {0.0f, 0.0f, 0.0f};
-    const V3 h = safe_normalized(v + l, n);
-    const float nh = sclamp(dot(n, h), 0.0f, 1.0f);
-    const float vh = sclamp(dot(v, h), 0.0f, 1.0f);
-    const float d = ggx_d(nh, r);
-    const float g = ggx_vis(nv, nl, r);
-    return schlick(f0, vh) * (d * g / smax(4.0f * nv * nl, 1.0e-6f));
-}
-__device__ __forceinline__ float spec_pdf(const V3& n, const V3& v, const V3& l, float r) {
-    const float nv = sclamp(dot(n, v), 0.0f, 1.0f);
-    const float nl = sclamp(dot(n, l), 0.0f, 1.0f);
-    if (nv <= 0.0f || nl <= 0.0f) return 0.0f;
-    const V3 h = safe_normalized(v + l, n);
-    const float nh = sclamp(dot(n, h), 0.0f, 1.0f);
-    const float vh = sclamp(dot(v, h), 1.0e-6f, 1.0f);
-    return ggx_d(nh, r) * nh / smax(4.0f * vh, 1.0e-6f);
-}
 __device__ __forceinline__ V3 proj_tangent(const Mat& m, const V3& n) {
     if (m.has_tangent_override) {
         const V3 to = ld3(m.tangent_override);
@@ -149,12 +129,6 @@ static __device__ __noinline__ V3 film_color(float thickness, float ior, float v
     const V3 iri{0.5f + 0.5f * cosf(p0), 0.5f + 0.5f * cosf(p1), 0.5f + 0.5f * cosf(p2)};
     const float strength = sclamp(thickness / 1200.0f, 0.0f, 1.0f);
     return lerp(V3{1.0f, 1.0f, 1.0f}, (V3{1.0f, 1.0f, 1.0f} + iri) * 0.5f, strength);
-}
-__device__ __forceinline__ V3 thin_film(const V3& lobe, const Mat& m, const V3& n, const V3& v, const V3& l) {
-    if (m.thin_film_thickness <= 0.0f) return lobe;
-    const V3 h = safe_normalized(v + l, n);
-    const float vh = sclamp(dot(v, h), 0.0f, 1.0f);
-    return lobe * film_color(m.thin_film_thickness, m.thin_film_ior, vh);
 }
 __device__ __forceinline__ V3 resolve_normal(const Mat& m, const V3& fb, bool coat) {
     const bool has = coat ? m.has_coat_normal_override != 0u : m.has_normal_override != 0u;
