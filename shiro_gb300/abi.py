@@ -353,6 +353,7 @@ def _same_memory(src, arr: np.ndarray) -> bool:
 # of 257 meshes and 65 materials took 4.7 ms to marshal, on every upload.
 _MATERIAL_FIELDS = [f.name for f in fields(Material)]
 _MATERIAL_TRIPLES = sum(1 for _, t in MaterialDesc._fields_ if t is F3)
+_MATERIAL_FLAGS = sum(1 for _, t in MaterialDesc._fields_ if t is C.c_uint32)  # the last ones
 _MATERIAL_PACK = struct.Struct("=" + "".join("3f" if t is F3 else ("I" if t is C.c_uint32 else "f")
                                              for _, t in MaterialDesc._fields_))
 _MATERIAL_GET = operator.attrgetter(*_MATERIAL_FIELDS)
@@ -362,16 +363,18 @@ assert _MESH_PACK.size == C.sizeof(MeshDesc)
 
 
 def _pack_material(buf, i: int, m: Material):
-    v = _MATERIAL_GET(m)
-    triples = v[:_MATERIAL_TRIPLES]
-    try:
-        if all(len(t) == 3 for t in triples):
-            _MATERIAL_PACK.pack_into(buf, i * _MATERIAL_PACK.size, *itertools.chain.from_iterable(triples),
-                                     *v[_MATERIAL_TRIPLES:])
-            return
-    except (struct.error, OverflowError, TypeError):
-        pass
-    buf[i] = m.to_desc()  # values that only the field types convert (past the range of a float, short tuples)
+    """Entry i of the material array: the bytes of m.to_desc()."""
+    if type(m) is Material:  # others describe themselves
+        v = _MATERIAL_GET(m)
+        triples, flags = v[:_MATERIAL_TRIPLES], v[-_MATERIAL_FLAGS:]
+        if all(isinstance(t, tuple) and len(t) == 3 for t in triples) and all(type(b) is bool for b in flags):
+            try:
+                _MATERIAL_PACK.pack_into(buf, i * _MATERIAL_PACK.size, *itertools.chain.from_iterable(triples),
+                                         *v[_MATERIAL_TRIPLES:])
+                return
+            except (struct.error, OverflowError, TypeError):  # past the range of a float, numbers as text
+                pass
+    buf[i] = m.to_desc()
 
 
 def _plain(src, dtype) -> bool:
