@@ -266,8 +266,8 @@ const char* shiro_gpu_last_error(const ShiroGpuContext* ctx);
 /* Selects the acceleration structure the kernels traverse: 2 the binary
  * BVH, 8 the compressed 8-wide BVH (quantised child boxes, octant-ordered
  * slots), 0 (default) each form its faster one on GB300: the wavefront
- * stages the wide BVH, the one-thread-per-path kernels (plain, adjoint,
- * probes) the binary one.  Both give identical hits; the choice only changes
+ * stages the wide BVH, the plain form, the one-thread adjoint, ray queries
+ * and probes the binary one.  Both give identical hits; the choice only changes
  * speed. */
 int shiro_gpu_set_bvh_width(ShiroGpuContext* ctx, uint32_t width);
 
@@ -349,7 +349,7 @@ int shiro_gpu_trim(ShiroGpuContext* ctx);
 
 /* FrameBuffer RenderSampleBatch(const RenderRequest&)
  * (RenderBackend.h:33; CpuPathTracer.cpp:2043-2170) with the plain
- * one-thread-per-path megakernel.  cancel (may be NULL) is polled between
+ * form, one kernel that follows every path to its end.  cancel (may be NULL) is polled between
  * launches of at most 2^24 paths while they run (with a flag given, two
  * launches are queued at most, so another host thread may set it mid-frame);
  * a set flag returns SHIRO_ERR_CANCELLED and leaves the AOVs cleared, as the

@@ -63,7 +63,6 @@ def render(backend, camera: Camera, settings: RenderSettings, base_color, roughn
            sample_start: int = 0, flags: int = 0, adjoint_sample_start=None, wavefront: bool = True):
     """Differentiable render of the backend's uploaded scene (see module doc).
     The forward runs the batched wavefront form (wavefront=True, the faster
-    one; its frames equal the plain form's bit for bit) or the plain
-    one-thread-per-path form."""
+    one; its frames equal the plain form's bit for bit) or the plain form."""
     return _Render.apply(base_color, roughness, metallic, env, backend, camera, settings, sample_start, flags,
                          adjoint_sample_start, wavefront)

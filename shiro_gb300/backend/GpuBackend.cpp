@@ -365,7 +365,7 @@ render::FrameBuffer GpuBackend::RenderSampleBatch(const RenderRequest& request) 
         aovs = FrameAovs(frame);
     }
     // the wavefront form: the faster one, with frames bit-identical to the
-    // one-thread-per-path form's
+    // plain form's
     int rc;
     {
         CancelForward cancel(request.cancel);

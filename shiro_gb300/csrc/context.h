@@ -65,8 +65,9 @@ struct ContextImpl {
     const float4* tris2 = nullptr;    // triangles in the binary BVH's leaf order
     uint32_t node8Count = 0, bvh8Depth = 0;
     // 2: traverse the binary BVH, 8: the compressed wide BVH, 0: the wide one
-    // in the wavefront stages and the binary one in the one-thread-per-path
-    // kernels (each measured faster there on GB300)
+    // in the wavefront stages and the binary one in the plain form, the
+    // one-thread adjoint, ray queries and diagnostics (the rule at
+    // launch_trace_rays says where the wide one would be faster)
     uint32_t bvhWidth = 0;
     // triangles per cluster below the binned-SAH top of the binary BVHs built
     // at the next upload (0: the Morton hierarchy throughout)
@@ -83,7 +84,8 @@ struct ContextImpl {
     DeviceBlock pathRecords;
     DeviceBlock aovScratch;
     DeviceBlock probeScratch;
-    uint32_t* errorWord = nullptr;  // 16 bytes: the error word, the plain form's path counter
+    uint32_t* errorWord = nullptr;  // 16 bytes: the error word, the plain form's path counter (one
+                                  // launch at a time: the context's calls and stream are in order)
     float* radicalTable = nullptr;  // DevScene::radical, built when the context is created
     // device address of the static path-record array of shiro_gpu_render_static
     // (render_static.cu), looked up when the context is created; staticError
