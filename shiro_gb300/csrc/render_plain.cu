@@ -327,11 +327,11 @@ static void launch_plain(const DevScene& s, const DevRequest& q, uint64_t pixelB
 // a block lengthen, the more the deeper the paths and the less of their time is
 // the traversal of a large tree.  Kernel us, kPlainSmall and
 // the larger shape, four samples a pixel: field of 256 objects, depth 3, 100
-// thousand paths 502 and 606, 140 thousand 694 and 662, 180 thousand 770 and 743;
-// field of 16, depth 4, 140 thousand 316 and 359, 180 thousand 351 and 406;
-// sphere, depth 4, 140 thousand 260 and 288, 200 thousand 297 and 308; depth 12,
-// field of 256, 200 thousand 1035 and 1079, 230 thousand 1045 and 976; field of
-// 16, 200 thousand 427 and 515; sphere, 200 thousand 374 and 431.
+// thousand paths 507 and 603, 140 thousand 701 and 673, 180 thousand 794 and 745;
+// field of 16, depth 4, 140 thousand 315 and 361, 180 thousand 345 and 417;
+// sphere, depth 4, 140 thousand 256 and 291, 200 thousand 295 and 310; depth 12,
+// field of 256, 200 thousand 1042 and 1077, 230 thousand 1064 and 964; field of
+// 16, 200 thousand 434 and 522; sphere, 200 thousand 379 and 430.
 // With the extended lobes in, the larger shape pays early where shading is most
 // of the work (every lobe in 36 thousand triangles, depth 4: of the time of a
 // thread per path, 100 thousand paths 0.70 and 0.79, 135 thousand 0.66 and 0.66,
